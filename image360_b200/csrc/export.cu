@@ -57,23 +57,103 @@ __global__ void k_export_source_table(float scale, int n, int* tab)
 }
 
 // Chunks [t0, t0 + gridDim.z) write their placements (PanoramaExporter.cpp:74-101).
-__global__ void k_export_place(const ExportTile* __restrict__ tiles, int t0, float scale, int ow, int oh,
-                               const int* __restrict__ srcOf, unsigned char* __restrict__ out)
+// A warp writes kExportWords x 32 aligned 4-byte words of one placement row,
+// a word per lane at a time, so its stores are whole 128-byte lines; the
+// row's first and last bytes, which may share a word with a neighbouring
+// placement, are stored by the byte.  Bound by HBM: at scale 1 (IDENTITY)
+// the source samples of a word are four consecutive u16, read as two or three
+// words (the samples of a row lie at one phase of the word grid); at any
+// other scale each byte looks its source pixel up.  `clear`: a pixel without
+// a source (rounding at the placement's edge) is written as 0 here - the
+// placements do not overlap and cover the canvas, which is then not cleared
+// beforehand.  Else such pixels are left alone.
+// 17700 x 9600 at scale 1 (1.53 GB): 247 us (0.94 of the copy rate); one pixel
+// per thread (2-byte loads, 1-byte stores) took 735 us and the clearing 83 us.
+constexpr int kExportWords = 8;
+
+template <bool IDENTITY>
+__global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restrict__ tiles, int t0, float scale,
+                                                      int ow, int oh, const int* __restrict__ srcOf, bool clear,
+                                                      unsigned char* __restrict__ out)
 {
     const ExportTile T = tiles[t0 + blockIdx.z];
     int p[4];
     placement(T, scale, p);
-    const int dx = blockIdx.x * blockDim.x + threadIdx.x, dy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (dx >= p[2] || dy >= p[3]) return;
-    const int ox = p[0] + dx, oy = p[1] + dy;
-    if (ox < 0 || ox >= ow || oy < 0 || oy >= oh) return;
-    const int sx = srcOf[dx], sy = srcOf[dy];
-    if (sx < 0 || sx >= T.w || sy < 0 || sy >= T.h) return;
-    const unsigned short* s = T.src + ((size_t)sy * T.w + sx) * 3;
-    unsigned char* o = out + ((size_t)oy * ow + ox) * 3;
-    o[0] = (unsigned char)(s[0] >> 8);
-    o[1] = (unsigned char)(s[1] >> 8);
-    o[2] = (unsigned char)(s[2] >> 8);
+    const int dy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (dy >= p[3]) return;
+    const int oy = p[1] + dy;
+    if (oy < 0 || oy >= oh) return;
+    const long long x0 = p[0] < 0 ? -(long long)p[0] : 0;
+    const long long x1 = (long long)p[0] + p[2] > ow ? (long long)ow - p[0] : p[2];
+    if (x0 >= x1) return;
+    const int sy = IDENTITY ? dy : srcOf[dy];
+    const bool rowIn = sy >= 0 && sy < T.h;
+    if (!rowIn && !clear) return;
+    // bytes [b0, b1) of the placement row, at o + b
+    const long long b0 = x0 * 3, b1 = x1 * 3;
+    unsigned char* o = out + ((long long)oy * ow + p[0]) * 3;
+    const long long rowElems = (long long)T.w * 3;
+    const unsigned short* src = T.src + (size_t)sy * rowElems;  // read only where rowIn
+    const long long chunkElems = (long long)T.h * rowElems;
+    const long long firstElem = (long long)sy * rowElems;  // of the row, in the chunk
+    const long long first = b0 - (long long)(reinterpret_cast<uintptr_t>(o + b0) & 3);  // first word's byte 0
+    const bool odd = (reinterpret_cast<uintptr_t>(src + first) & 2) != 0;  // the samples straddle the word grid
+    const long long base = first + (long long)blockIdx.x * (kExportWords * 128) + threadIdx.x * 4;
+    if (base >= b1) return;
+    // Samples [e0, e1) of the row may be read as words: the words that hold
+    // samples b .. b + 3 hold b - 1 .. b + 4 at most, inside the chunk.
+    const long long e0 = firstElem > 0 ? 0 : 1, e1 = firstElem + rowElems < chunkElems ? rowElems : rowElems - 1;
+    if (IDENTITY && rowIn && base >= b0 && base >= e0 && base + (kExportWords - 1) * 128 + 4 <= b1 &&
+        base + (kExportWords - 1) * 128 + 4 <= e1)
+    {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(src + base - (odd ? 1 : 0));
+        uint32_t* d = reinterpret_cast<uint32_t*>(o + base);
+        uint32_t r[kExportWords];
+        if (!odd)
+        {
+#pragma unroll
+            for (int j = 0; j < kExportWords; ++j)
+                r[j] = __byte_perm(__ldcs(w + j * 64), __ldcs(w + j * 64 + 1), 0x7531);
+        }
+        else
+        {
+#pragma unroll
+            for (int j = 0; j < kExportWords; ++j)
+                r[j] = __byte_perm(__byte_perm(__ldcs(w + j * 64), __ldcs(w + j * 64 + 1), 0x0753),
+                                   __ldcs(w + j * 64 + 2), 0x5210);
+        }
+#pragma unroll
+        for (int j = 0; j < kExportWords; ++j) d[j * 32] = r[j];
+        return;
+    }
+    // the ends of a row, and any other scale
+    for (int j = 0; j < kExportWords; ++j)
+    {
+        const long long b = base + j * 128;
+        if (b >= b1) return;
+        const bool whole = b >= b0 && b + 4 <= b1;
+        uint32_t v = 0;
+        unsigned have = 0;  // bytes with a source
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            const long long e = b + i;
+            if (!rowIn || e < b0 || e >= b1) continue;
+            const int dx = (int)(e / 3);
+            const int sx = IDENTITY ? dx : srcOf[dx];
+            if (sx < 0 || sx >= T.w) continue;
+            v |= (uint32_t)(__ldg(src + (size_t)sx * 3 + (int)(e - (long long)dx * 3)) >> 8) << (8 * i);
+            have |= 1u << i;
+        }
+        if (whole && (have == 15u || clear))
+            *reinterpret_cast<uint32_t*>(o + b) = v;
+        else
+        {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (b + i >= b0 && b + i < b1 && (clear || ((have >> i) & 1u))) o[b + i] = (unsigned char)(v >> (8 * i));
+        }
+    }
 }
 
 struct Scratch
@@ -110,8 +190,11 @@ int export_preview(const std::vector<ExportTile>& tiles, int totalW, int totalH,
         return fail(I360B_INVALID_PARAM, "The %dx%d preview needs %lld bytes (capacity %lld).", ow, oh,
                     (long long)ow * oh * 3, capacity);
     if (!dOut) return fail(I360B_INVALID_PARAM, "Null pointer argument.");
-    I360B_CUDA(cudaMemsetAsync(dOut, 0, (size_t)ow * oh * 3, s), "preview export");
-    if (tiles.empty()) return I360B_SUCCESS;
+    if (tiles.empty())
+    {
+        I360B_CUDA(cudaMemsetAsync(dOut, 0, (size_t)ow * oh * 3, s), "preview export");
+        return I360B_SUCCESS;
+    }
     // placements clipped to the canvas; overlap decides between one launch
     // and one launch per chunk
     std::vector<int> pl(tiles.size() * 4);
@@ -132,6 +215,19 @@ int export_preview(const std::vector<ExportTile>& tiles, int totalW, int totalH,
             const int y0 = std::max(std::max(A[1], B[1]), 0), y1 = std::min(std::min(A[1] + A[3], B[1] + B[3]), oh);
             overlap = x0 < x1 && y0 < y1;
         }
+    // Placements that do not overlap and cover the canvas write every pixel
+    // themselves (a chunk grid at scale 1: one pass over the output instead of
+    // two); else the canvas is cleared first.
+    long long placed = 0;
+    for (size_t t = 0; t < tiles.size(); ++t)
+    {
+        const int* A = &pl[t * 4];
+        const long long x0 = std::max(A[0], 0), x1 = std::min<long long>((long long)A[0] + A[2], ow);
+        const long long y0 = std::max(A[1], 0), y1 = std::min<long long>((long long)A[1] + A[3], oh);
+        if (x0 < x1 && y0 < y1) placed += (x1 - x0) * (y1 - y0);
+    }
+    const bool clear = !overlap && placed == (long long)ow * oh;
+    if (!clear) I360B_CUDA(cudaMemsetAsync(dOut, 0, (size_t)ow * oh * 3, s), "preview export");
     Scratch desc, tab;
     desc.s = tab.s = s;
     const int tabN = std::max(maxW, maxH);
@@ -144,18 +240,20 @@ int export_preview(const std::vector<ExportTile>& tiles, int totalW, int totalH,
     const dim3 block(32, 8);
     const ExportTile* dT = static_cast<const ExportTile*>(desc.p);
     const int* dTab = static_cast<const int*>(tab.p);
-    if (!overlap)
-    {
-        const dim3 grid((maxW + 31) / 32, (maxH + 7) / 8, (unsigned)tiles.size());
-        k_export_place<<<grid, block, 0, s>>>(dT, 0, scale, ow, oh, dTab, dOut);
+    // int(d / 1.0f) = d while the float holds d exactly
+    const bool identity = scale == 1.0f && tabN <= (1 << 24);
+    // a row of w pixels spans at most 3w + 3 bytes from its first word on
+    auto grid = [&](int w, int h, size_t chunks) {
+        return dim3((unsigned)((3ll * w + 3 + kExportWords * 128 - 1) / (kExportWords * 128)), (unsigned)((h + 7) / 8),
+                    (unsigned)chunks);
+    };
+    auto place = [&](const dim3& g, int t0) {
+        if (identity) k_export_place<true><<<g, block, 0, s>>>(dT, t0, scale, ow, oh, dTab, clear, dOut);
+        else k_export_place<false><<<g, block, 0, s>>>(dT, t0, scale, ow, oh, dTab, clear, dOut);
         return check_launch("preview placement kernel");
-    }
-    for (size_t t = 0; t < tiles.size(); ++t)
-    {
-        const dim3 grid((pl[t * 4 + 2] + 31) / 32, (pl[t * 4 + 3] + 7) / 8, 1);
-        k_export_place<<<grid, block, 0, s>>>(dT, (int)t, scale, ow, oh, dTab, dOut);
-        I360B_TRY(check_launch("preview placement kernel"));
-    }
+    };
+    if (!overlap) return place(grid(maxW, maxH, tiles.size()), 0);
+    for (size_t t = 0; t < tiles.size(); ++t) I360B_TRY(place(grid(pl[t * 4 + 2], pl[t * 4 + 3], 1), (int)t));
     return I360B_SUCCESS;
 }
 

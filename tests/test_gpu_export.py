@@ -148,3 +148,30 @@ def test_plan_export_of_a_render(backend, oracle_c, tmp_path):
     with open(path, "rb") as f:
         assert f.read() == oracle_c.tiff16(canvas)
     plan.close()
+
+
+@pytest.mark.parametrize("W,H,cs,shift", [(1, 1, 4, 0), (341, 7, 341, 1), (1025, 130, 64, 0), (1031, 65, 97, 1)])
+def test_preview_full_grid_at_every_alignment(backend, oracle_c, W, H, cs, shift):
+    """A chunk grid that covers the canvas (written without a clear) at full
+    resolution, half and double: odd widths put the rows of source and output
+    at every phase of the 4-byte words; `shift` moves the buffers by one
+    sample / byte.  Exact: bytes."""
+    import torch
+    rng = np.random.default_rng(W + H)
+    tiles, rects = _grid(rng, W, H, cs, missing=())
+    devs = []
+    for t in tiles:
+        d = torch.zeros(t.size + 1, dtype=torch.int16, device="cuda")
+        d[shift:shift + t.size] = _dev(t).reshape(-1)
+        devs.append(d)
+    for md in (max(W, H), max(1, max(W, H) // 2), 2 * max(W, H)):
+        cap = (2 * W + 2) * (2 * H + 2) * 3
+        out = torch.full((cap + 8,), 7, dtype=torch.uint8, device="cuda")
+        r, ow, oh = backend.launch_export_preview([d.data_ptr() + 2 * shift for d in devs], rects, W, H, md,
+                                                  out.data_ptr() + shift, cap)
+        assert r == ComputeResult.SUCCESS
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        exp = oracle_c.export_preview(tiles, rects, W, H, md)
+        assert np.array_equal(got[shift:shift + ow * oh * 3].reshape(oh, ow, 3), exp), md
+        assert (got[:shift] == 7).all() and (got[shift + ow * oh * 3:] == 7).all()
