@@ -33,6 +33,62 @@ __device__ __forceinline__ float fdiv(float a, float b) { return __fdiv_rn(a, b)
 __device__ __forceinline__ float u2f(uint32_t v) { return __fsub_rn(__uint_as_float(0x4B000000u | v), 8388608.0f); }
 __device__ __forceinline__ uint32_t f2u_floor(float x) { return __float_as_uint(__fadd_rz(x, 8388608.0f)) & 0x7FFFFFu; }
 
+// ---------------------------------------------------------------------------
+// Two FP32 operations per instruction (the f32x2 instructions of sm_100).
+// The pixel kernels are bound by instruction issue with the FP32 pipe about a
+// third busy, so pairing their sums and products shortens them.  Each half is
+// rounded on its own, as the scalar operation.  A paired product must not be
+// written as mul.f32x2 where it feeds a paired sum: the assembler contracts
+// the two into a fused multiply-add even under -fmad=false (observed), which
+// drops the product's rounding.  A product is therefore a paired fma, which
+// cannot be contracted with the sum that follows: either with an addend that
+// is exact (an integer t held as T = 2^23 + t: w t = w T - 2^23 w, and the
+// fma rounds that once), or mulx2, whose addend is a -0 read from constant
+// memory, which the assembler cannot take for a constant (x * y + -0 rounds
+// to exactly the product, for zeros of either sign too).
+// ---------------------------------------------------------------------------
+struct f32x2
+{
+    unsigned long long v;
+};
+__device__ __forceinline__ f32x2 pack2(float lo, float hi)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float lo2(f32x2 a)
+{
+    return __uint_as_float((uint32_t)a.v);
+}
+__device__ __forceinline__ float hi2(f32x2 a)
+{
+    return __uint_as_float((uint32_t)(a.v >> 32));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2_rz(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// a * b, rounded once per half; `nz` is neg_zero2().
+__device__ __forceinline__ f32x2 mulx2(f32x2 a, f32x2 b, f32x2 nz) { return fma2(a, b, nz); }
+static __constant__ float2 g_negZero2 = {-0.0f, -0.0f};
+__device__ __forceinline__ f32x2 neg_zero2() { return pack2(g_negZero2.x, g_negZero2.y); }
+__device__ __forceinline__ f32x2 dup2(float v) { return pack2(v, v); }
+
 // (unsigned short)min(max(v, 0), 65535): clamp then truncate toward zero, the
 // quantisation at every stage boundary of the reference (e.g.
 // WarpPerspectiveKernels.h:41, BayerDemosaicKernels.h:58,73, GainColorOps.cpp:23).

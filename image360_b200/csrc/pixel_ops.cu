@@ -3,6 +3,7 @@
 // reference CPU backend's arithmetic bit for bit (FP32, no FMA contraction,
 // truncation at the same points) so outputs match Kernels::Scalar::* exactly.
 #include "common.cuh"
+#include "warp_taps.cuh"
 
 namespace i360b
 {
@@ -228,6 +229,10 @@ __global__ void __launch_bounds__(256) k_demosaic(const unsigned short* __restri
 // ---------------------------------------------------------------------------
 // Warp: backward bilinear homography warp (WarpPerspective_Scalar.cpp:8-45,
 // WarpPerspectiveKernels.h:16-43), with RenderExecutor's ApplyGain fused.
+// A warp makes 64 consecutive pixels of a row, lane l the pixels l and l + 32
+// (consecutive lanes gather neighbouring taps, and the two pixels' arithmetic
+// is paired).  Bound by instruction issue and tap latency: a 2048 x 2048 tile
+// 22.9 us, 26.9 us with scalar arithmetic and 2-byte taps.
 // ---------------------------------------------------------------------------
 struct WarpParams
 {
@@ -236,189 +241,225 @@ struct WarpParams
     int applyGain;
 };
 
-__device__ __forceinline__ void warp_pixel(const unsigned short* __restrict__ src, int sw, int sh, const WarpParams& P,
-                                           float dX, float dY, unsigned short o[3])
+template <bool AFFINE>
+__global__ void __launch_bounds__(256) k_warp(WarpSource src, unsigned short* __restrict__ dst, int dw, int dh,
+                                              int offX, int offY, WarpParams P)
 {
-    float sx = fadd(fadd(fmul(P.H[0], dX), fmul(P.H[1], dY)), P.H[2]);
-    float sy = fadd(fadd(fmul(P.H[3], dX), fmul(P.H[4], dY)), P.H[5]);
-    float sw1 = fadd(fadd(fmul(P.H[6], dX), fmul(P.H[7], dY)), P.H[8]);
-    o[0] = o[1] = o[2] = 0;
-    if (fabsf(sw1) < 1e-10f) return;
-    sx = fdiv(sx, sw1);
-    sy = fdiv(sy, sw1);
-    // floor(s) >= 0 && floor(s) + 1 < size, stated on the float: NaN and
-    // out-of-int-range positions are invalid, as the reference's int
-    // conversion makes them.
-    if (!(sx >= 0.0f && sx < (float)(sw - 1) && sy >= 0.0f && sy < (float)(sh - 1))) return;
-    int x0 = (int)f2u_floor(sx), y0 = (int)f2u_floor(sy);  // 0 <= sx, sy < 2^23 here
-    float fx = fsub(sx, u2f((uint32_t)x0)), fy = fsub(sy, u2f((uint32_t)y0));
-    float gx = fsub(1.0f, fx), gy = fsub(1.0f, fy);
-    float w00 = fmul(gx, gy), w10 = fmul(fx, gy), w01 = fmul(gx, fy), w11 = fmul(fx, fy);
-    const unsigned short* r0 = src + ((size_t)y0 * sw + x0) * 3;
-    const unsigned short* r1 = r0 + (size_t)sw * 3;
+    const int y = blockIdx.y * 8 + threadIdx.y;
+    const int xa = blockIdx.x * 64 + threadIdx.x, xb = xa + 32;
+    if (y >= dh || xa >= dw) return;
+    const float dY = (float)(y + offY);
+    const float hy[3] = {fmul(P.H[1], dY), fmul(P.H[4], dY), fmul(P.H[7], dY)};
+    f32x2 v[3];
+    warp_pair23<AFFINE>(src, P.H, hy, (float)(xa + offX), (float)(xb + offX), true, xb < dw, v);
+    unsigned short* d = dst + ((size_t)y * dw + xa) * 3;
 #pragma unroll
     for (int c = 0; c < 3; ++c)
     {
-        float v = fadd(fadd(fadd(fmul(w00, u2f(__ldg(r0 + c))), fmul(w10, u2f(__ldg(r0 + 3 + c)))),
-                            fmul(w01, u2f(__ldg(r1 + c)))),
-                       fmul(w11, u2f(__ldg(r1 + 3 + c))));
-        o[c] = P.applyGain ? clamp_trunc_u16(fmul(clamp_floor_u16f(v), P.gain)) : clamp_trunc_u16(v);
+        if (P.applyGain) v[c] = gain_pair23(v[c], P.gain);
+        d[c] = (unsigned short)__float_as_uint(lo2(v[c]));
+        if (xb < dw) d[96 + c] = (unsigned short)__float_as_uint(hi2(v[c]));
     }
-}
-
-__global__ void __launch_bounds__(256) k_warp(const unsigned short* __restrict__ src, int sw, int sh,
-                                              unsigned short* __restrict__ dst, int dw, int dh, int offX, int offY,
-                                              WarpParams P)
-{
-    int x = blockIdx.x * 32 + threadIdx.x;
-    int y = blockIdx.y * 8 + threadIdx.y;
-    if (x >= dw || y >= dh) return;
-    unsigned short o[3];
-    warp_pixel(src, sw, sh, P, (float)(x + offX), (float)(y + offY), o);
-    unsigned short* d = dst + ((size_t)y * dw + x) * 3;
-    d[0] = o[0];
-    d[1] = o[1];
-    d[2] = o[2];
 }
 
 // ---------------------------------------------------------------------------
 // Median stack (MedianStackKernels.h:19-55, MedianStack_Scalar.cpp:8-24).
 //
 // Two output scalars per thread, packed as the low and high halves of one
-// 32-bit word per input (one 4-byte load per input: a warp reads 128
-// contiguous bytes of each input).  Per scalar the statistics are
-// accumulated sequentially in input order in FP32 (sumSq exceeds 2^24, so
-// the order is part of the result), exactly as the reference.  The sort is a
-// bitonic network on the packed words with __vminu2/__vmaxu2, so one
-// compare-exchange instruction pair sorts both scalars' stacks.  A clipped
-// value, and every slot past the input count, becomes 0xFFFF: the maximum of
-// the type, so the first keptCount sorted positions hold exactly the sorted
-// kept values (ties with a kept 65535 do not change any value there), and
-// the median is element keptCount/2 - the reference's values[count / 2].
+// 32-bit word per input.  Per scalar the statistics are accumulated
+// sequentially in input order in FP32 (sumSq exceeds 2^24, so the order is
+// part of the result), exactly as the reference.  A value is kept when it
+// lies between the sigma bounds; values are integers, so the bounds become
+// integers (ceil and floor) and both halves are tested at once with
+// __vmaxu2/__vminu2.  A clipped value, and every slot past the input count,
+// becomes 0xFFFF: the maximum of the type, so the first keptCount sorted
+// positions hold exactly the sorted kept values (ties with a kept 65535 do
+// not change any value there), and the median is element keptCount/2 - the
+// reference's values[count / 2].  The sort is Batcher's odd-even merge
+// network (Batcher 1968) for N values on the same packed min/max, cut off at
+// N wires (the wires above would hold the maximum and never move), and only
+// elements 0 .. N/2 are read, so the last stages' unread halves drop out of
+// the code: 26 comparators for 9 inputs and 63 for 16, where a bitonic
+// network of the next power of two has 80 for either.  Bound by the integer
+// pipe (min, max and logic issue at half rate): 72 % busy.  9 inputs of 3001 x
+// 2003: 146 us; one scalar per thread and an unpruned network, which odd
+// counts took before, 469 us.
 // ---------------------------------------------------------------------------
 struct MedianInputs
 {
     const unsigned short* p[kMaxContributors];
 };
 
-template <int P>
-__device__ __forceinline__ void bitonic_sort_u16x2(uint32_t (&v)[P])
+// The stack sizes with a network of their own; a stack in between is padded
+// to the next.  Every size up to 10, where a value adds 2-5 comparators (a
+// tenth to a fifth of the kernel), coarser above.
+#define I360B_STACK_SIZES(X) \
+    X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(16) X(20) X(24) X(28) X(32)
+// The fewest inputs that take network N: inputs below it need no count test.
+__host__ __device__ constexpr int stack_floor(int N) { return N <= 2 ? 1 : N <= 10 ? N : N <= 16 ? N - 1 : N - 3; }
+
+template <int N>
+__device__ __forceinline__ void merge_sort_u16x2(uint32_t (&v)[N])
 {
 #pragma unroll
-    for (int k = 2; k <= P; k <<= 1)
+    for (int p = 1; p < N; p <<= 1)
 #pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1)
+        for (int k = p; k > 0; k >>= 1)
 #pragma unroll
-            for (int i = 0; i < P; ++i)
+            for (int i = 0; i < N; ++i)
             {
-                const int l = i ^ j;
-                if (l > i)
+                const int j0 = k % p;
+                if (i >= j0 && ((i - j0) / k) % 2 == 0 && i + k < N && i / (2 * p) == (i + k) / (2 * p))
                 {
-                    const uint32_t lo = __vminu2(v[i], v[l]), hi = __vmaxu2(v[i], v[l]);
-                    const bool up = (i & k) == 0;
-                    v[i] = up ? lo : hi;
-                    v[l] = up ? hi : lo;
+                    const uint32_t lo = __vminu2(v[i], v[i + k]), hi = __vmaxu2(v[i], v[i + k]);
+                    v[i] = lo;
+                    v[i + k] = hi;
                 }
             }
 }
 
-// Sigma bounds of one scalar's stack (MedianStackKernels.h:22-27).
-__device__ __forceinline__ void clip_bounds(float sum, float sumSq, int n, float sigma, float& lo, float& hi)
+// Running statistics of a packed pair of scalars, added as 2^23 + value.
+struct PairSums
 {
-    const float fn = (float)n;
-    const float mean = fdiv(sum, fn);
-    const float var = fsub(fdiv(sumSq, fn), fmul(mean, mean));
-    const float sd = __fsqrt_rn(var < 0.0f ? 0.0f : var);
-    lo = fsub(mean, fmul(sigma, sd));
-    hi = fadd(mean, fmul(sigma, sd));
+    f32x2 s, q;
+    __device__ __forceinline__ void clear() { s = q = dup2(0.0f); }
+    __device__ __forceinline__ void add23(f32x2 t, f32x2 nz)
+    {
+        const f32x2 m23 = dup2(-8388608.0f);
+        const f32x2 a = add2(t, m23);
+        s = add2(s, a);
+        q = add2(q, fma2(a, t, mulx2(a, m23, nz)));  // a t - 2^23 a = a a, rounded once
+    }
+};
+
+// a / n for a whole n of 2..32 (fn = n, inv = RN(1/n)): Markstein's division
+// with one correction (P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990).  With q0 = RN(a inv), at most 2
+// ulp off, a - n q0 is a multiple of q0's ulp below 64 of them, so the first
+// fma is exact; the second rounds a / n plus an error below 2^-22 ulp, and
+// a / n is either a rounding midpoint - only for n a power of two, where inv
+// and all of this is exact - or at least 1/64 ulp away from one.
+__device__ __forceinline__ float div_count(float a, float fn, float inv)
+{
+    const float q = fmul(a, inv);
+    return __fmaf_rn(__fmaf_rn(-fn, q, a), inv, q);
 }
 
-// The sigma-clipped median of both halves of v[0..n) (v[i] for i >= n must
-// be 0xFFFFFFFF), packed the same way.  v is sorted in place.
-template <int P>
-__device__ __forceinline__ uint32_t median_pair(uint32_t (&v)[P], int n, float sigma)
+// Sigma bounds of one scalar's stack (MedianStackKernels.h:22-27) as the low
+// 16 bits of lo, hi: the whole numbers that pass lo <= value <= hi; every
+// number when none would pass (an empty range, or a bound that is not a
+// number), as the reference then keeps every value.
+__device__ __forceinline__ void clip_range(float sum, float sumSq, float fn, float inv, float sigma, uint32_t& lo,
+                                           uint32_t& hi)
+{
+    const float mean = div_count(sum, fn, inv);
+    const float var = fsub(div_count(sumSq, fn, inv), fmul(mean, mean));
+    const float sd = __fsqrt_rn(var < 0.0f ? 0.0f : var);
+    const float fl = fsub(mean, fmul(sigma, sd)), fh = fadd(mean, fmul(sigma, sd));
+    // on [0, 65535] a sum with 2^23 rounded up / down is 2^23 + ceil / floor
+    const uint32_t l = __float_as_uint(__fadd_ru(fmaxf(fl, 0.0f), 8388608.0f));
+    const uint32_t h = __float_as_uint(__fadd_rd(fminf(fh, 65535.0f), 8388608.0f));
+    const bool some = fl <= 65535.0f && fh >= 0.0f && l <= h;
+    lo = some ? l : 0u;
+    hi = some ? h : 0xffffu;
+}
+
+// The sigma-clipped median of both halves of v[0..n), n <= N (v[i] for
+// i >= n must be 0xFFFFFFFF), packed the same way, from the stack's sums.
+// v is sorted in place; reload(v) restores it.
+template <int N, typename Reload>
+__device__ __forceinline__ uint32_t median_pair(uint32_t (&v)[N], int n, float inv, float sigma, const PairSums& S,
+                                                Reload reload)
 {
     int cntL = n, cntH = n;
-    if (n > 3)
+    if (N > 3 && n > 3)
     {
-        float sL = 0.0f, qL = 0.0f, sH = 0.0f, qH = 0.0f;
-#pragma unroll
-        for (int i = 0; i < P; ++i)
-            if (i < n)
-            {
-                const float a = u2f(v[i] & 0xffffu), b = u2f(v[i] >> 16);
-                sL = fadd(sL, a);
-                qL = fadd(qL, fmul(a, a));
-                sH = fadd(sH, b);
-                qH = fadd(qH, fmul(b, b));
-            }
-        float loL, hiL, loH, hiH;
-        clip_bounds(sL, qL, n, sigma, loL, hiL);
-        clip_bounds(sH, qH, n, sigma, loH, hiH);
-        uint32_t outL = 0, outH = 0;  // bit i: value i is clipped
-        int kL = 0, kH = 0;
-#pragma unroll
-        for (int i = 0; i < P; ++i)
-            if (i < n)
-            {
-                const float a = u2f(v[i] & 0xffffu), b = u2f(v[i] >> 16);
-                const bool keepA = a >= loL && a <= hiL, keepB = b >= loH && b <= hiH;
-                kL += keepA ? 1 : 0;
-                kH += keepB ? 1 : 0;
-                outL |= keepA ? 0u : (1u << i);
-                outH |= keepB ? 0u : (1u << i);
-            }
-        // if nothing is kept the reference keeps every value
-        if (kL == 0) outL = 0;
-        else cntL = kL;
-        if (kH == 0) outH = 0;
-        else cntH = kH;
-#pragma unroll
-        for (int i = 0; i < P; ++i)
+        const float fn = (float)n;
+        uint32_t loL, hiL, loH, hiH;
+        clip_range(lo2(S.s), lo2(S.q), fn, inv, sigma, loL, hiL);
+        clip_range(hi2(S.s), hi2(S.q), fn, inv, sigma, loH, hiH);
+        uint32_t lw = __byte_perm(loL, loH, 0x5410), hw = __byte_perm(hiL, hiH, 0x5410);
+#pragma unroll 1
+        for (;;)
         {
-            if ((outL >> i) & 1u) v[i] |= 0x0000ffffu;
-            if ((outH >> i) & 1u) v[i] |= 0xffff0000u;
+            uint32_t out = 0;  // clipped values per half
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+            {
+                // 1 in a half whose value lies outside its bounds
+                const uint32_t z = __vminu2(__vminu2(__vmaxu2(v[i], lw), hw) ^ v[i], 0x00010001u);
+                out += z;
+                v[i] |= z * 0xffffu;
+            }
+            // the padding slots counted as clipped where the bound is below 0xFFFF
+            out -= (uint32_t)(N - n) * __vminu2(~hw, 0x00010001u);
+            cntL = n - (int)(out & 0xffffu);
+            cntH = n - (int)(out >> 16);
+            if (cntL > 0 && cntH > 0) break;
+            // nothing kept: the reference keeps every value
+            if (cntL == 0) lw &= 0xffff0000u, hw |= 0x0000ffffu;
+            if (cntH == 0) lw &= 0x0000ffffu, hw |= 0xffff0000u;
+            reload(v);
         }
     }
-    bitonic_sort_u16x2<P>(v);
-    const int mL = cntL >> 1, mH = cntH >> 1;
+    merge_sort_u16x2<N>(v);
+    const int mL = cntL >> 1, mH = cntH >> 1;  // <= N / 2
     uint32_t rL = v[0], rH = v[0];
 #pragma unroll
-    for (int i = 1; i < P; ++i)
+    for (int i = 1; i <= N / 2 && i < N; ++i)
     {
         rL = (i == mL) ? v[i] : rL;
         rH = (i == mH) ? v[i] : rH;
     }
-    return (rL & 0x0000ffffu) | (rH & 0xffff0000u);
+    return __byte_perm(rL, rH, 0x7610);
 }
 
-// Packed path: scalars 2t and 2t+1 of every input (4-byte aligned inputs
-// and output, even scalar count).
-template <int P>
-__global__ void __launch_bounds__(256) k_median2(MedianInputs in, int n, long long pairs, float sigma,
-                                                 uint32_t* __restrict__ out)
+// Scalars 2t and 2t+1 of every input; the last scalar of an odd count by
+// itself.  WORDS: every input and the output are 4-byte aligned, so a pair is
+// one word; else two 2-byte accesses.
+template <int N, bool WORDS>
+__global__ void __launch_bounds__(256) k_median(const __grid_constant__ MedianInputs in, int n, float inv,
+                                                long long total, float sigma, unsigned short* __restrict__ out)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= pairs) return;
-    uint32_t v[P];
+    const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2;
+    if (e >= total) return;
+    const bool two = e + 1 < total;
+    auto load = [&](uint32_t (&v)[N]) {
+        if (WORDS && two)
+        {
 #pragma unroll
-    for (int i = 0; i < P; ++i)
-        v[i] = i < n ? __ldg(reinterpret_cast<const uint32_t*>(in.p[i]) + t) : 0xffffffffu;
-    out[t] = median_pair<P>(v, n, sigma);
-}
-
-// General path (any alignment or odd count): one scalar per thread, in the
-// low half of the packed words.
-template <int P>
-__global__ void __launch_bounds__(256) k_median1(MedianInputs in, int n, long long total, float sigma,
-                                                 unsigned short* __restrict__ out)
-{
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= total) return;
-    uint32_t v[P];
+            for (int i = 0; i < N; ++i)
+                v[i] = (i < stack_floor(N) || i < n) ? __ldg(reinterpret_cast<const uint32_t*>(in.p[i] + e))
+                                                     : 0xffffffffu;
+        }
+        else
+        {
 #pragma unroll
-    for (int i = 0; i < P; ++i) v[i] = i < n ? ((uint32_t)__ldg(in.p[i] + idx) | 0xffff0000u) : 0xffffffffu;
-    out[idx] = (unsigned short)(median_pair<P>(v, n, sigma) & 0xffffu);
+            for (int i = 0; i < N; ++i)
+                v[i] = (i < stack_floor(N) || i < n)
+                           ? (uint32_t)__ldg(in.p[i] + e) | (two ? (uint32_t)__ldg(in.p[i] + e + 1) << 16 : 0u)
+                           : 0xffffffffu;
+        }
+    };
+    uint32_t v[N];
+    load(v);
+    PairSums S;
+    S.clear();
+    if (N > 3)
+    {
+        const f32x2 nz = neg_zero2();
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (i < stack_floor(N) || i < n) S.add23(pack2(u16lo23(v[i]), u16hi23(v[i])), nz);
+    }
+    const uint32_t m = median_pair<N>(v, n, inv, sigma, S, load);
+    if (WORDS && two)
+        *reinterpret_cast<uint32_t*>(out + e) = m;
+    else
+    {
+        out[e] = (unsigned short)(m & 0xffffu);
+        if (two) out[e + 1] = (unsigned short)(m >> 16);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -426,69 +467,77 @@ __global__ void __launch_bounds__(256) k_median1(MedianInputs in, int n, long lo
 // same destination grid (IComputeBackend::WarpPerspective of every frame,
 // then MedianStack over the warped buffers: CpuComputeBackend.cpp:112-159).
 // Each destination pixel's n samples are computed with the warp's exact FP32
-// arithmetic and stacked in registers, so the warped frames are never
-// written; a thread makes two horizontally adjacent pixels and stacks their
-// channels as three packed pairs (r, g, b of pixel x in the low halves, of
-// pixel x+1 in the high halves).
+// arithmetic, so the warped frames are never written.  A thread makes the
+// pixels l and l + 32 of its warp's 64-pixel row segment and stacks their
+// channels as three packed pairs.  Bound by instruction issue.  The frames
+// are walked by a rolled loop that leaves the packed samples in shared memory
+// (12 n bytes per thread) and the running sums in registers, and the channels
+// are then sorted one after another by one rolled loop: the unrolled form
+// held 48 samples in registers and its code did not fit the instruction cache.
+// 16 frames of 4000 x 3000: 1.90 ms unrolled with scalar arithmetic and 2-byte
+// taps, 1.23 ms rolled with the taps as words, 1.14 ms with the paired
+// arithmetic (6155 -> 4783 instructions per warp; issue 69 % busy, the rest
+// waiting for taps).  Two frames in flight, 64 threads or 10 blocks per SM
+// were no faster.
 // ---------------------------------------------------------------------------
+constexpr int kWmThreads = 128;
+
 struct StackParams
 {
     const unsigned short* src[kMaxContributors];
     float H[kMaxContributors][9];
+    uint32_t affine;  // bit i: frame i's homography has the third row (0, 0, 1)
 };
 
-template <int P>
-__global__ void __launch_bounds__(256) k_warp_median(StackParams S, int n, int sw, int sh,
-                                                     unsigned short* __restrict__ dst, int dw, int dh, int offX,
-                                                     int offY, float sigma)
+template <int N>
+__global__ void __launch_bounds__(kWmThreads) k_warp_median(const __grid_constant__ StackParams S, int n, float inv,
+                                                            int sw, int sh, unsigned short* __restrict__ dst, int dw,
+                                                            int dh, int offX, int offY, float sigma)
 {
-    const int x = (blockIdx.x * 32 + threadIdx.x) * 2;
-    const int y = blockIdx.y * 8 + threadIdx.y;
-    if (x >= dw || y >= dh) return;
-    const bool two = x + 1 < dw;
-    const float dX = (float)(x + offX), dY = (float)(y + offY);
-    uint32_t r[P], g[P], b[P];
+    extern __shared__ uint32_t stack[];  // [frame][channel][thread]
+    const int tilesX = (dw + 63) / 64;   // blocks in row order (a linear grid holds any number of rows)
+    const int by = blockIdx.x / tilesX, bx = blockIdx.x - by * tilesX;
+    const int y = by * (kWmThreads / 32) + threadIdx.y;
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    const int xa = bx * 64 + threadIdx.x, xb = xa + 32;
+    if (y >= dh || xa >= dw) return;  // no barrier below: a thread reads only what it wrote
+    const float dY = (float)(y + offY), dXa = (float)(xa + offX), dXb = (float)(xb + offX);
+    const f32x2 nz = neg_zero2();
+    PairSums sums[3];
 #pragma unroll
-    for (int i = 0; i < P; ++i)
+    for (int c = 0; c < 3; ++c) sums[c].clear();
+#pragma unroll 1
+    for (int i = 0; i < n; ++i)
     {
-        r[i] = g[i] = b[i] = 0xffffffffu;
-        if (i < n)
-        {
-            WarpParams W;
+        const float* H = S.H[i];
+        const WarpSource src = warp_source(S.src[i], sw, sh);
+        const float hy[3] = {fmul(H[1], dY), fmul(H[4], dY), fmul(H[7], dY)};
+        f32x2 v[3];
+        if ((S.affine >> i) & 1u) warp_pair23<true>(src, H, hy, dXa, dXb, true, xb < dw, v);
+        else warp_pair23<false>(src, H, hy, dXa, dXb, true, xb < dw, v);
 #pragma unroll
-            for (int q = 0; q < 9; ++q) W.H[q] = S.H[i][q];
-            W.gain = 1.0f;
-            W.applyGain = 0;
-            unsigned short a[3], c[3] = {0, 0, 0};
-            warp_pixel(S.src[i], sw, sh, W, dX, dY, a);
-            if (two) warp_pixel(S.src[i], sw, sh, W, (float)(x + 1 + offX), dY, c);
-            r[i] = (uint32_t)a[0] | ((uint32_t)c[0] << 16);
-            g[i] = (uint32_t)a[1] | ((uint32_t)c[1] << 16);
-            b[i] = (uint32_t)a[2] | ((uint32_t)c[2] << 16);
+        for (int c = 0; c < 3; ++c)
+        {
+            stack[(i * 3 + c) * kWmThreads + tid] =
+                __byte_perm(__float_as_uint(lo2(v[c])), __float_as_uint(hi2(v[c])), 0x5410);
+            sums[c].add23(v[c], nz);
         }
     }
-    const uint32_t mr = median_pair<P>(r, n, sigma);
-    const uint32_t mg = median_pair<P>(g, n, sigma);
-    const uint32_t mb = median_pair<P>(b, n, sigma);
-    unsigned short* o = dst + ((size_t)y * dw + x) * 3;
-    if (two && ((reinterpret_cast<uintptr_t>(o) & 3) == 0))
+    unsigned short* oa = dst + ((size_t)y * dw + xa) * 3;
+#pragma unroll 1
+    for (int c = 0; c < 3; ++c)
     {
-        uint32_t* o32 = reinterpret_cast<uint32_t*>(o);
-        o32[0] = (mr & 0xffffu) | (mg << 16);
-        o32[1] = (mb & 0xffffu) | (mr & 0xffff0000u);
-        o32[2] = (mg >> 16) | (mb & 0xffff0000u);
-    }
-    else
-    {
-        o[0] = (unsigned short)(mr & 0xffffu);
-        o[1] = (unsigned short)(mg & 0xffffu);
-        o[2] = (unsigned short)(mb & 0xffffu);
-        if (two)
-        {
-            o[3] = (unsigned short)(mr >> 16);
-            o[4] = (unsigned short)(mg >> 16);
-            o[5] = (unsigned short)(mb >> 16);
-        }
+        auto load = [&](uint32_t (&v)[N]) {
+#pragma unroll
+            for (int i = 0; i < N; ++i)
+                v[i] = (i < stack_floor(N) || i < n) ? stack[(i * 3 + c) * kWmThreads + tid] : 0xffffffffu;
+        };
+        uint32_t v[N];
+        load(v);
+        const PairSums sc = c == 0 ? sums[0] : c == 1 ? sums[1] : sums[2];
+        const uint32_t m = median_pair<N>(v, n, inv, sigma, sc, load);
+        oa[c] = (unsigned short)(m & 0xffffu);
+        if (xb < dw) oa[96 + c] = (unsigned short)(m >> 16);
     }
 }
 
@@ -551,8 +600,10 @@ int launch_warp(const unsigned short* src, int sw, int sh, unsigned short* dst, 
     for (int i = 0; i < 9; ++i) P.H[i] = H[i];
     P.gain = gain;
     P.applyGain = gain_is_identity(gain) ? 0 : 1;
-    dim3 grid((dw + 31) / 32, (dh + 7) / 8);
-    k_warp<<<grid, dim3(32, 8), 0, s>>>(src, sw, sh, dst, dw, dh, offX, offY, P);
+    const WarpSource S = warp_source(src, sw, sh);
+    const dim3 grid((dw + 63) / 64, (dh + 7) / 8), block(32, 8);
+    if (homography_affine(H)) k_warp<true><<<grid, block, 0, s>>>(S, dst, dw, dh, offX, offY, P);
+    else k_warp<false><<<grid, block, 0, s>>>(S, dst, dw, dh, offX, offY, P);
     return check_launch("warp kernel");
 }
 
@@ -568,44 +619,51 @@ int launch_median(const unsigned short* const* inputs, int n, unsigned short* ou
         if (i < cnt) align |= reinterpret_cast<uintptr_t>(inputs[i]);
     }
     const long long total = (long long)w * h * 3;
-    if ((total & 1) == 0 && (align & 3) == 0)
-    {
-        const long long pairs = total >> 1;
-        const unsigned blocks = (unsigned)((pairs + 255) / 256);
-        uint32_t* o = reinterpret_cast<uint32_t*>(out);
-        if (cnt <= 4) k_median2<4><<<blocks, 256, 0, s>>>(in, cnt, pairs, sigma, o);
-        else if (cnt <= 8) k_median2<8><<<blocks, 256, 0, s>>>(in, cnt, pairs, sigma, o);
-        else if (cnt <= 16) k_median2<16><<<blocks, 256, 0, s>>>(in, cnt, pairs, sigma, o);
-        else k_median2<32><<<blocks, 256, 0, s>>>(in, cnt, pairs, sigma, o);
+    const unsigned blocks = (unsigned)(((total + 1) / 2 + 255) / 256);
+    const bool words = (align & 3) == 0;
+    const float inv = 1.0f / (float)cnt;
+#define I360B_MEDIAN(N)                                                              \
+    if (cnt <= N)                                                                    \
+    {                                                                                \
+        if (words) k_median<N, true><<<blocks, 256, 0, s>>>(in, cnt, inv, total, sigma, out); \
+        else k_median<N, false><<<blocks, 256, 0, s>>>(in, cnt, inv, total, sigma, out); \
+        return check_launch("median kernel");                                        \
     }
-    else
-    {
-        const unsigned blocks = (unsigned)((total + 255) / 256);
-        if (cnt <= 4) k_median1<4><<<blocks, 256, 0, s>>>(in, cnt, total, sigma, out);
-        else if (cnt <= 8) k_median1<8><<<blocks, 256, 0, s>>>(in, cnt, total, sigma, out);
-        else if (cnt <= 16) k_median1<16><<<blocks, 256, 0, s>>>(in, cnt, total, sigma, out);
-        else k_median1<32><<<blocks, 256, 0, s>>>(in, cnt, total, sigma, out);
-    }
-    return check_launch("median kernel");
+    I360B_STACK_SIZES(I360B_MEDIAN)
+#undef I360B_MEDIAN
+    return fail(I360B_INVALID_PARAM, "numInputs must be 1-32.");
 }
+
+namespace
+{
+template <int N>
+int run_warp_median(const StackParams& S, int cnt, int sw, int sh, unsigned short* out, int dw, int dh, int offX,
+                    int offY, float sigma, cudaStream_t s)
+{
+    const size_t smem = (size_t)cnt * 3 * kWmThreads * sizeof(uint32_t);  // at most 48 KB, at 32 frames
+    const unsigned grid = (unsigned)((dw + 63) / 64) * (unsigned)((dh + kWmThreads / 32 - 1) / (kWmThreads / 32));
+    k_warp_median<N><<<grid, dim3(32, kWmThreads / 32), smem, s>>>(S, cnt, 1.0f / (float)cnt, sw, sh, out, dw, dh, offX, offY, sigma);
+    return check_launch("warp + median kernel");
+}
+}  // namespace
 
 int launch_warp_median(const unsigned short* const* frames, int n, int sw, int sh, const float* H, unsigned short* out,
                        int dw, int dh, int offX, int offY, float sigma, cudaStream_t s)
 {
     StackParams S;
+    S.affine = 0;
     const int cnt = n < kMaxContributors ? n : kMaxContributors;
     for (int i = 0; i < kMaxContributors; ++i)
     {
         S.src[i] = i < cnt ? frames[i] : nullptr;
         for (int q = 0; q < 9; ++q) S.H[i][q] = i < cnt ? H[(size_t)i * 9 + q] : 0.0f;
+        if (i < cnt && homography_affine(S.H[i])) S.affine |= 1u << i;
     }
-    dim3 grid((unsigned)((dw + 63) / 64), (unsigned)((dh + 7) / 8));
-    dim3 block(32, 8);
-    if (cnt <= 4) k_warp_median<4><<<grid, block, 0, s>>>(S, cnt, sw, sh, out, dw, dh, offX, offY, sigma);
-    else if (cnt <= 8) k_warp_median<8><<<grid, block, 0, s>>>(S, cnt, sw, sh, out, dw, dh, offX, offY, sigma);
-    else if (cnt <= 16) k_warp_median<16><<<grid, block, 0, s>>>(S, cnt, sw, sh, out, dw, dh, offX, offY, sigma);
-    else k_warp_median<32><<<grid, block, 0, s>>>(S, cnt, sw, sh, out, dw, dh, offX, offY, sigma);
-    return check_launch("warp + median kernel");
+#define I360B_WARP_MEDIAN(N) \
+    if (cnt <= N) return run_warp_median<N>(S, cnt, sw, sh, out, dw, dh, offX, offY, sigma, s);
+    I360B_STACK_SIZES(I360B_WARP_MEDIAN)
+#undef I360B_WARP_MEDIAN
+    return fail(I360B_INVALID_PARAM, "numInputs must be 1-32.");
 }
 
 int launch_gain(unsigned short* data, long long n, float gain, cudaStream_t s)

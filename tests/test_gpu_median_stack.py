@@ -123,3 +123,58 @@ def test_warp_median_argument_errors(backend):
     assert backend.launch_warp_median([1] * 33, 10, 10, np.tile(np.eye(3), (33, 1, 1)), 1, 10, 10) == \
         ComputeResult.INVALID_PARAM
     assert backend.launch_warp_median([1], 0, 10, np.eye(3)[None], 1, 10, 10) == ComputeResult.INVALID_PARAM
+
+
+@pytest.mark.parametrize("n", range(1, 33))
+def test_median_every_stack_size_and_threshold(backend, oracle_c, n):
+    """Every sorting network, on an odd scalar count (the last scalar alone)
+    of full-range values, with thresholds that keep nothing (the reference
+    then keeps everything), one value, or all.  Exact."""
+    import torch
+    rng = np.random.default_rng(5000 + n)
+    w, h = 37, 11
+    ins = [rng.integers(0, 65536, (h, w, 3), dtype=np.uint16) for _ in range(n)]
+    for a in ins:
+        a[2] = 65535
+        a[3] = 40000 + rng.integers(0, 3)
+        a[4, ::2] = 0
+    d_in = [_dev(a) for a in ins]
+    for sigma in (2.0, 0.3, 0.0, -1.0, float("inf"), float("nan")):
+        d_out = torch.zeros((h, w, 3), dtype=torch.int16, device="cuda")
+        assert backend.launch_median([t.data_ptr() for t in d_in], w, h, d_out.data_ptr(), sigma) == 0
+        torch.cuda.synchronize()
+        assert np.array_equal(_host(d_out), oracle_c.median(ins, sigma)), sigma
+
+
+@pytest.mark.parametrize("sw,sh,dw,dh,shift,proj", [(2, 2, 5, 4, 0, False), (3, 5, 33, 9, 1, True),
+                                                    (64, 40, 64, 8, 0, False), (65, 41, 63, 17, 1, False),
+                                                    (66, 30, 129, 7, 1, True), (1, 7, 4, 4, 0, False)])
+def test_warp_taps_at_every_phase(backend, oracle_c, sw, sh, dw, dh, shift, proj):
+    """Taps read as aligned words: odd source widths and a source that starts
+    one sample past a word put the rows at both phases; destination widths
+    around the 64-pixel segment; affine and projective homographies; gains.
+    Full-range values.  Exact, alone and as a stack of two."""
+    import torch
+    rng = np.random.default_rng(sw * 100 + dw)
+    src = rng.integers(0, 65536, (sh, sw, 3), dtype=np.uint16)
+    src[0, 0] = 65535
+    src[-1, -1] = 65535
+    buf = torch.zeros(src.size + 1, dtype=torch.int16, device="cuda")
+    buf[shift:shift + src.size] = _dev(src).reshape(-1)
+    H = np.array([[0.93, 0.11, -1.25], [-0.08, 0.97, 0.75], [0, 0, 1]], np.float32)
+    if proj:
+        H[2] = [3e-4, -2e-4, 1.0001]
+    for off in ((0, 0), (-3, 2)):
+        ref = oracle_c.warp(src, dw, dh, H, *off)
+        for gain in (1.0, 1.37, 0.0, -1.0):
+            out = torch.full((dh, dw, 3), 9, dtype=torch.int16, device="cuda")
+            assert backend.launch_warp(buf.data_ptr() + 2 * shift, sw, sh, out.data_ptr(), dw, dh, H, *off,
+                                       gain=gain) == 0
+            torch.cuda.synchronize()
+            exp = ref if gain == 1.0 else oracle_c.gain(ref.copy(), gain).reshape(ref.shape)
+            assert np.array_equal(_host(out), exp), (off, gain)
+        out = torch.zeros((dh, dw, 3), dtype=torch.int16, device="cuda")
+        p = buf.data_ptr() + 2 * shift
+        assert backend.launch_warp_median([p, p], sw, sh, np.stack([H, H]), out.data_ptr(), dw, dh, *off) == 0
+        torch.cuda.synchronize()
+        assert np.array_equal(_host(out), ref)
