@@ -2,6 +2,7 @@
 // arithmetic of WindowsApp.Core/SourceFiles/SeamBlend.cpp in the same order,
 // so the GPU owner map and output are bit-identical to the CPU backend's.
 #include "blend_kernels.cuh"
+#include "warp_taps.cuh"
 
 #include <cuda/atomic>
 #include <cuda_fp16.h>
@@ -202,28 +203,6 @@ __device__ __forceinline__ void warp_zero_u16(unsigned short* p, int n, int lane
     if (lane < n - t0) p[t0 + lane] = 0;
 }
 
-// One destination pixel read straight from the source frame (the row-band
-// form below): the four taps by 2-byte loads through L1.
-__device__ __forceinline__ void warp_px(const WarpItem& it, float dX, const float* hy, unsigned short o[3])
-{
-    o[0] = o[1] = o[2] = 0;
-    int x0, y0;
-    float fx, fy;
-    if (!warp_pos(it, dX, hy, x0, y0, fx, fy)) return;
-    const unsigned short* r0 = it.src + ((size_t)y0 * it.srcW + x0) * 3;
-    const unsigned short* r1 = r0 + (size_t)it.srcW * 3;
-    unsigned short t00[3], t10[3], t01[3], t11[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-        t00[c] = __ldg(r0 + c);
-        t10[c] = __ldg(r0 + 3 + c);
-        t01[c] = __ldg(r1 + c);
-        t11[c] = __ldg(r1 + 3 + c);
-    }
-    warp_mix(it, fx, fy, t00, t10, t01, t11, o);
-}
-
 __device__ __forceinline__ WarpItem warp_item(const ItemDev& it)
 {
     WarpItem wi;
@@ -238,15 +217,16 @@ __device__ __forceinline__ WarpItem warp_item(const ItemDev& it)
 }
 
 // Row-band form (warp shape 0): a CTA makes a.bandRows full-width rows of one
-// contributor, each warp whole rows in 64-pixel segments with two pixels per
-// lane in flight, gathering taps from the frame through L1; rows and segments
+// contributor, each warp whole rows in 64-pixel segments, lane l the pixels l
+// and l + 32 as one paired computation (warp_taps.cuh), gathering taps from
+// the frame through L1; rows and segments
 // outside the frame's footprint box are written as zeros without evaluating
 // the mapping.  The warps take the band's rows interleaved (warp w: rows w,
 // w + 8, ...), so at any time the CTA's warps walk eight neighbouring rows
 // side by side and the source rows they share (a bilinear tap pair reads two
 // rows, each also read by the next output row) are reused from L1 rather
 // than fetched again from DRAM after the whole GPU has streamed past them.
-__global__ void __launch_bounds__(256, 8) k_warp_rows(BlendArgs a, const Unit* __restrict__ units)
+__global__ void __launch_bounds__(256, 5) k_warp_rows(BlendArgs a, const Unit* __restrict__ units)
 {
     const Unit u = units[blockIdx.x];
     const ItemDev& it = a.items[u.id];
@@ -254,6 +234,8 @@ __global__ void __launch_bounds__(256, 8) k_warp_rows(BlendArgs a, const Unit* _
     const int W = T.w, H = T.h, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned short* img = const_cast<unsigned short*>(it.img);
     const WarpItem wi = warp_item(it);
+    const WarpSource src = warp_source(wi.src, wi.srcW, wi.srcH);
+    const bool aff = homography_affine(wi.H);
     const int offX = it.offX, offY = it.offY, vx0 = it.vx0, vx1 = it.vx1, vy0 = it.vy0, vy1 = it.vy1;
     BoxAcc box;
     const int rowsPerWarp = a.bandRows >> 3;
@@ -282,23 +264,31 @@ __global__ void __launch_bounds__(256, 8) k_warp_rows(BlendArgs a, const Unit* _
         for (int x0 = s0; x0 < s1; x0 += 64)
         {
             const int xa = x0 + lane, xb = x0 + 32 + lane;
-            unsigned short oa[3] = {0, 0, 0}, ob[3] = {0, 0, 0};
-            if (xa < W && xa >= vx0 && xa <= vx1) warp_px(wi, (float)(xa + offX), hy, oa);
-            if (xb < W && xb >= vx0 && xb <= vx1) warp_px(wi, (float)(xb + offX), hy, ob);
-            const bool ca = (oa[0] | oa[1] | oa[2]) != 0, cb = (ob[0] | ob[1] | ob[2]) != 0;
+            const bool inA = xa < W && xa >= vx0 && xa <= vx1, inB = xb < W && xb >= vx0 && xb <= vx1;
+            f32x2 v[3];
+            if (aff) warp_pair23<true>(src, wi.H, hy, (float)(xa + offX), (float)(xb + offX), inA, inB, v);
+            else warp_pair23<false>(src, wi.H, hy, (float)(xa + offX), (float)(xb + offX), inA, inB, v);
+            uint32_t oa[3], ob[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+            {
+                if (wi.applyGain) v[c] = gain_pair23(v[c], wi.gain);
+                oa[c] = __float_as_uint(lo2(v[c]));
+                ob[c] = __float_as_uint(hi2(v[c]));
+            }
+            const bool ca = ((oa[0] | oa[1] | oa[2]) & 0xffffu) != 0, cb = ((ob[0] | ob[1] | ob[2]) & 0xffffu) != 0;
+            unsigned short* d = row + (size_t)xa * 3;
             if (xa < W)
             {
-                unsigned short* d = row + (size_t)xa * 3;
-                d[0] = oa[0];
-                d[1] = oa[1];
-                d[2] = oa[2];
+                d[0] = (unsigned short)oa[0];
+                d[1] = (unsigned short)oa[1];
+                d[2] = (unsigned short)oa[2];
             }
             if (xb < W)
             {
-                unsigned short* d = row + (size_t)xb * 3;
-                d[0] = ob[0];
-                d[1] = ob[1];
-                d[2] = ob[2];
+                d[96] = (unsigned short)ob[0];
+                d[97] = (unsigned short)ob[1];
+                d[98] = (unsigned short)ob[2];
             }
             const unsigned ma = __ballot_sync(kFull, ca), mb = __ballot_sync(kFull, cb);
             if (lane == 0)
