@@ -468,46 +468,103 @@ __global__ void __launch_bounds__(256) k_warp_tiles(BlendArgs a, const Unit* __r
 // upright+sqrt2) is a DAG with a unique solution, so any schedule that applies
 // the same rounded operations (min is exact and order-free) reproduces the CPU
 // result bit for bit.  Neighbours outside the tile are skipped by the
-// reference; here they are virtual cells of value +inf, which min() ignores
-// (inf + c = inf), so one uniform step serves every pixel.
+// reference.  Here they are virtual: above the first row +inf, which min()
+// ignores, and beside the tile (and below it, which the backward pass meets
+// first) ordinary cells without a seed.  Those change nothing: a path through
+// them can be pushed onto the tile's edge column, where a sideways step falls
+// away and a diagonal one becomes vertical, so each of its rounded sums is at
+// least the pushed path's (rounding is monotone), whose cells the recurrence
+// visits; and a value that comes from no seed is kInf + something, never below
+// a cell's own kInf.  So one uniform step serves every cell.
 //
-// Systolic wavefront: lane r of a warp owns row 32g + r and at step t
-// computes column x = t - 2r - 2, two columns behind the lane above.  The
-// value it needs from the row above at x+1 is the lane above's output of the
-// previous step and arrives by one __shfl_up_sync; the values at x and x-1
-// are the ones received one and two steps earlier.  Lane 0 takes its row
-// above from a shared-memory ring slot written by lane 31 of the previous row
-// group.  A warp runs kDtChunk steps between hand-offs: before a chunk, lane
-// 0 waits (bounded) until the previous group has published every column the
-// chunk reads; after it, lane 31 publishes how many columns of its row are
-// final.  The initial values of a chunk (one or two coverage words, or eight
-// pairs of the forward result) are loaded before its first step, and only
-// chunks that touch the tile's edges test cells for being virtual.  The
-// backward pass is the same code on mirrored coordinates with the forward
-// result as init.
+// Systolic wavefront: a warp owns a strip of 64 rows, lane q the rows 2q and
+// 2q + 1 of it, and at step t computes column t - 6q - 2 of the first and two
+// columns behind it of the second.  Every operand of a step is then a result
+// of an earlier one: the second row's from the same lane, one step old; the
+// first row's from the lane above, three steps old, so its shuffle has two
+// steps to arrive.  A step's dependency chain is one add and one minimum (of
+// three operands, an instruction of sm_100), and its two cells are
+// independent.  With a row per lane each step waited for a shuffle.
 //
-// Progress is published per row group (prog[g] = columns of row group g's
-// last row that are final), never per ring slot: group g + nslots reuses
-// group g's slot while group g + 1 may still be waiting for columns of group
-// g, so a per-slot counter would let g + nslots's progress release that wait
-// early.  The slot data itself is safe to reuse: a group runs a chunk only
-// when the group above has finished at least 64 further steps, so when group
-// g + nslots (nslots >= 2) writes column x of the slot, group g + 1 has run
-// more than 64 steps past the one where it read x.
+// Lane 0 takes its row above from a ring slot in shared memory, written by
+// lane 31 of the strip above.  A warp runs kDtChunk steps between hand-offs:
+// before a chunk, lane 0 waits (bounded) until the strip above has published
+// every column the chunk reads; after it, lane 31 publishes how many columns
+// of its last row are final.  What a chunk reads from memory is requested a
+// chunk ahead in one block: loads spread over the steps share scoreboards
+// with later ones and made every step wait for memory.
+//
+// The forward result is stored by anti-diagonal: the cells that a strip of n
+// rows computes in one step lie next to each other, row r of it at (t - 2) mod
+// W times n plus r (a row's W columns fall on W consecutive steps, so the
+// remainder is one-to-one for each row and the field needs no padding).  The
+// backward pass is the same code on mirrored coordinates, and the cells of one
+// of its steps are the cells of one forward step - column x of row (l, j)
+// belongs to step x + 6l + 2j + 2 forward and W + 191 minus that backward - so
+// it reads them back in the same whole lines.  Its own result goes through a
+// staging tile to row order, which the ownership kernel reads.
+//
+// Progress is published per strip (prog[g] = columns of strip g's last row
+// that are final), never per ring slot: strip g + nslots reuses strip g's
+// slot while strip g + 1 may still be waiting for columns of strip g, so a
+// per-slot counter would let g + nslots's progress release that wait early.
+// The slot data itself is safe to reuse: a strip runs at least 174 steps
+// behind the one above, so when strip g + nslots (nslots >= 2) writes column x
+// of the slot, at its step x + 190, strip g + 1 has passed the step x + 2
+// where it read x.
 // ---------------------------------------------------------------------------
-constexpr int kDtChunk = 16;  // steps between hand-offs
-constexpr int kDtRing = 4;    // row-group hand-off slots
-constexpr int kDtWarps = 16;  // warps per CTA
-constexpr int kDtStR = 20;    // staging row stride (floats): 16 columns + pad, 16-byte rows
-constexpr size_t kDtStageBytes = (size_t)kDtWarps * 32 * kDtStR * sizeof(float);
-// Ring slot: columns -4 .. W of a row (index = column + 4); columns < 0 and
-// column W hold +inf.
-__host__ __device__ __forceinline__ int dt_ring_stride(int W) { return (W + 8) & ~3; }
+constexpr int kDtChunk = 16;   // steps between hand-offs
+constexpr int kDtRing = 4;     // strip hand-off slots
+constexpr int kDtWarps = 12;   // warps per CTA at most (fewer where a wide row leaves no room, see launch_dt)
+constexpr int kDtStrip = 64;   // rows per strip
+constexpr int kDtLag = 190;    // step at which the last row of a strip computes its column 0
+constexpr int kDtStR = 20;     // staging row stride (floats): 16 columns + pad, 16-byte rows
+constexpr size_t kDtStageBytes = (size_t)kDtStrip * kDtStR * sizeof(float);  // per warp
+// Ring slot: a row from column -6 on (index = column + 6); columns outside
+// [0, W) hold +inf.
+__host__ __device__ __forceinline__ int dt_ring_stride(int W) { return (W + 16) & ~3; }
+
+// Stores to global memory through a pointer read from a descriptor: as generic
+// stores they could alias shared memory, and the staging reads below would
+// each wait for the store before it.
+__device__ __forceinline__ void st_global(float* p, float v)
+{
+    asm volatile("st.global.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v));
+}
+__device__ __forceinline__ void st_global(float* p, float a, float b)
+{
+    asm volatile("st.global.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(p)), "f"(a), "f"(b));
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// One row's state between steps: the value to the left, and the sums with the
+// row above that later steps use again (fadd(up, 1) is formed one step ahead;
+// the up-left sum is the up-right sum of two steps back).
+struct DtRow
+{
+    float left, up1, dg1, dg2;
+    // The minimum over the neighbours and init, given the row above at x + 1.
+    __device__ __forceinline__ float step(float upp1, float init)
+    {
+        const float dg = fadd(upp1, 1.41421356f);
+        const float v = min3(min3(up1, dg2, dg), fadd(left, 1.0f), init);
+        up1 = fadd(upp1, 1.0f);
+        dg2 = dg1;
+        dg1 = dg;
+        return v;
+    }
+};
 
 template <bool BACK>
-__global__ void __launch_bounds__(32 * kDtWarps, 2) k_dt(BlendArgs a, const int* __restrict__ itemList, int nslots)
+__global__ void __launch_bounds__(32 * kDtWarps, 1) k_dt(BlendArgs a, const int* __restrict__ itemList, int nslots)
 {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];
     const ItemDev& it = a.items[itemList[blockIdx.x]];
     const TileDev& T = a.tiles[it.tile];
     const int Wt = T.w, Ht = T.h, covWords = T.covWords;
@@ -531,59 +588,141 @@ __global__ void __launch_bounds__(32 * kDtWarps, 2) k_dt(BlendArgs a, const int*
     const int ry0 = max(it.bbox[1] - 1, 0), ry1 = min(it.bbox[3] + 1, Ht - 1);
     const int W = rx1 - rx0 + 1, H = ry1 - ry0 + 1;  // R's extent; the recurrence below runs on R
     const int RS = dt_ring_stride(W);
-    float* ring = smem + kDtStageBytes / sizeof(float);
+    const int nw = blockDim.x >> 5;
+    float* ring = smem + (size_t)nw * (kDtStageBytes / sizeof(float));
     int* prog = reinterpret_cast<int*>(ring + (size_t)nslots * RS);
     const float INF = f_inf();
-    const int nG = (H + 31) >> 5;
+    const int nG = (H + kDtStrip - 1) / kDtStrip;
     for (int i = threadIdx.x; i < nG; i += blockDim.x) prog[i] = -1;
-    for (int i = threadIdx.x; i < nslots * 5; i += blockDim.x)
-    {
-        const int sl = i / 5, e = i - sl * 5;
-        ring[(size_t)sl * RS + (e < 4 ? e : W + 4)] = INF;
-    }
+    for (int sl = 0; sl < nslots; ++sl)
+        for (int e = threadIdx.x; e < RS; e += blockDim.x)
+            if (e < 6 || e >= W + 6) ring[(size_t)sl * RS + e] = INF;
     __syncthreads();
     const float kInf = (float)(Wt + Ht);
-    const float kDiag = 1.41421356f;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nwarps = blockDim.x >> 5;
-    const float* src = BACK ? it.d1 : nullptr;
-    float* dst = BACK ? it.d : it.d1;
-    // 8-byte pairs of columns: even row length and 8-byte aligned buffers.
-    const bool pairs = (W & 1) == 0 && (Wt & 1) == 0 &&
-                       ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 7) == 0;
-    const int nSteps = W + 64;  // lane 31 computes column W - 1 at step W + 63
+    const int warp = threadIdx.x >> 5, q = threadIdx.x & 31;
+    const int nSteps = W + kDtLag;
+    const bool pairs = ((W | Wt) & 1) == 0 && (reinterpret_cast<uintptr_t>(it.d) & 7) == 0;
 
-    for (int g = warp; g < nG; g += nwarps)
+    for (int g = warp; g < nG; g += nw)
     {
-        const int vy = g * 32 + lane;  // row in the pass's (mirrored) order
-        const bool rowOk = vy < H;
-        const bool fullGroup = g * 32 + 31 < H;
-        const bool hasAbove = g > 0;  // lane 0's row above: the ring, else virtual
-        const int ty = rowOk ? (BACK ? ry1 - vy : ry0 + vy) : ry0;  // tile row
-        float* outRow = dst + (size_t)ty * Wt;
-        const float* inRow = BACK ? src + (size_t)ty * Wt : nullptr;
-        const uint32_t* covRow = it.cov + (size_t)ty * covWords;
-        // Staging rows of this warp: a chunk's 32 x 16 values cross between
-        // lanes (one row each) and 8-lane groups (one 64-byte row segment per
-        // global access) here.
-        float* st = smem + (size_t)warp * 32 * kDtStR;
-        const int sj = lane >> 3, sp = lane & 7;  // transposed role: rows sj + 4k, pair sp
-        float* ringOut = ring + (size_t)(g % nslots) * RS + 4;
-        const float* ringIn = ring + (size_t)((g + nslots - 1) % nslots) * RS + 4;
-        float left = INF, up0 = INF, upm1 = INF;  // own x-1; row above at x and x-1
-        int seen = -1;                            // lane 0: progress of the group above already observed
-        int wIdx = -4;                            // forward: coverage words wIdx .. wIdx+2 held
-        uint32_t wLo = 0, wHi = 0, wNx = 0;
-        // Interior chunk: every lane's row and columns lie in the tile, so no
-        // cell is virtual (but lane 0's row above, in group 0).
-        auto is_interior = [&](int c0) { return fullGroup && c0 - 64 >= 0 && c0 + kDtChunk - 2 <= W; };
+        const int s = BACK ? nG - 1 - g : g;  // the strip in tile order
+        const int rows = min(kDtStrip, H - kDtStrip * s);
+        const int l = BACK ? 31 - q : q;      // this lane's place in the strip, in tile order
+        // this lane's rows of R (first, second in the pass's order)
+        const int rA = kDtStrip * s + 2 * l + (BACK ? 1 : 0), rB = rA + (BACK ? -1 : 1);
+        const bool okA = rA < H, okB = rB < H;
+        const bool full = rows == kDtStrip;
+        const bool hasAbove = g > 0;
+        // the lane's pair of rows in the anti-diagonal field
+        float* const field = it.d1 + (size_t)kDtStrip * s * W + 2 * l;
+        const uint32_t* covA = it.cov + (size_t)(ry0 + (okA ? rA : 0)) * covWords;
+        const uint32_t* covB = it.cov + (size_t)(ry0 + (okB ? rB : 0)) * covWords;
+        const float* ringIn = ring + (size_t)((g + nslots - 1) % nslots) * RS;
+        float* ringOut = ring + (size_t)(g % nslots) * RS;
+        float* const st = smem + (size_t)warp * kDtStrip * kDtStR;  // this warp's staging tile
+
+        DtRow A{INF, INF, INF, INF}, B{INF, INF, INF, INF};
+        float prevA = INF, prevB = INF;  // the last step's results
+        float recv1 = INF, recv2 = INF;  // the lane above's second row, two and three steps old
+        int seen = -1;                   // lane 0: progress of the strip above already observed
+
+        // Bit i: cell i of a row's chunk (from column x on) lies in R.
+        auto valid_bits = [&](bool ok, int x) -> uint32_t {
+            const int b0 = min(max(-x, 0), 16), b1 = min(max(W - x, 0), 16);
+            return ok ? ((1u << b1) - 1u) & ~((1u << b0) - 1u) : 0u;
+        };
+        // Forward: the two coverage words that hold a chunk's 16 cells of a row.
+        auto cov_words = [&](const uint32_t* row, bool ok, int x, uint32_t& w0, uint32_t& w1) {
+            const int i = (rx0 + x) >> 5;
+            w0 = ok && i >= 0 && i < covWords ? __ldg(row + i) : 0u;
+            w1 = ok && i + 1 >= 0 && i + 1 < covWords ? __ldg(row + i + 1) : 0u;
+        };
+        uint32_t ca0 = 0, ca1 = 0, cb0 = 0, cb1 = 0;  // the next chunk's coverage words
+        float nextA[kDtChunk], nextB[kDtChunk];       // the next chunk's forward values
+        // Backward: the slot (time modulo W) of the next chunk's first step;
+        // it decreases.  Any slot of a valid row may be read, so cells outside
+        // R are sorted out by their valid bits, not here.
+        int m = (W + kDtLag - 1) % W;
+        auto fetch = [&](int t0) {
+            if (!BACK)
+            {
+                cov_words(covA, okA, t0 - 6 * q - 2, ca0, ca1);
+                cov_words(covB, okB, t0 - 6 * q - 4, cb0, cb1);
+            }
+            else if (m >= kDtChunk - 1)
+            {
+                const float* p = field + (ptrdiff_t)m * rows;
+                if (full)
+                {
+#pragma unroll
+                    for (int i = 0; i < kDtChunk; ++i)
+                    {
+                        const float2 v = __ldg(reinterpret_cast<const float2*>(p - i * kDtStrip));
+                        nextA[i] = v.y;  // (backward: the odd row comes first)
+                        nextB[i] = v.x;
+                    }
+                }
+                else
+                {
+#pragma unroll
+                    for (int i = 0; i < kDtChunk; ++i)
+                    {
+                        nextA[i] = nextB[i] = 0.0f;
+                        if (okA) nextA[i] = __ldg(p + 1);
+                        if (okB) nextB[i] = __ldg(p);
+                        p -= rows;
+                    }
+                }
+                m -= kDtChunk;
+                if (m < 0) m += W;
+            }
+            else
+            {
+#pragma unroll
+                for (int i = 0; i < kDtChunk; ++i)
+                {
+                    const float* p = field + (ptrdiff_t)m * rows;
+                    nextA[i] = nextB[i] = 0.0f;
+                    if (okA) nextA[i] = __ldg(p + 1);
+                    if (okB) nextB[i] = __ldg(p);
+                    m = m == 0 ? W - 1 : m - 1;
+                }
+            }
+        };
+        // Backward: the way of a staged chunk to row order.  Staging row
+        // 4k + sj is row j = k / 8 of lane qr = 4 (k % 8) + sj, row
+        // 64s + 63 - 2qr - j of R; the pair sp of its 16 columns lies at tile
+        // column rx1 - 13 - t0 + 6qr + 2j + 2sp.
+        const int sj = q >> 3, sp = q & 7;
+        const int rr = kDtStrip * s + kDtStrip - 1 - 2 * sj, mm = rx1 - 13 + 6 * sj + 2 * sp;
+        float* const dBase = it.d + (ptrdiff_t)(ry0 + rr) * Wt + mm;
+        const ptrdiff_t lane4 = 24 - (ptrdiff_t)8 * Wt;  // to the row of the lane four further
+
+        fetch(0);
         for (int t0 = 0; t0 < nSteps; t0 += kDtChunk)
         {
-            int bad = 0;
-            if (hasAbove && lane == 0)
+            uint32_t bitsA = 0, bitsB = 0;
+            float inA[kDtChunk], inB[kDtChunk];
+            if (BACK)
             {
-                // this chunk reads columns up to t0 + kDtChunk - 1 of the row above
-                const int need = min(t0 + kDtChunk, W);
+#pragma unroll
+                for (int i = 0; i < kDtChunk; ++i)
+                {
+                    inA[i] = nextA[i];
+                    inB[i] = nextB[i];
+                }
+            }
+            else
+            {
+                bitsA = __funnelshift_r(ca0, ca1, (rx0 + t0 - 6 * q - 2) & 31);
+                bitsB = __funnelshift_r(cb0, cb1, (rx0 + t0 - 6 * q - 4) & 31);
+            }
+            if (t0 + kDtChunk < nSteps) fetch(t0 + kDtChunk);
+            int bad = 0;
+            if (hasAbove && q == 0)
+            {
+                // this chunk reads columns up to t0 + kDtChunk - 2 of the row above
+                const int need = min(t0 + kDtChunk - 1, W);
                 if (seen < need)
                 {
                     cuda::atomic_ref<int, cuda::thread_scope_block> pr(prog[g - 1]);
@@ -591,7 +730,7 @@ __global__ void __launch_bounds__(32 * kDtWarps, 2) k_dt(BlendArgs a, const int*
                     int spins = 0;
                     while ((seen = pr.load(cuda::memory_order_acquire)) < need)
                     {
-                        if (++spins > 32) __nanosleep(128);
+                        if (++spins > 32) __nanosleep(64);
                         if (((spins & 63) == 0 || a.spinLimit == 0) &&
                             (*(volatile int*)a.error || clock64() - tstart > a.spinLimit))
                         {
@@ -604,220 +743,152 @@ __global__ void __launch_bounds__(32 * kDtWarps, 2) k_dt(BlendArgs a, const int*
                 }
             }
             if (__shfl_sync(kFull, bad, 0)) return;  // gave up waiting (error flag set)
-            const int xs = t0 - 2 * lane - 2;  // this lane's column at the chunk's first step
-            // Outside interior chunks cells outside the tile are +inf and never
-            // stored; with an even row length a column pair is in or out as a
-            // whole.  The backward pass takes its edge chunks cell by cell
-            // (fewer registers in its staged path).
-            const bool interior = is_interior(t0);
-            if (pairs && (!BACK || interior))
+            // Lane 0's row above: columns t0-1 .. t0+14 (entries t0+5 ..
+            // t0+20) of five 16-byte reads, the same for every lane (past the
+            // row's end the slot's last entries, +inf).
+            float ab[kDtChunk + 4];
+#pragma unroll
+            for (int i = 0; i < kDtChunk / 4 + 1; ++i)
             {
-                // The chunk's initial values enter, and its results leave, this
-                // lane's staging row in memory order (the backward pass's columns
-                // reversed), four at a time.
-                float* const cur = st;
-                float4* myRow = reinterpret_cast<float4*>(cur + lane * kDtStR);
-                uint32_t bits = 0;
-                __syncwarp();  // the previous chunk's row-segment reads are done
+                float4 v = make_float4(INF, INF, INF, INF);
+                if (hasAbove) v = reinterpret_cast<const float4*>(ringIn)[min((t0 >> 2) + 1 + i, (RS >> 2) - 1)];
+                ab[4 * i] = v.x;
+                ab[4 * i + 1] = v.y;
+                ab[4 * i + 2] = v.z;
+                ab[4 * i + 3] = v.w;
+            }
+            // Interior chunk: every lane's rows and columns lie in R.
+            const bool beforeEnd = t0 + kDtChunk - 2 <= W;
+            const bool interior = full && t0 >= kDtLag && beforeEnd;
+            uint32_t validA = 0xffffu, validB = 0xffffu;
+            if (!interior)
+            {
+                validA = valid_bits(okA, t0 - 6 * q - 2);
+                validB = valid_bits(okB, t0 - 6 * q - 4);
+                // cells outside R have no seed
+                bitsA |= ~validA;
+                bitsB |= ~validB;
                 if (BACK)
                 {
-                    // Row j's 16 values sit at tile columns rx1-15-xs_j .. rx1-xs_j
-                    // (mirrored); 8 lanes load each row as 8-byte pairs.
 #pragma unroll
-                    for (int k = 0; k < 8; ++k)
+                    for (int i = 0; i < kDtChunk; ++i)
                     {
-                        const int j = 4 * k + sj;
-                        const int vyj = g * 32 + j, m0 = rx1 - 15 - (t0 - 2 * j - 2) + 2 * sp;
-                        *reinterpret_cast<float2*>(cur + j * kDtStR + 2 * sp) =
-                            __ldg(reinterpret_cast<const float2*>(src + (size_t)(ry1 - vyj) * Wt + m0));
+                        inA[i] = ((validA >> i) & 1u) ? inA[i] : kInf;
+                        inB[i] = ((validB >> i) & 1u) ? inB[i] : kInf;
                     }
-                    __syncwarp();
                 }
-                else
+            }
+            float outA[kDtChunk], outB[kDtChunk];
+#pragma unroll
+            for (int i = 0; i < kDtChunk; ++i)
+            {
+                const float upA = q == 0 ? ab[i + 1] : recv2;
+                const float upB = prevA;
+                recv2 = recv1;
+                recv1 = __shfl_up_sync(kFull, prevB, 1);
+                float vA = A.step(upA, BACK ? inA[i] : kInf), vB = B.step(upB, BACK ? inB[i] : kInf);
+                if (!BACK)
                 {
-                    // Coverage words xs>>5 and the next, held across chunks (the
-                    // word after them loaded a chunk early).
-                    const int xa = rx0 + xs;  // tile column of the chunk's first step
-                    const int w0 = xa >> 5;
-                    if (w0 != wIdx)
-                    {
-                        if (w0 == wIdx + 1)
-                        {
-                            wLo = wHi;
-                            wHi = wNx;
-                        }
-                        else
-                        {
-                            wLo = w0 >= 0 && w0 < covWords ? __ldg(covRow + w0) : 0u;
-                            wHi = w0 + 1 >= 0 && w0 + 1 < covWords ? __ldg(covRow + w0 + 1) : 0u;
-                        }
-                        wNx = w0 + 2 >= 0 && w0 + 2 < covWords ? __ldg(covRow + w0 + 2) : 0u;
-                        wIdx = w0;
-                    }
-                    bits = __funnelshift_r(wLo, wHi, xa & 31);
+                    vA = ((bitsA >> i) & 1u) ? vA : 0.0f;
+                    vB = ((bitsB >> i) & 1u) ? vB : 0.0f;
                 }
-                // Lane 0's row above: columns t0-1 .. t0+14 (slot entries
-                // t0+3 .. t0+18) as five 16-byte reads, the same for every lane.
-                const float4* slot4 = reinterpret_cast<const float4*>(ringIn - 4) + (t0 >> 2);
-                // The chunk's initial values, four columns at a time.
-                auto chunk_in = [&](int m4, float in[4]) {
-                    if (BACK)
-                    {
-                        const float4 v = myRow[3 - m4];  // memory columns 12-4m4 .. 15-4m4
-                        in[0] = v.w;
-                        in[1] = v.z;
-                        in[2] = v.y;
-                        in[3] = v.x;
-                    }
-                    else
-                    {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) in[i] = ((bits >> (4 * m4 + i)) & 1u) ? kInf : 0.0f;
-                    }
-                };
-                auto chunk_out = [&](int m4, const float o[4]) {
-                    if (BACK) myRow[3 - m4] = make_float4(o[3], o[2], o[1], o[0]);
-                    else myRow[m4] = make_float4(o[0], o[1], o[2], o[3]);
-                };
-                if (interior)
+                A.left = prevA = outA[i] = vA;
+                B.left = prevB = outB[i] = vB;
+            }
+            const int xOut = t0 - kDtLag;  // the chunk's first column of the strip's last row
+            if (q == 31 && xOut > -kDtChunk)
+            {
+                if (xOut >= 0 && xOut + kDtChunk <= W)
                 {
-                    // Every cell of the chunk is in the tile.  The sums with the
-                    // row above are carried between steps: fadd(up0, 1) is formed
-                    // one step ahead, and fadd(upm1, kDiag) is the fadd(upp1,
-                    // kDiag) of two steps back (the same operands, so the same
-                    // value).  min is exact in any order, so the candidates known
-                    // early are combined first and a step's dependency chain is
-                    // the shuffle, one add and two mins.  Lane 0 of group 0 has no
-                    // row above (+inf).
-                    const float4 inf4 = make_float4(INF, INF, INF, INF);
-                    float prevW = hasAbove ? slot4[0].w : INF;
-                    float up1 = fadd(up0, 1.0f), dg1 = fadd(up0, kDiag), dg2 = fadd(upm1, kDiag);
-                    float u1 = up0, u2 = upm1;  // the row above at x and x - 1 after the chunk
+                    float4* o = reinterpret_cast<float4*>(ringOut + xOut + 6);
 #pragma unroll
-                    for (int m4 = 0; m4 < kDtChunk / 4; ++m4)
-                    {
-                        float in[4], o[4];
-                        chunk_in(m4, in);
-                        const float4 blk = hasAbove ? slot4[m4 + 1] : inf4;
-                        const float above[4] = {prevW, blk.x, blk.y, blk.z};
-                        prevW = blk.w;
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                        {
-                            const float recv = __shfl_up_sync(kFull, left, 1);
-                            const float upp1 = lane == 0 ? above[i] : recv;
-                            const float dg = fadd(upp1, kDiag);
-                            float av = fminf(fminf(in[i], up1), dg2);
-                            av = fminf(av, dg);
-                            av = fminf(av, fadd(left, 1.0f));
-                            up1 = fadd(upp1, 1.0f);
-                            dg2 = dg1;
-                            dg1 = dg;
-                            u2 = u1;
-                            u1 = upp1;
-                            left = av;
-                            o[i] = av;
-                        }
-                        chunk_out(m4, o);
-                    }
-                    up0 = u1;
-                    upm1 = u2;
+                    for (int i = 0; i < kDtChunk / 4; ++i)
+                        o[i] = make_float4(outB[4 * i], outB[4 * i + 1], outB[4 * i + 2], outB[4 * i + 3]);
                 }
                 else
                 {
 #pragma unroll
-                    for (int m4 = 0; m4 < kDtChunk / 4; ++m4)
-                    {
-                        float in[4], o[4];
-                        chunk_in(m4, in);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                        {
-                            const int x = xs + 4 * m4 + i;
-                            const bool ok = rowOk && x >= 0 && x < W;
-                            const float recv = __shfl_up_sync(kFull, left, 1);
-                            // lane 0 reads columns >= -1 of the row above (the ring
-                            // holds +inf outside [0, W)); group 0 has no row above
-                            float upp1 = recv;
-                            if (lane == 0) upp1 = hasAbove ? ringIn[min(max(x + 1, -1), W)] : INF;
-                            float av = fminf(in[i], fadd(up0, 1.0f));
-                            av = fminf(av, fadd(upm1, kDiag));
-                            av = fminf(av, fadd(upp1, kDiag));
-                            av = fminf(av, fadd(left, 1.0f));
-                            const float d = ok ? av : INF;
-                            upm1 = up0;
-                            up0 = upp1;
-                            left = d;
-                            o[i] = d;
-                        }
-                        chunk_out(m4, o);
-                    }
+                    for (int i = 0; i < kDtChunk; ++i)
+                        if (xOut + i >= 0 && xOut + i < W) ringOut[xOut + i + 6] = outB[i];
                 }
-                // 64-byte row segments to the output.
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < 8; ++k)
+                // how many columns of the strip's last row are final
+                cuda::atomic_ref<int, cuda::thread_scope_block> pr(prog[g]);
+                pr.store(min(xOut + kDtChunk, W), cuda::memory_order_release);
+            }
+            if (!BACK)
+            {
+                if (beforeEnd)
                 {
-                    const int j = 4 * k + sj;
-                    const int vyj = g * 32 + j, xsj = t0 - 2 * j - 2;
-                    const float2 v = *reinterpret_cast<const float2*>(cur + j * kDtStR + 2 * sp);
-                    if (BACK)
+                    // Slot t0 - 2 + i without wrapping.  A cell left of R is
+                    // stored too: the cell that owns its slot comes W steps
+                    // later, from the same lane.
+                    float* p = field + (ptrdiff_t)(t0 - 2) * rows;
+                    if (full)
                     {
-                        const int m0 = rx1 - 15 - xsj + 2 * sp;  // chunk columns xs_j+15-2sp, xs_j+14-2sp
-                        if (interior || (vyj < H && m0 >= rx0 && m0 < rx1))
-                        {
-                            *reinterpret_cast<float2*>(dst + (size_t)(ry1 - vyj) * Wt + m0) = v;
-                            if (j == 31) *reinterpret_cast<float2*>(ringOut + xsj + 14 - 2 * sp) = make_float2(v.y, v.x);
-                        }
+#pragma unroll
+                        for (int i = 0; i < kDtChunk; ++i)
+                            if (i >= 2 || t0 > 0) st_global(p + i * kDtStrip, outA[i], outB[i]);
                     }
                     else
                     {
-                        const int c0 = xsj + 2 * sp;
-                        if (interior || (vyj < H && c0 >= 0 && c0 < W))
+#pragma unroll
+                        for (int i = 0; i < kDtChunk; ++i)
                         {
-                            *reinterpret_cast<float2*>(dst + (size_t)(ry0 + vyj) * Wt + rx0 + c0) = v;
-                            if (j == 31) *reinterpret_cast<float2*>(ringOut + c0) = v;
+                            if (okA && (i >= 2 || t0 > 0)) st_global(p, outA[i]);
+                            if (okB && (i >= 2 || t0 > 0)) st_global(p + 1, outB[i]);
+                            p += rows;
                         }
+                    }
+                }
+                else
+                {
+                    int slot = (t0 + W - 2) % W;  // (W > 1, or t0 >= 2)
+#pragma unroll
+                    for (int i = 0; i < kDtChunk; ++i)
+                    {
+                        float* p = field + (ptrdiff_t)slot * rows;
+                        if ((validA >> i) & 1u) st_global(p, outA[i]);
+                        if ((validB >> i) & 1u) st_global(p + 1, outB[i]);
+                        slot = slot + 1 == W ? 0 : slot + 1;
                     }
                 }
             }
             else
             {
+                // The chunk's row segments to the staging tile: the first rows
+                // in staging rows 0..31, the second rows in 32..63 (16-byte
+                // stores without bank conflicts), values in memory order (the
+                // pass's columns reversed); then 8 lanes per segment.
+                __syncwarp();  // the previous chunk's reads are done
+                float4* ra = reinterpret_cast<float4*>(st + q * kDtStR);
+                float4* rb = reinterpret_cast<float4*>(st + (32 + q) * kDtStR);
 #pragma unroll
-                for (int q = 0; q < kDtChunk; ++q)
+                for (int i = 0; i < kDtChunk / 4; ++i)
                 {
-                    const int x = xs + q;
-                    const bool ok = rowOk && x >= 0 && x < W;
-                    float iv = INF;
-                    if (ok)
-                        iv = BACK ? __ldg(inRow + (rx1 - x))
-                                  : (((__ldg(covRow + ((rx0 + x) >> 5)) >> ((rx0 + x) & 31)) & 1u) ? kInf : 0.0f);
-                    const float recv = __shfl_up_sync(kFull, left, 1);
-                    // lane 0 reads columns >= -1 of the row above (ring holds +inf
-                    // outside [0, W)); group 0 has no row above
-                    float upp1 = recv;
-                    if (lane == 0) upp1 = hasAbove ? ringIn[min(max(x + 1, -1), W)] : INF;
-                    float av = fminf(iv, fadd(up0, 1.0f));
-                    av = fminf(av, fadd(upm1, kDiag));
-                    av = fminf(av, fadd(upp1, kDiag));
-                    av = fminf(av, fadd(left, 1.0f));
-                    const float d = ok ? av : INF;
-                    upm1 = up0;
-                    up0 = upp1;
-                    left = d;
-                    if (ok)
+                    ra[3 - i] = make_float4(outA[4 * i + 3], outA[4 * i + 2], outA[4 * i + 1], outA[4 * i]);
+                    rb[3 - i] = make_float4(outB[4 * i + 3], outB[4 * i + 2], outB[4 * i + 1], outB[4 * i]);
+                }
+                __syncwarp();
+                float2 v[kDtStrip / 4];
+#pragma unroll
+                for (int k = 0; k < kDtStrip / 4; ++k)
+                    v[k] = *reinterpret_cast<const float2*>(st + (4 * k + sj) * kDtStR + 2 * sp);
+#pragma unroll
+                for (int k = 0; k < kDtStrip / 4; ++k)
+                {
+                    const int kl = k & 7, j = k >> 3;
+                    float* o = dBase - t0 + kl * lane4 + (j ? 2 - (ptrdiff_t)Wt : 0);
+                    const int r = rr - 8 * kl - j, m0 = mm - t0 + 24 * kl + 2 * j;
+                    if (pairs)
                     {
-                        outRow[BACK ? rx1 - x : rx0 + x] = d;
-                        if (lane == 31) ringOut[x] = d;
+                        if (interior || (r < H && m0 >= rx0 && m0 < rx1)) st_global(o, v[k].x, v[k].y);
+                    }
+                    else
+                    {
+                        if (r < H && m0 >= rx0 && m0 <= rx1) st_global(o, v[k].x);
+                        if (r < H && m0 + 1 >= rx0 && m0 + 1 <= rx1) st_global(o + 1, v[k].y);
                     }
                 }
-            }
-            // Lane 31 publishes how many columns of its row are final.
-            if (lane == 31)
-            {
-                const int done = min(max(t0 - 64 + kDtChunk, 0), W);
-                cuda::atomic_ref<int, cuda::thread_scope_block> pr(prog[g]);
-                pr.store(done, cuda::memory_order_release);
             }
         }
     }
@@ -3268,10 +3339,12 @@ size_t dt_prog_bytes(int maxH) { return (size_t)(((maxH + 31) >> 5) + 1) * sizeo
 
 int dt_rows_in_flight(int maxW, int maxH)
 {
-    const size_t row = (size_t)dt_ring_stride(maxW) * sizeof(float);
-    const size_t fixed = dt_prog_bytes(maxH) + kDtStageBytes;
+    // (counted by a row of W + 8 floats and 40 KB of staging; launch_dt takes
+    // the warps that fit beside the slots)
+    const size_t row = (size_t)((maxW + 8) & ~3) * sizeof(float);
+    const size_t fixed = dt_prog_bytes(maxH) + 40 * 1024;
     auto fit = [&](size_t budget) { return budget > fixed ? (int)((budget - fixed) / row) : 0; };
-    int n = fit(110 * 1024);  // two CTAs per SM
+    int n = fit(110 * 1024);
     if (n < 2) n = fit(220 * 1024);
     return n > kDtRing ? kDtRing : n;
 }
@@ -3304,17 +3377,20 @@ int launch_dt(const BlendArgs& a, const int* itemList, int n, bool backward, int
     if (slotsWanted >= 2 && slotsWanted < slots) slots = slotsWanted;
     if (slots < 2)
         return fail(I360B_NOT_SUPPORTED, "Chunk %dx%d exceeds the distance-transform row ring.", maxW, maxH);
-    size_t smem = kDtStageBytes + (size_t)slots * dt_ring_stride(maxW) * sizeof(float) + dt_prog_bytes(maxH);
-    if (backward)
-    {
-        cudaFuncSetAttribute(k_dt<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_dt<true><<<n, 32 * kDtWarps, smem, s>>>(a, itemList, slots);
-    }
-    else
-    {
-        cudaFuncSetAttribute(k_dt<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_dt<false><<<n, 32 * kDtWarps, smem, s>>>(a, itemList, slots);
-    }
+    // 12 warps of 168 registers, one CTA per SM: with 128 registers (16 warps,
+    // or two CTAs of 8) the backward pass serialises its block loads.  On the
+    // 90-tile panorama forward + backward 0.80 + 1.40 ms (a row per lane:
+    // 1.31 + 2.33), 16 warps 0.82 + 1.70, 8 warps 0.99 + 1.44, two CTAs of 8
+    // 0.95 + 1.61; one 2048 x 2048 chunk of 4 contributors 307 + 505 us (437 +
+    // 983).  Spreading a contributor over a cluster of 2-8 CTAs was slower:
+    // the hand-off's release then waits for the strip's stores to reach L2.
+    const size_t fixed = (size_t)slots * dt_ring_stride(maxW) * sizeof(float) + dt_prog_bytes(maxH);
+    int warps = kDtWarps;
+    while (warps > 1 && fixed + warps * kDtStageBytes > 224 * 1024) --warps;
+    const size_t smem = fixed + warps * kDtStageBytes;
+    auto* kernel = backward ? k_dt<true> : k_dt<false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kernel<<<n, 32 * warps, smem, s>>>(a, itemList, slots);
     return check_launch("distance transform kernel");
 }
 

@@ -280,3 +280,25 @@ def test_blend_seam_dp_value_ranges(backend, oracle_c, hi, noise):
         assert backend.blend_chunk_contributors(bufs, ww, hh, out, 4) == ComputeResult.SUCCESS, backend.get_last_error()
         ref = oracle_c.blend(bufs, 4)
         assert np.array_equal(out, ref), (hi, noise, int(np.abs(out.astype(int) - ref).max()))
+
+
+@pytest.mark.parametrize("w,h", [(1, 70), (2, 64), (7, 129), (31, 65), (33, 63), (40, 128), (203, 66), (206, 193),
+                                 (222, 64), (389, 130), (150, 770)])
+def test_blend_chamfer_strip_edges(backend, oracle_c, w, h):
+    """Chunks around the chamfer's 64-row strips, its 16-step chunks and the
+    190 steps that a strip's last row lags (one strip, a partial last strip of
+    one row, rows narrower than a chunk, more strips than warps): scattered
+    holes make every distance matter.  Exact: owner-dependent output."""
+    rng = np.random.default_rng(w * 1000 + h)
+    bufs = []
+    for k in range(3):
+        b = rng.integers(1, 16384, (h, w, 3)).astype(np.uint16)
+        b[rng.random((h, w)) < (0.002, 0.02, 0.2)[k]] = 0
+        if k == 1:
+            b[:, : w // 4] = 0
+        if k == 2:
+            b[: h // 3] = 0
+        bufs.append(b)
+    out = np.zeros((h, w, 3), np.uint16)
+    assert backend.blend_chunk_contributors(bufs, w, h, out, 4) == ComputeResult.SUCCESS, backend.get_last_error()
+    assert np.array_equal(out, oracle_c.blend(bufs, 4))
