@@ -184,6 +184,9 @@ extern "C" void i360b_shutdown(void)
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_init.load()) return;
     cudaDeviceSynchronize();
+    // give the pool's unused memory back
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, g_device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     g_generation.fetch_add(1);
     g_init.store(false);
 }

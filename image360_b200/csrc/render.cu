@@ -99,6 +99,11 @@ __global__ void k_setup_items(ItemDev* items, const double* toCanvas, const int*
     }
 }
 
+// Scratch of a one-chunk blend up to this size comes from the pool, which
+// keeps it (i360b_shutdown gives it back); larger scratch is allocated and
+// freed by the call.  A 4096 x 4096 chunk of 8 contributors needs 2.6 GB.
+constexpr size_t kPooledArenaMax = size_t(4) << 30;
+
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 __global__ void k_count_cov(const ItemDev* items, const TileDev* tiles, int n, unsigned long long* out)
@@ -115,7 +120,7 @@ __global__ void k_count_cov(const ItemDev* items, const TileDev* tiles, int n, u
 }  // namespace
 
 int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPath, void* extArena, size_t extBytes,
-                cudaStream_t stream)
+                cudaStream_t stream, bool oneShot)
 {
     render = renderPath;
     nTiles = (int)specs.size();
@@ -237,6 +242,7 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
     balanced_chains();
     // ---- work lists -------------------------------------------------------
     std::vector<Unit> units;
+    if (!oneShot)
     {
         // the largest list any band height and warp form needs
         const int shape = warpShape;
@@ -251,6 +257,7 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
         unitCap = (int)cap;
     }
     make_units(bandRows, units);
+    if (oneShot) unitCap = (int)units.size();
     std::vector<int> ints;
     const int seamStart = chain_lists(ints);
     if (nChains > 1)
@@ -279,6 +286,12 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
                         extBytes);
         arena = extArena;
         ownsArena = false;
+    }
+    else if (oneShot && bytes <= kPooledArenaMax)
+    {
+        I360B_TRY(dev_alloc(&arena, bytes, stream, "render plan"));
+        poolStream = stream;
+        pooled = true;
     }
     else
     {
@@ -327,35 +340,23 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
     dError = reinterpret_cast<int*>(base + metaOff + unitBytes + intBytes + itemBytes + tileBytes);
     dSeamCycles = reinterpret_cast<unsigned long long*>(base + metaOff + unitBytes + intBytes + itemBytes + tileBytes + 256);
     dSeamTile = reinterpret_cast<unsigned long long*>(base + metaOff + unitBytes + intBytes + itemBytes + tileBytes + 512);
-    if (extArena)
+    // The tables lie next to each other (unused list capacity, then zeroed
+    // flags and counters included): one upload.
     {
-        // Caller-provided scratch: upload the tables on the caller's stream
-        // (the scratch may still be in use by earlier work on that stream).
-        I360B_CUDA(cudaMemcpyAsync(dUnits, units.data(), units.size() * sizeof(Unit), cudaMemcpyHostToDevice, stream),
-                   "plan upload");
-        I360B_CUDA(cudaMemcpyAsync(dInts, ints.data(), ints.size() * sizeof(int), cudaMemcpyHostToDevice, stream),
-                   "plan upload");
-        if (nItems)
-            I360B_CUDA(cudaMemcpyAsync(dItems, items.data(), nItems * sizeof(ItemDev), cudaMemcpyHostToDevice, stream),
-                       "plan upload");
-        if (nTiles)
-            I360B_CUDA(cudaMemcpyAsync(dTiles, tiles.data(), nTiles * sizeof(TileDev), cudaMemcpyHostToDevice, stream),
-                       "plan upload");
-        I360B_CUDA(cudaMemsetAsync(dError, 0, 2 * sizeof(int), stream), "plan upload");
-        I360B_CUDA(cudaMemsetAsync(dSeamCycles, 0, 5 * sizeof(unsigned long long), stream), "plan upload");
-        I360B_CUDA(cudaMemsetAsync(dSeamTile, 0, std::max(nTiles, 1) * sizeof(unsigned long long), stream),
-                   "plan upload");
-        I360B_CUDA(cudaStreamSynchronize(stream), "plan upload");
-    }
-    else
-    {
-        I360B_CUDA(cudaMemcpy(dUnits, units.data(), units.size() * sizeof(Unit), cudaMemcpyHostToDevice), "plan upload");
-        I360B_CUDA(cudaMemcpy(dInts, ints.data(), ints.size() * sizeof(int), cudaMemcpyHostToDevice), "plan upload");
-        if (nItems) I360B_CUDA(cudaMemcpy(dItems, items.data(), nItems * sizeof(ItemDev), cudaMemcpyHostToDevice), "plan upload");
-        if (nTiles) I360B_CUDA(cudaMemcpy(dTiles, tiles.data(), nTiles * sizeof(TileDev), cudaMemcpyHostToDevice), "plan upload");
-        I360B_CUDA(cudaMemset(dError, 0, 2 * sizeof(int)), "plan upload");
-        I360B_CUDA(cudaMemset(dSeamCycles, 0, 5 * sizeof(unsigned long long)), "plan upload");
-        I360B_CUDA(cudaMemset(dSeamTile, 0, std::max(nTiles, 1) * sizeof(unsigned long long)), "plan upload");
+        const size_t metaBytes = bytes - metaOff;
+        std::vector<char> meta(metaBytes, 0);
+        char* m = meta.data();
+        if (!units.empty()) std::memcpy(m, units.data(), units.size() * sizeof(Unit));
+        if (!ints.empty()) std::memcpy(m + unitBytes, ints.data(), ints.size() * sizeof(int));
+        if (nItems) std::memcpy(m + unitBytes + intBytes, items.data(), nItems * sizeof(ItemDev));
+        if (nTiles) std::memcpy(m + unitBytes + intBytes + itemBytes, tiles.data(), nTiles * sizeof(TileDev));
+        // Scratch that is the caller's or the pool's may still be in use by
+        // earlier work on the caller's stream; the copy from pageable memory
+        // returns once the source has been read.
+        if (extArena || pooled)
+            I360B_CUDA(cudaMemcpyAsync(base + metaOff, m, metaBytes, cudaMemcpyHostToDevice, stream), "plan upload");
+        else
+            I360B_CUDA(cudaMemcpy(base + metaOff, m, metaBytes, cudaMemcpyHostToDevice), "plan upload");
     }
     seamList = dInts + seamStart;
     return I360B_SUCCESS;
@@ -633,7 +634,8 @@ Plan::~Plan()
     if (graphExec) cudaGraphExecDestroy(graphExec);
     if (graph) cudaGraphDestroy(graph);
     if (hostErr) cudaFreeHost(hostErr);
-    if (arena && ownsArena) cudaFree(arena);
+    if (arena && pooled) dev_free(arena, poolStream);
+    else if (arena && ownsArena) cudaFree(arena);
 }
 
 // Stages 5-9 with the fused pyramid (depth 2): level 0 -> 2 of every
@@ -933,6 +935,16 @@ done:
     return rc;
 }
 
+// Waits for a one-chunk plan's run and reports a kernel that gave up.
+static int chunk_status(const Plan& p, cudaStream_t s)
+{
+    int flag = 0;
+    I360B_CUDA(cudaMemcpyAsync(&flag, p.dError + 1, sizeof(int), cudaMemcpyDeviceToHost, s), "error flag readback");
+    I360B_CUDA(cudaStreamSynchronize(s), "blend synchronize");
+    if (flag) return fail(I360B_KERNEL_LAUNCH_FAILED, "A blend kernel gave up waiting (bounded spin); output invalid.");
+    return I360B_SUCCESS;
+}
+
 int launch_blend_chunk(const unsigned short* const* warped, int k, int w, int h, int bands, unsigned short* out,
                        cudaStream_t s)
 {
@@ -946,10 +958,14 @@ int launch_blend_chunk(const unsigned short* const* warped, int k, int w, int h,
         it.img = warped[i];
         specs[0].items.push_back(it);
     }
+    // One chunk, run once: the scratch comes from the stream-ordered pool
+    // (cudaMalloc and cudaFree synchronise the device and took 0.5 to 5 ms a
+    // call), and the status of the bounded waits is read without a pinned
+    // staging buffer.
     Plan p;
-    I360B_TRY(p.build(specs, bands, false));
-    I360B_TRY(p.execute(s, false));
-    return p.check(s);
+    I360B_TRY(p.build(specs, bands, false, nullptr, 0, s, true));
+    I360B_TRY(p.enqueue(s));
+    return chunk_status(p, s);
 }
 
 int launch_blend_chunk_in(void* arena, size_t arenaBytes, const unsigned short* const* warped, int k, int w, int h,
@@ -968,12 +984,7 @@ int launch_blend_chunk_in(void* arena, size_t arenaBytes, const unsigned short* 
     Plan p;
     I360B_TRY(p.build(specs, bands, false, arena, arenaBytes, s));
     I360B_TRY(p.enqueue(s));
-    // Status of the bounded waits, read without a pinned staging buffer.
-    int flag = 0;
-    I360B_CUDA(cudaMemcpyAsync(&flag, p.dError + 1, sizeof(int), cudaMemcpyDeviceToHost, s), "error flag readback");
-    I360B_CUDA(cudaStreamSynchronize(s), "blend synchronize");
-    if (flag) return fail(I360B_KERNEL_LAUNCH_FAILED, "A blend kernel gave up waiting (bounded spin); output invalid.");
-    return I360B_SUCCESS;
+    return chunk_status(p, s);
 }
 }  // namespace i360b
 

@@ -126,10 +126,13 @@ struct Plan
 
     // With extArena non-null the plan lives in that caller-provided device
     // buffer of extBytes bytes (no allocation; INVALID_PARAM if too small)
-    // and its tables are uploaded on stream `s`.
+    // and its tables are uploaded on stream `s`.  oneShot: the plan runs once
+    // on `s` and is not retuned; its scratch is taken from and returned to
+    // the stream-ordered pool.
     int build(const std::vector<TileSpec>& specs, int numBands, bool renderPath, void* extArena = nullptr,
-              size_t extBytes = 0, cudaStream_t s = nullptr);
-    bool ownsArena = true;
+              size_t extBytes = 0, cudaStream_t s = nullptr, bool oneShot = false);
+    bool ownsArena = true, pooled = false;
+    cudaStream_t poolStream = nullptr;
     // Enqueues the kernel sequence; with `ev` non-null records ev[i] before
     // stage i and ev[kStages] at the end (stage order of kStageNames).
     int enqueue(cudaStream_t s, cudaEvent_t* ev = nullptr);
