@@ -302,3 +302,27 @@ def test_blend_chamfer_strip_edges(backend, oracle_c, w, h):
     out = np.zeros((h, w, 3), np.uint16)
     assert backend.blend_chunk_contributors(bufs, w, h, out, 4) == ComputeResult.SUCCESS, backend.get_last_error()
     assert np.array_equal(out, oracle_c.blend(bufs, 4))
+
+
+@pytest.mark.parametrize("w,h", [(96, 80), (128, 200), (333, 97), (97, 333), (160, 160)])
+def test_blend_seam_many_contributors(backend, oracle_c, w, h):
+    """Seven overlapping rectangles in a ring and one across all of them: pairs
+    that own no common line, pairs whose owned boxes meet only after an
+    earlier pair's reassignment, row and column scans, row pitches that are
+    and are not a multiple of 16.  Exact."""
+    rng = np.random.default_rng(w * 7 + h)
+    base = rng.integers(2000, 6000, (h, w, 3))
+    bufs = []
+    for k in range(7):
+        cx, cy = w * (0.5 + 0.36 * np.cos(k * 0.9)), h * (0.5 + 0.36 * np.sin(k * 0.9))
+        hw, hh = w * rng.uniform(0.2, 0.32), h * rng.uniform(0.2, 0.32)
+        yy, xx = np.mgrid[0:h, 0:w]
+        inside = (abs(xx - cx + 0.1 * (yy - cy)) < hw) & (abs(yy - cy) < hh)
+        b = np.clip(base + rng.integers(-400, 400, (h, w, 3)), 1, 65535)
+        bufs.append(np.where(inside[..., None], b, 0).astype(np.uint16))
+    bar = np.zeros((h, w, 3), np.uint16)
+    bar[h // 3: h // 2] = rng.integers(1, 9000, (h // 2 - h // 3, w, 3))
+    bufs.insert(3, bar)
+    out = np.zeros((h, w, 3), np.uint16)
+    assert backend.blend_chunk_contributors(bufs, w, h, out, 4) == ComputeResult.SUCCESS, backend.get_last_error()
+    assert np.array_equal(out, oracle_c.blend(bufs, 4))
