@@ -16,11 +16,10 @@
 // TMEM, two slots so the epilogue of one tile overlaps the MMAs of the next,
 // and halos are double-buffered with cp.async so the next load overlaps both.
 //
-// Weight gradient: D[(tap, cin)][cout] += X[pixel + tap][cin] * G[pixel][cout]
-// summed over pixels (K), with both operands MN-major (the 8 channels of a
-// pixel are the contiguous 16 bytes); each CTA owns a 128-row chunk of
-// (tap, cin) and a slice of the pixels, and writes an fp32 partial that a
-// small kernel reduces.
+// Weight gradient: D[(dy, cin)][(dx, cout)] += X[q + dy][cin] * G[q - dx][cout]
+// summed over pixels q (K), all nine taps in one MMA per 16 pixels; each CTA
+// owns a share of the pixels and writes fp32 partial sums that a small kernel
+// reduces (see k_conv3x3_wgrad).
 #include "common.cuh"
 #include "render_plan.hpp"
 #include "tc_common.cuh"
@@ -43,7 +42,7 @@ namespace
 {
 using bf16 = __nv_bfloat16;
 
-constexpr int kTileX = 128;                // pixels per weight-gradient tile (one row)
+constexpr int kTileX = 128;                // weight-gradient widths are multiples of this
 constexpr long long kWaitSpins = 1ll << 26;  // bounded mbarrier waits
 constexpr int kSlots = 4;
 constexpr float kInScale = 1.0f / 32768.0f;
@@ -142,18 +141,6 @@ __device__ __forceinline__ void unpack8_bf16(uint4 q, float* v)
         v[2 * i] = f.x;
         v[2 * i + 1] = f.y;
     }
-}
-
-// Source of one 16-byte (8-channel) chunk of the convolution input at (img,
-// yy, xx); yy, xx inside the image.
-template <int CIN, int LD>
-__device__ __forceinline__ const bf16* input_chunk(const bf16* x, const bf16* u, int cs, int h, int w, int img, int yy,
-                                                   int xx, int c8)
-{
-    if (LD == LD_PLAIN) return x + ((((size_t)img * h + yy) * w + xx) * CIN + c8 * 8);
-    const int sc8 = cs >> 3;
-    if (c8 < sc8) return x + ((((size_t)img * h + yy) * w + xx) * cs + c8 * 8);
-    return u + ((((size_t)img * (h >> 1) + (yy >> 1)) * (w >> 1) + (xx >> 1)) * (CIN - cs) + (c8 - sc8) * 8);
 }
 
 // Softmax-weighted composite of a pixel's covered layers (the network head).
@@ -535,152 +522,319 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
 }
 
 // ---------------------------------------------------------------------------
-// Weight gradient.  grid = (slices, chunks); CTA (s, c) accumulates rows
-// c*128 .. c*128+127 of (tap, cin) over pixel tiles s, s + slices, ... (one
-// tile = 128 pixels of one row) and writes partial[s][row][cout].
+// Weight gradient, all nine taps from one MMA per 16 pixels:
+//   D[(dy, cin)][(dx, cout)] += A[(dy, cin)][q] * B[q][(dx, cout)],
+//   A = X[y + dy - 1][q][cin],  B = G[y][q - (dx - 1)][cout],
+// summed over image rows y and pixels q (K, 16 per MMA), accumulators in TMEM
+// over the CTA's whole share.  Both operands are MN-major: a pixel's CX = 16
+// or 32 input channels, or its output channels, are rows of 32, 64 or 128
+// bytes in the swizzle of that width, as TMA writes them.  X lies in shared
+// memory as [row][pixel][CX], so the operand of output row y is 128 / CX
+// successive rows from y on: the three dy, then rows whose accumulators are
+// not looked at.  G is loaded three times, a pixel further each time, so its
+// dx are a copy apart.  One MMA per tap would have N = cout = 16..64 columns,
+// and fetching the 4 KB of A takes several times such a multiplication; here
+// N = 3 cout.  A layer of more than 32 input channels is a job per 32.
+//
+// How far a sum is cut into slices (a CTA's share of the tiles) is not free:
+// the tensor core truncates as it adds to an accumulator, so a sum comes out
+// too small by an amount that grows with the number of MMAs - 1.5e-4 of it
+// for 1772 of them over positive data.  The slices are therefore the ones of
+// one 128-row block of (tap, cin) per SM, 74, 49, 29 or 21 by layer, that
+// results have always come from: gradients of a batch of 64 windows agree
+// with those to 8e-7, and one slice per SM is 1.3e-4 away.
+//
+// That leaves two thirds of the SMs idle, so one launch takes the jobs of
+// several layers, longest first, a CTA per (job, slice).  CTA `b` of a job
+// handles tiles b, b + slices, ... of 32 x 4 pixels.
+//   warp 4     lane 0 loads a tile's X and G by TMA (zero fill outside the
+//              image) into a ring of stages;
+//   warp 5     lane 0 issues the MMAs; a commit frees the stage;
+//   warps 0-3  sum G for the bias gradient (where asked for); with an
+//              upsampled input expand the half-resolution box into the
+//              stage's X; at the end write the accumulators as this slice's
+//              partial sums.
+// Every wait is bounded; a timeout sets the error flag and the CTA winds down
+// after its loads have landed.
+//
+// What bounds it is shared memory: a 32 -> 32 tile takes 718 cycles, of which
+// TMA writes 37 KB (288 cycles at 128 B, and 580 at the 64 B/clk that L2
+// gives an SM) and the MMAs read 56 KB (448).
+// 64 windows of 256 x 256, all eight layers with their bias gradients: 0.95 ms
+// (2.5 ms with a launch per layer), and 0.06 for the reduction; one 128-row
+// chunk of (tap, cin) per CTA gathered by cp.async, N = cout and a kernel of
+// its own for the bias took 10.9 + 0.29 ms.
 // ---------------------------------------------------------------------------
-struct WgradArgs
+enum WgradKind
 {
-    const bf16* x;
-    const bf16* u;
-    int cs;
-    const bf16* g;  // [n][h][w][COUT]
+    WG_16_32,
+    WG_32_32,
+    WG_32_64,
+    WG_32_16,
+    WG_UP32_32,  // X at half resolution, upsampled (nearest)
+};
+
+struct WgradJob
+{
+    CUtensorMap mapX, mapG;
+    int kind, firstBlock, slices;
     int n, h, w;
-    float* partial;  // [gridDim.x][gridDim.y * 128][COUT]
+    int cin, c0;     // channels of the layer, and the first of X's among them
+    int xc0;         // the first of X's channels in its tensor
+    int bias;        // write the sums of g
+    float* partial;  // per slice [3 cin][3 COUT], then [COUT] sums of g
+};
+
+constexpr int kWgJobs = 9;  // a 96-, two 64- and two 32-channel layers
+
+struct WgradBatch
+{
+    WgradJob job[kWgJobs];
+    int jobs;
     int* error;
 };
 
-template <int CIN, int COUT>
+constexpr int kWgRows = 4, kWgTW = 32;  // pixels of a tile
+
+template <int CX, int COUT, bool UP>
 struct WgradShape
 {
-    static constexpr int kC8 = CIN / 8;
-    static constexpr int kRows8 = 9 * kC8;
-    static constexpr int kChunks = (kRows8 + 15) / 16;
-    static constexpr uint32_t kA = 16 * 2048;
-    static constexpr uint32_t kB = (COUT / 8) * 2048;
-    static constexpr uint32_t kStage = kA + kB;
-    static constexpr uint32_t kSmem = 2 * kStage + 64;
-    static constexpr uint32_t kTmem = tc::tmem_cols(COUT);
-    static_assert(COUT % 16 == 0 && COUT >= 16 && COUT <= 256, "MMA shape");
+    static constexpr int kAtoms = 128 / CX;     // rows of X in an MMA
+    static constexpr int kXRows = kWgRows + 2;  // rows loaded
+    static constexpr uint32_t kXRow = kWgTW * CX * 2, kGRow = kWgTW * COUT * 2;
+    static constexpr uint32_t kX = ((kWgRows - 1 + kAtoms) * kXRow + 1023) / 1024 * 1024;
+    static constexpr uint32_t kGCopy = kWgRows * kGRow;
+    static constexpr uint32_t kG = (3 * kGCopy + 1023) / 1024 * 1024;
+    // Upsampled input: the half-resolution box behind a tile's X rows.
+    static constexpr int kHalfRows = kWgRows / 2 + 2;
+    static constexpr uint32_t kHalfRow = kWgTW / 2 * CX * 2, kHalf = UP ? kHalfRows * kHalfRow : 0;
+    static constexpr uint32_t kStage = kX + kG + (kHalf + 1023) / 1024 * 1024;
+    static constexpr int kStages = 214 * 1024 / kStage > 6 ? 6 : 214 * 1024 / kStage;
+    static constexpr uint32_t kSmem = 1024 + kStages * kStage + 256;
+    static constexpr int kN = 3 * COUT;
+    static constexpr uint32_t kTmem = tc::tmem_cols(kN);
+    static_assert(CX == 16 || CX == 32, "X rows of a swizzle's width, three of them in an MMA");
+    static_assert(COUT == 16 || COUT == 32 || COUT == 64, "G rows of a swizzle's width");
+    static_assert(!UP || CX == 32, "upsampled input: 32 channels");
+    static_assert(kStages >= 2 && kSmem <= 227u * 1024u, "shared memory");
 };
 
-template <int CIN, int COUT, int LD>
-__global__ void __launch_bounds__(128, 1) k_conv3x3_wgrad(WgradArgs a)
+// Position of the 16-byte channel chunk c of pixel px in a row of C channels
+// (C * 2 bytes a pixel) under the swizzle of that width; its own inverse in c.
+template <int C>
+__device__ __forceinline__ int swizzled_chunk(int px, int c)
 {
-    using S = WgradShape<CIN, COUT>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + 2 * S::kStage);
-    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(mbar + 2);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int chunk = blockIdx.y;
-    const int tilesX = a.w / kTileX;
-    const long long nTiles = (long long)a.n * a.h * tilesX;
-    const int myTiles = (long long)blockIdx.x < nTiles ? (int)((nTiles - 1 - blockIdx.x) / gridDim.x) + 1 : 0;
-    float* part = a.partial + ((size_t)blockIdx.x * (gridDim.y * 128) + (size_t)chunk * 128) * COUT;
-    if (myTiles == 0)
-    {
-        for (int q = tid; q < 128 * COUT; q += 128) part[q] = 0.0f;
-        return;
-    }
+    return C == 64 ? c ^ (px & 7) : C == 32 ? c ^ ((px >> 1) & 3) : c ^ ((px >> 2) & 1);
+}
 
-    auto load = [&](long long t, unsigned char* buf) {
-        const int x0 = (int)(t % tilesX) * kTileX;
-        const long long r = t / tilesX;
-        const int y = (int)(r % a.h), img = (int)(r / a.h);
-        for (int q = tid; q < 16 * kTileX; q += 128)
-        {
-            const int lg = q & 15, px = q >> 4;
-            const int r8 = chunk * 16 + lg;
-            const int tap = r8 / S::kC8, c8 = r8 % S::kC8;
-            const int yy = y + tap / 3 - 1, xx = x0 + px + tap % 3 - 1;
-            const bool ok = r8 < S::kRows8 && yy >= 0 && yy < a.h && xx >= 0 && xx < a.w;
-            const bf16* src = ok ? input_chunk<CIN, LD>(a.x, a.u, a.cs, a.h, a.w, img, yy, xx, c8) : a.x;
-            tc::cp_async16(buf + lg * 2048 + px * 16, src, ok ? 16 : 0);
-        }
-        constexpr int kG8 = COUT / 8;
-        for (int q = tid; q < kG8 * kTileX; q += 128)
-        {
-            const int c8 = q % kG8, px = q / kG8;
-            const bf16* src = a.g + ((((size_t)img * a.h + y) * a.w + x0 + px) * COUT + c8 * 8);
-            tc::cp_async16(buf + S::kA + c8 * 2048 + px * 16, src, 16);
-        }
-    };
+template <int CX, int COUT, bool UP>
+__device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float (&sBias)[128][9], int* error)
+{
+    using S = WgradShape<CX, COUT, UP>;
+    extern __shared__ unsigned char smemRaw[];
+    unsigned char* smem =
+        reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kStages * S::kStage);
+    uint64_t* empty = full + S::kStages;
+    uint64_t* halfFull = empty + S::kStages;
+    uint64_t* done = halfFull + S::kStages;
+    uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(done + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tilesX = a.w / kWgTW, tilesY = (a.h + kWgRows - 1) / kWgRows;
+    const long long nTiles = (long long)a.n * tilesX * tilesY;  // >= a.slices
+    const int myTiles = (int)((nTiles - 1 - slice) / a.slices) + 1;
+    const bool bias = !UP && a.bias;
+    const bool helpers = UP || bias;  // warps 0-3 take part in every tile
 
     if (warp == 0) tc::tmem_alloc(tmemSlot, S::kTmem);
     if (tid == 0)
     {
-        tc::mbar_init(&mbar[0], 1);
-        tc::mbar_init(&mbar[1], 1);
+        for (int s = 0; s < S::kStages; ++s)
+        {
+            tc::mbar_init(&full[s], UP ? 1 + 128 : 1);
+            tc::mbar_init(&empty[s], bias ? 1 + 4 : 1);
+            tc::mbar_init(&halfFull[s], 1);
+        }
+        tc::mbar_init(done, 1);
         tc::fence_mbar_init();
     }
-    load(blockIdx.x, smem);
-    tc::cp_async_commit();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tmem = *tmemSlot;
-    constexpr uint32_t idesc = tc::idesc_bf16_f32(128, COUT) | (1u << 15) | (1u << 16);  // A, B MN-major
-
     bool ok = true;
-    for (int i = 0; i < myTiles; ++i)
+
+    if (warp == 4)
     {
-        const int s = i & 1;
-        const long long t = blockIdx.x + (long long)i * gridDim.x;
-        if (i + 1 < myTiles)
+        if (lane == 0)
         {
-            if (i >= 1 && !tc::mbar_wait(&mbar[s ^ 1], ((i - 1) >> 1) & 1, kWaitSpins)) ok = false;
-            if (ok) load(t + gridDim.x, smem + (s ^ 1) * S::kStage);
-            tc::cp_async_commit();
-            tc::cp_async_wait<1>();
-        }
-        else
-        {
-            tc::cp_async_wait<0>();
-        }
-        tc::fence_proxy_async();
-        if (__syncthreads_or(!ok))
-        {
-            ok = false;
-            break;
-        }
-        if (tid == 0)
-        {
-            tc::fence_after_sync();
-            const uint32_t a0 = tc::smem_u32(smem + s * S::kStage), b0 = a0 + S::kA;
-#pragma unroll
-            for (int j = 0; j < kTileX / 16; ++j)
-                tc::mma_bf16(tmem, tc::smem_desc(a0 + j * 256, 128, 2048), tc::smem_desc(b0 + j * 256, 128, 2048),
-                             idesc, (i > 0 || j > 0) ? 1u : 0u);
-            tc::mma_commit(&mbar[s]);
+            int issued = 0;
+            // Tile (tx, ty, img), stepped by a.slices tiles with carries: this
+            // one thread's divisions per tile took longer than its copies.
+            const int nx = a.slices % tilesX, ny = a.slices / tilesX % tilesY, ni = a.slices / tilesX / tilesY;
+            int tx = slice % tilesX, ty = slice / tilesX % tilesY, img = slice / tilesX / tilesY;
+            int s = -1;
+            uint32_t phase = 0;  // of the empty barrier: one before the first use
+            for (int i = 0; i < myTiles; ++i)
+            {
+                if (++s == S::kStages) s = 0;
+                if (s == 0) phase ^= 1;
+                if (!tc::mbar_wait(&empty[s], phase, kWaitSpins))
+                {
+                    ok = false;
+                    break;
+                }
+                const int x0 = tx * kWgTW, y0 = ty * kWgRows;
+                unsigned char* st = smem + s * S::kStage;
+                if (UP)
+                {
+                    tc::mbar_arrive_expect_tx(&halfFull[s], S::kHalf);
+                    tc::tma_load_4d(st + S::kX + S::kG, &a.mapX, a.xc0, x0 >> 1, (y0 >> 1) - 1, img, &halfFull[s]);
+                }
+                tc::mbar_arrive_expect_tx(&full[s], (UP ? 0u : S::kXRows * S::kXRow) + 3 * S::kGCopy);
+                if (!UP) tc::tma_load_4d(st, &a.mapX, a.xc0, x0, y0 - 1, img, &full[s]);
+                for (int dx = 0; dx < 3; ++dx)
+                    tc::tma_load_4d(st + S::kX + dx * S::kGCopy, &a.mapG, 0, x0 - (dx - 1), y0, img, &full[s]);
+                tx += nx;
+                ty += ny + (tx >= tilesX);
+                if (tx >= tilesX) tx -= tilesX;
+                img += ni + (ty >= tilesY);
+                if (ty >= tilesY) ty -= tilesY;
+                issued = i + 1;
+            }
+            // The last loads must land before the CTA may exit.
+            for (int j = max(0, issued - S::kStages); j < issued; ++j)
+            {
+                const int s = j % S::kStages;
+                if (UP && !tc::mbar_wait(&halfFull[s], (j / S::kStages) & 1, kWaitSpins)) ok = false;
+                if (!tc::mbar_wait(&full[s], (j / S::kStages) & 1, kWaitSpins)) ok = false;
+            }
         }
     }
-    if (ok)
+    else if (warp == 5)
     {
-        const int last = myTiles - 1;
-        bool done = tc::mbar_wait(&mbar[last & 1], (last >> 1) & 1, kWaitSpins);
-        done = __all_sync(0xffffffffu, done);
-        if (!done) ok = false;
+        if (lane == 0)
+        {
+            constexpr uint32_t idesc = tc::idesc_bf16_f32(128, S::kN) | (1u << 15) | (1u << 16);  // A, B MN-major
+            for (int i = 0; i < myTiles; ++i)
+            {
+                const int s = i % S::kStages;
+                if (!tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins))
+                {
+                    ok = false;
+                    break;
+                }
+                tc::fence_after_sync();
+                const uint32_t xa = tc::smem_u32(smem + s * S::kStage);
+                const uint64_t aBase = tc::smem_desc_mn<CX>(xa, S::kXRow),
+                               bBase = tc::smem_desc_mn<COUT>(xa + S::kX, S::kGCopy);
+#pragma unroll
+                for (int r = 0; r < kWgRows; ++r)
+#pragma unroll
+                    for (int k = 0; k < kWgTW / 16; ++k)
+                        tc::mma_bf16(tmem, aBase + ((r * S::kXRow + k * 16 * CX * 2) >> 4),
+                                     bBase + ((r * S::kGRow + k * 16 * COUT * 2) >> 4), idesc,
+                                     (i > 0 || r > 0 || k > 0) ? 1u : 0u);
+                tc::mma_commit(&empty[s]);
+            }
+            tc::mma_commit(done);
+        }
+    }
+    else if (helpers)
+    {
+        // Bias: this thread's chunk position and pixels of the copy dx = 1,
+        // rows of 32 pixels with COUT / 8 chunks; the pixels it sees keep the
+        // chunk's place in the swizzle, so its channels are fixed.
+        constexpr int kO8 = COUT / 8;
+        const int pos = tid % kO8, px0 = tid / kO8;
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (int i = 0; i < myTiles; ++i)
+        {
+            const int s = i % S::kStages;
+            unsigned char* st = smem + s * S::kStage;
+            if (UP)
+            {
+                if (!tc::mbar_wait(&halfFull[s], (i / S::kStages) & 1, kWaitSpins))
+                {
+                    ok = false;
+                    break;
+                }
+                // X row j is image row y0 - 1 + j, y0 a multiple of 4: row
+                // (j + 1) / 2 of the box
+                const unsigned char* half = st + S::kX + S::kG;
+#pragma unroll
+                for (int k = 0; k < S::kXRows * kWgTW * 4 / 128; ++k)
+                {
+                    const int c = tid & 3, px = tid >> 2, j = k;
+                    const int hr = (j + 1) >> 1, hp = px >> 1;
+                    *reinterpret_cast<uint4*>(st + j * S::kXRow + px * 64 + swizzled_chunk<32>(px, c) * 16) =
+                        *reinterpret_cast<const uint4*>(half + hr * S::kHalfRow + hp * 64 +
+                                                        swizzled_chunk<32>(hp, c) * 16);
+                }
+                tc::fence_proxy_async();  // generic smem writes -> tensor core
+                tc::mbar_arrive(&full[s]);
+            }
+            else
+            {
+                if (!tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins))
+                {
+                    ok = false;
+                    break;
+                }
+                const unsigned char* g = st + S::kX + S::kGCopy;
+#pragma unroll
+                for (int k = 0; k < kWgRows * kWgTW * kO8 / 128; ++k)
+                {
+                    const int p = px0 + k * (128 / kO8);  // pixel of the tile, rows of 32
+                    float v[8];
+                    unpack8_bf16(*reinterpret_cast<const uint4*>(g + p * COUT * 2 + pos * 16), v);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[j] += v[j];
+                }
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive(&empty[s]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sBias[tid][j] = acc[j];
+    }
+    __syncthreads();
+    float* out = a.partial + (size_t)slice * (9 * a.cin * COUT + COUT);
+    if (warp < 4)
+    {
+        bool got = tc::mbar_wait(done, 0, kWaitSpins);
+        got = __all_sync(0xffffffffu, got);
+        if (!got) ok = false;
         else
         {
             tc::fence_after_sync();
-            float* row = part + (size_t)(warp * 32 + lane) * COUT;
+            const int m = warp * 32 + lane, dy = m / CX;
+            float* row = out + ((size_t)dy * a.cin + a.c0 + m % CX) * S::kN;
 #pragma unroll 1
-            for (int cb = 0; cb < COUT / 16; ++cb)
+            for (int cb = 0; cb < S::kN / 16; ++cb)
             {
                 float v[16];
                 tc::tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + cb * 16, v);
-                float4* o = reinterpret_cast<float4*>(row + cb * 16);
-                o[0] = make_float4(v[0], v[1], v[2], v[3]);
-                o[1] = make_float4(v[4], v[5], v[6], v[7]);
-                o[2] = make_float4(v[8], v[9], v[10], v[11]);
-                o[3] = make_float4(v[12], v[13], v[14], v[15]);
+                if (dy < 3)
+                {
+                    float4* o = reinterpret_cast<float4*>(row + cb * 16);
+                    o[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    o[1] = make_float4(v[4], v[5], v[6], v[7]);
+                    o[2] = make_float4(v[8], v[9], v[10], v[11]);
+                    o[3] = make_float4(v[12], v[13], v[14], v[15]);
+                }
             }
             tc::fence_before_sync();
         }
+        if (bias && tid < COUT)
+        {
+            float b = 0.0f;
+            for (int t = 0; t < 128; ++t)
+                if (swizzled_chunk<COUT>(t / (COUT / 8), t % (COUT / 8)) == tid >> 3) b += sBias[t][tid & 7];
+            out[9 * a.cin * COUT + tid] = b;
+        }
     }
-    if (!ok && lane == 0) atomicOr(a.error, 1);
-    tc::cp_async_wait<0>();
-    tc::fence_before_sync();
+    if (!ok && lane == 0) atomicOr(error, 1);
     __syncthreads();
     if (warp == 0)
     {
@@ -689,21 +843,86 @@ __global__ void __launch_bounds__(128, 1) k_conv3x3_wgrad(WgradArgs a)
     }
 }
 
-// dW[co][k] = sum over slices of partial[slice][k][co] (k = tap * cin + ci).
-__global__ void k_wgrad_reduce(const float* __restrict__ partial, int slices, int rowsTotal, int coutStride, int cin,
-                               int cout, float* __restrict__ dw)
+__global__ void __launch_bounds__(192, 1) k_conv3x3_wgrad(const __grid_constant__ WgradBatch b)
 {
-    const int K = 9 * cin;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= K * cout) return;
-    const int co = idx / K, k = idx % K;
+    int j = 0;
+    while (j + 1 < b.jobs && (int)blockIdx.x >= b.job[j + 1].firstBlock) ++j;
+    const WgradJob& a = b.job[j];
+    const int slice = blockIdx.x - a.firstBlock;
+    __shared__ float sBias[128][9];
+    switch (a.kind)
+    {
+        case WG_16_32: wgrad_slice<16, 32, false>(a, slice, sBias, b.error); break;
+        case WG_32_32: wgrad_slice<32, 32, false>(a, slice, sBias, b.error); break;
+        case WG_32_64: wgrad_slice<32, 64, false>(a, slice, sBias, b.error); break;
+        case WG_32_16: wgrad_slice<32, 16, false>(a, slice, sBias, b.error); break;
+        default: wgrad_slice<32, 32, true>(a, slice, sBias, b.error); break;
+    }
+}
+constexpr uint32_t kWgSmem = std::max({WgradShape<16, 32, false>::kSmem, WgradShape<32, 32, false>::kSmem,
+                                       WgradShape<32, 64, false>::kSmem, WgradShape<32, 16, false>::kSmem,
+                                       WgradShape<32, 32, true>::kSmem});
+
+// The concatenation of x (cs channels) and the nearest 2x upsample of u as one
+// tensor, for splits that no kernel above takes directly.
+__global__ void k_concat(const bf16* __restrict__ x, const bf16* __restrict__ u, int cs, int cin, int n, int h, int w,
+                         bf16* __restrict__ out)
+{
+    const int c8n = cin / 8, sc8 = cs / 8;
+    const long long total = (long long)n * h * w * c8n;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
+         i += (long long)gridDim.x * blockDim.x)
+    {
+        const int c8 = (int)(i % c8n);
+        const long long p = i / c8n;
+        const int xx = (int)(p % w);
+        const long long r = p / w;
+        const int yy = (int)(r % h), img = (int)(r / h);
+        const bf16* src = c8 < sc8 ? x + p * cs + c8 * 8
+                                   : u + (((size_t)img * (h >> 1) + (yy >> 1)) * (w >> 1) + (xx >> 1)) * (cin - cs) +
+                                         (c8 - sc8) * 8;
+        reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(src);
+    }
+}
+
+// dW[co][dy][dx][c] = sum over slices of partial[slice][(dy, c)][(dx, co)], and
+// db[co] (unless null) the sums of g, in slice order, for the layers of a
+// batch; consecutive threads take consecutive partial sums.
+struct WgradReduce
+{
+    struct Layer
+    {
+        const float* partial;
+        int slices, cin, coutPad, cout, firstBlock;
+        float *dw, *db;
+    } layer[kWgJobs];
+    int layers;
+};
+
+__global__ void k_wgrad_reduce(const __grid_constant__ WgradReduce r)
+{
+    int l = 0;
+    while (l + 1 < r.layers && (int)blockIdx.x >= r.layer[l + 1].firstBlock) ++l;
+    const WgradReduce::Layer& a = r.layer[l];
+    const int N = 3 * a.coutPad, weights = 3 * a.cin * N, count = weights + a.coutPad;
+    const int idx = (blockIdx.x - a.firstBlock) * blockDim.x + threadIdx.x;
+    if (idx >= count) return;
+    if (idx >= weights && !a.db) return;
     float s = 0.0f;
-    for (int g = 0; g < slices; ++g) s += partial[((size_t)g * rowsTotal + k) * coutStride + co];
-    dw[(size_t)co * K + k] = s;
+#pragma unroll 8
+    for (int g = 0; g < a.slices; ++g) s += __ldg(a.partial + (size_t)g * count + idx);
+    if (idx < weights)
+    {
+        const int m = idx / N, col = idx - m * N;
+        const int dy = m / a.cin, c = m - dy * a.cin, dx = col / a.coutPad, co = col - dx * a.coutPad;
+        if (co < a.cout) a.dw[((size_t)co * 9 + dy * 3 + dx) * a.cin + c] = s;
+    }
+    else if (idx - weights < a.cout)
+        a.db[idx - weights] = s;
 }
 
 // ---------------------------------------------------------------------------
-// Glue: input packing, pooling, loss, gradient routing, bias gradients, Adam.
+// Glue: input packing, pooling, loss, gradient routing, Adam.
 // ---------------------------------------------------------------------------
 // The mask channel of a covered pixel: 0.25 + 0.75 min(1, d / kFeather) with
 // d the distance from (x, y) to the nearest of the slot's boundary segments
@@ -910,34 +1129,6 @@ __global__ void k_loss(const i360b_blend_job* __restrict__ jobs, int n, int h, i
     }
 }
 
-// db[c] += sum over pixels of g[p][c], c < cout (g has C = 8 * c8n channels).
-__global__ void k_bias_grad(const bf16* __restrict__ g, long long pixels, int c8n, int cout, float* __restrict__ db)
-{
-    __shared__ float red[256 * 8];
-    const int lanes = blockDim.x / c8n;
-    const int c8 = threadIdx.x % c8n, lane = threadIdx.x / c8n;
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (lane < lanes)
-        for (long long p = (long long)blockIdx.x * lanes + lane; p < pixels; p += (long long)gridDim.x * lanes)
-        {
-            float v[8];
-            unpack8_bf16(reinterpret_cast<const uint4*>(g + p * c8n * 8)[c8], v);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] += v[j];
-        }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[threadIdx.x * 8 + j] = lane < lanes ? acc[j] : 0.0f;
-    __syncthreads();
-    const int C = c8n * 8;
-    if ((int)threadIdx.x < C && (int)threadIdx.x < cout)
-    {
-        const int cc8 = threadIdx.x >> 3, j = threadIdx.x & 7;
-        float s = 0.0f;
-        for (int l = 0; l < lanes; ++l) s += red[(l * c8n + cc8) * 8 + j];
-        atomicAdd(&db[threadIdx.x], s);
-    }
-}
-
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
                        int count, float lr, float c1, float c2)
 {
@@ -1014,10 +1205,12 @@ int elementwise_grid(long long n, int block = 256)
     return (int)std::max<long long>(1, std::min<long long>((n + block - 1) / block, (long long)sm_count() * 16));
 }
 
-// Tensor map of an NHWC bf16 tensor as (C, W, H, N) with a box of 8
-// channels x boxW x boxH x 1 (zero fill outside).  The encoder comes from the
-// driver through the runtime (no link against the driver library).
-int make_input_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxW, int boxH)
+// Tensor map of an NHWC bf16 tensor as (C, W, H, N) with a box of boxC
+// channels x boxW x boxH x 1 (zero fill outside) under a shared-memory
+// swizzle.  The encoder comes from the driver through the runtime (no link
+// against the driver library).
+int make_tile_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxC, int boxW, int boxH,
+                  CUtensorMapSwizzle swizzle)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     static std::once_flag once;
@@ -1033,13 +1226,19 @@ int make_input_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w,
         return fail(I360B_INVALID_PARAM, "conv3x3 input must be 16-byte aligned with channels a multiple of 8");
     const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
     const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
-    const cuuint32_t box[4] = {8, (cuuint32_t)boxW, (cuuint32_t)boxH, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)boxC, (cuuint32_t)boxW, (cuuint32_t)boxH, 1};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(base), dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(I360B_CUDA_ERROR, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return I360B_SUCCESS;
+}
+
+// The convolutions' 8-channel boxes.
+int make_input_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxW, int boxH)
+{
+    return make_tile_map(m, base, c, n, h, w, 8, boxW, boxH, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 template <int CIN, int NPAD, int TW, int TH, int STAGES, int LD, int EP, int EW>
@@ -1100,63 +1299,106 @@ int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cuda
                 ep);
 }
 
-template <int CIN, int COUT, int LD>
-int run_wgrad(const WgradArgs& base, float* dw, int cout, void* scratch, size_t scratchBytes, cudaStream_t s)
+constexpr CUtensorMapSwizzle swizzle_of(int channels)
 {
-    using S = WgradShape<CIN, COUT>;
-    static std::once_flag once;
-    static int perSm = 1;
-    static cudaError_t attrErr = cudaSuccess;
-    std::call_once(once, [] {
-        attrErr = cudaFuncSetAttribute(k_conv3x3_wgrad<CIN, COUT, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)S::kSmem);
-        int occ = 1;
-        if (attrErr == cudaSuccess)
-            attrErr = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_conv3x3_wgrad<CIN, COUT, LD>, 128, S::kSmem);
-        perSm = std::max(1, std::min<int>(std::min(occ, 2), 512 / (int)S::kTmem));
-    });
-    if (attrErr != cudaSuccess) return cuda_fail(attrErr, "wgrad attributes");
-    const long long tiles = (long long)base.n * base.h * (base.w / kTileX);
-    const int slices = (int)std::max<long long>(
-        1, std::min<long long>(tiles, (long long)sm_count() * perSm / S::kChunks));
-    const size_t need = (size_t)slices * S::kChunks * 128 * COUT * sizeof(float);
-    if (need > scratchBytes) return fail(I360B_OUT_OF_MEMORY, "wgrad scratch too small (%zu > %zu)", need, scratchBytes);
-    WgradArgs a = base;
-    a.partial = static_cast<float*>(scratch);
-    k_conv3x3_wgrad<CIN, COUT, LD><<<dim3(slices, S::kChunks), 128, S::kSmem, s>>>(a);
-    I360B_TRY(check_launch("wgrad kernel"));
-    const int total = 9 * CIN * cout;
-    k_wgrad_reduce<<<(total + 255) / 256, 256, 0, s>>>(a.partial, slices, S::kChunks * 128, COUT, CIN, cout, dw);
-    return check_launch("wgrad reduce kernel");
+    return channels == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+           : channels == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                            : CU_TENSOR_MAP_SWIZZLE_32B;
 }
 
+// Slices of a layer's sums at most: one 128-row block of (tap, cin) per SM.
+int wgrad_slices(int cin) { return std::max(1, sm_count() / ((9 * cin / 8 + 15) / 16)); }
+
+// The weight and bias gradients of one layer.
+struct WgradLayer
+{
+    const bf16* x;  // [n][h][w][cin], or the skip [n][h][w][cs] where cs > 0
+    const bf16* u;  // [n][h/2][w/2][cin - cs]
+    int cs;
+    const bf16* g;  // [n][h][w][cout]
+    int n, h, w, cin, cout, coutReal;
+    float *dw, *db;  // db may be null
+
+    int slices() const
+    {
+        const long long tiles = (long long)n * ((h + kWgRows - 1) / kWgRows) * (w / kWgTW);
+        return (int)std::max<long long>(1, std::min<long long>(tiles, wgrad_slices(cin)));
+    }
+    size_t partials() const { return (size_t)slices() * (9 * cin * cout + cout); }
+};
+
+// Partial sums of the network's layers 3..7 in one batch, the most at a time.
 size_t wgrad_scratch_bytes()
 {
-    // Upper bound over the supported shapes: slices <= 2 * SMs / chunks.
-    size_t mx = 0;
-    const int sms = sm_count();
-    auto f = [&](int cin, int cout) {
-        const int chunks = (9 * cin / 8 + 15) / 16;
-        const size_t slices = std::max(1, 2 * sms / chunks);
-        mx = std::max(mx, slices * chunks * 128 * cout * sizeof(float));
-    };
-    f(16, 32), f(32, 32), f(32, 64), f(64, 64), f(96, 32), f(32, 16);
-    return mx;
+    constexpr int shapes[][2] = {{32, 32}, {32, 16}, {64, 64}, {64, 64}, {96, 32}};
+    size_t floats = 0;
+    for (const auto& c : shapes) floats += (size_t)(9 * c[0] * c[1] + c[1]) * wgrad_slices(c[0]);
+    return floats * sizeof(float);
 }
 
-int dispatch_wgrad(int cin, int cout, int loader, const WgradArgs& a, float* dw, int coutReal, void* scratch,
-                   size_t bytes, cudaStream_t s)
+// `count` layers in one launch each of the sums and of their reduction.
+int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, size_t bytes, cudaStream_t s)
 {
-#define I360B_WG(CI, CO, LD) \
-    if (cin == CI && cout == CO && loader == LD) return run_wgrad<CI, CO, LD>(a, dw, coutReal, scratch, bytes, s);
-    I360B_WG(16, 32, LD_PLAIN)
-    I360B_WG(32, 32, LD_PLAIN)
-    I360B_WG(32, 64, LD_PLAIN)
-    I360B_WG(64, 64, LD_PLAIN)
-    I360B_WG(96, 32, LD_CONCAT)
-    I360B_WG(32, 16, LD_PLAIN)
-#undef I360B_WG
-    return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", cin, cout, loader);
+    static std::once_flag once;
+    static cudaError_t attrErr = cudaSuccess;
+    std::call_once(once, [] {
+        attrErr = cudaFuncSetAttribute(k_conv3x3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem);
+    });
+    if (attrErr != cudaSuccess) return cuda_fail(attrErr, "wgrad attributes");
+    WgradBatch b{};
+    WgradReduce r{};
+    b.error = error;
+    float* part = static_cast<float*>(scratch);
+    size_t used = 0;
+    int blocks = 0, reduceBlocks = 0;
+    for (int i = 0; i < count; ++i)
+    {
+        const WgradLayer& L = layers[i];
+        used += L.partials() * sizeof(float);
+        if (used > bytes) return fail(I360B_OUT_OF_MEMORY, "wgrad scratch too small");
+        const int kind = L.cout == 64                    ? (L.cin == 32 || L.cin == 64 ? WG_32_64 : -1)
+                         : L.cout == 16                  ? (L.cin == 32 ? WG_32_16 : -1)
+                         : L.cout != 32                  ? -1
+                         : L.cin == 16                   ? WG_16_32
+                         : L.cin == 32 || L.cin == 96    ? WG_32_32
+                                                         : -1;
+        if (kind < 0 || L.cs % 32 || (L.cs > 0 && L.cin != 96))
+            return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", L.cin, L.cout,
+                        L.cs ? LD_CONCAT : LD_PLAIN);
+        for (int c = 0; c < L.cin; c += 32)
+        {
+            if (b.jobs == kWgJobs) return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: batch too large");
+            WgradJob& j = b.job[b.jobs++];
+            const int cx = std::min(L.cin, 32);
+            const bool up = L.cs > 0 && c >= L.cs;
+            j.kind = up ? WG_UP32_32 : kind;
+            j.firstBlock = blocks;
+            j.slices = L.slices();
+            j.n = L.n;
+            j.h = L.h;
+            j.w = L.w;
+            j.cin = L.cin;
+            j.c0 = c;
+            j.xc0 = up ? c - L.cs : c;
+            j.bias = L.db && c == 0;
+            j.partial = part;
+            if (up)
+                I360B_TRY(make_tile_map(&j.mapX, L.u, L.cin - L.cs, L.n, L.h / 2, L.w / 2, cx, kWgTW / 2,
+                                        kWgRows / 2 + 2, swizzle_of(cx)));
+            else
+                I360B_TRY(make_tile_map(&j.mapX, L.x, L.cs > 0 ? L.cs : L.cin, L.n, L.h, L.w, cx, kWgTW, kWgRows + 2,
+                                        swizzle_of(cx)));
+            I360B_TRY(make_tile_map(&j.mapG, L.g, L.cout, L.n, L.h, L.w, L.cout, kWgTW, kWgRows, swizzle_of(L.cout)));
+            blocks += j.slices;
+        }
+        r.layer[r.layers++] = {part, L.slices(), L.cin, L.cout, L.coutReal, reduceBlocks, L.dw, L.db};
+        reduceBlocks += (9 * L.cin * L.cout + L.cout + 127) / 128;
+        part += L.partials();
+    }
+    k_conv3x3_wgrad<<<blocks, 192, kWgSmem, s>>>(b);
+    I360B_TRY(check_launch("wgrad kernel"));
+    k_wgrad_reduce<<<reduceBlocks, 128, 0, s>>>(r);
+    return check_launch("wgrad reduce kernel");
 }
 
 int check_window(int n, int w, int h)
@@ -1457,64 +1699,48 @@ struct BlendNet
         return dispatch_conv(pad16(kNet[l].cout), kNet[l].cin, LD_PLAIN, ep, a, s);
     }
 
-    int wgrad(int l, const bf16* x, const bf16* u, int cs, const bf16* g, int n, int w, int h, cudaStream_t s)
+    WgradLayer wgrad(int l, const bf16* x, const bf16* g, int n, int w, int h, const bf16* u = nullptr, int cs = 0) const
     {
-        WgradArgs a{};
-        a.x = x;
-        a.u = u;
-        a.cs = cs;
-        a.g = g;
-        a.n = n;
-        a.h = h;
-        a.w = w;
-        a.error = dError;
-        I360B_TRY(dispatch_wgrad(kNet[l].cin, pad16(kNet[l].cout), cs ? LD_CONCAT : LD_PLAIN, a, grads + wOff[l],
-                                 kNet[l].cout, wgScratch, wgBytes, s));
-        const long long pixels = (long long)n * w * h;
-        const int c8n = pad16(kNet[l].cout) / 8;
-        k_bias_grad<<<std::min<long long>(sm_count() * 4, (pixels + 255) / 256), 256, 0, s>>>(g, pixels, c8n,
-                                                                                              kNet[l].cout,
-                                                                                              grads + bOff[l]);
-        return check_launch("bias gradient kernel");
+        return {x, u, cs, g, n, h, w, kNet[l].cin, pad16(kNet[l].cout), kNet[l].cout, grads + wOff[l], grads + bOff[l]};
     }
 
-    // Loss, then every parameter gradient into `grads`.
+    // Loss, then every parameter gradient into `grads`.  The weight gradients
+    // are taken in two batches, each once the next step would overwrite an
+    // output gradient that they read.
     int backward(int n, int w, int h, cudaStream_t s)
     {
         const int hw = w / 2, hh = h / 2;
         const long long pix = (long long)n * w * h;
         I360B_CUDA(cudaMemsetAsync(dLoss, 0, sizeof(double), s), "loss reset");
-        I360B_CUDA(cudaMemsetAsync(grads, 0, (size_t)nParams * sizeof(float), s), "grad reset");
         k_loss<<<elementwise_grid(pix), 256, 0, s>>>(dJobs, n, h, w, reinterpret_cast<const float4*>(logits),
                                                    (float)(1.0 / (3.0 * (double)pix)), g8, dLoss);
         I360B_TRY(check_launch("loss kernel"));
         // layer 8 (32 -> 4): input a7
-        I360B_TRY(wgrad(7, a7, nullptr, 0, g8, n, w, h, s));
         I360B_TRY(dgrad(7, g8, n, w, h, a7, gA, EP_MASK, s));  // gA = g7
         // layer 7 (32 -> 32): input a6
-        I360B_TRY(wgrad(6, a6, nullptr, 0, gA, n, w, h, s));
         I360B_TRY(dgrad(6, gA, n, w, h, a6, gB, EP_MASK, s));  // gB = g6
         // layer 6 (96 -> 32): input concat(a2, up(a5))
-        I360B_TRY(wgrad(5, a2, a5, 32, gB, n, w, h, s));
         I360B_TRY(dgrad(5, gB, n, w, h, nullptr, du, EP_RAW, s));
         k_upsample_grad<<<elementwise_grid((long long)n * hw * hh * 8), 256, 0, s>>>(du, 96, 32, a5, n, h, w, 8, gh1);
         I360B_TRY(check_launch("upsample gradient kernel"));  // gh1 = g5
         // layer 5 (64 -> 64): input a4
-        I360B_TRY(wgrad(4, a4, nullptr, 0, gh1, n, hw, hh, s));
         I360B_TRY(dgrad(4, gh1, n, hw, hh, a4, gh2, EP_MASK, s));  // gh2 = g4
+        const WgradLayer late[] = {wgrad(5, a2, gB, n, w, h, a5, 32), wgrad(6, a6, gA, n, w, h),
+                                   wgrad(7, a7, g8, n, w, h), wgrad(4, a4, gh1, n, hw, hh),
+                                   wgrad(3, a3, gh2, n, hw, hh)};
+        I360B_TRY(run_wgrad(late, 5, dError, wgScratch, wgBytes, s));
         // layer 4 (64 -> 64): input a3
-        I360B_TRY(wgrad(3, a3, nullptr, 0, gh2, n, hw, hh, s));
         I360B_TRY(dgrad(3, gh2, n, hw, hh, a3, gh1, EP_MASK, s));  // gh1 = g3
         // layer 3 (32 -> 64): input p2
-        I360B_TRY(wgrad(2, p2, nullptr, 0, gh1, n, hw, hh, s));
         I360B_TRY(dgrad(2, gh1, n, hw, hh, nullptr, dp, EP_RAW, s));  // dp = d(pool)
         k_skip_grad<<<elementwise_grid(pix * 4), 256, 0, s>>>(du, 96, dp, a2, n, h, w, 4, gA);
         I360B_TRY(check_launch("skip gradient kernel"));  // gA = g2
         // layer 2 (32 -> 32): input a1
-        I360B_TRY(wgrad(1, a1, nullptr, 0, gA, n, w, h, s));
         I360B_TRY(dgrad(1, gA, n, w, h, a1, gB, EP_MASK, s));  // gB = g1
         // layer 1 (16 -> 32): input x0
-        return wgrad(0, x0, nullptr, 0, gB, n, w, h, s);
+        const WgradLayer early[] = {wgrad(1, a1, gA, n, w, h), wgrad(0, x0, gB, n, w, h),
+                                    wgrad(2, p2, gh1, n, hw, hh)};
+        return run_wgrad(early, 3, dError, wgScratch, wgBytes, s);
     }
 
     int adam(float lr, cudaStream_t s)
@@ -1820,17 +2046,29 @@ extern "C" int i360b_conv3x3_wgrad(const void* dX, const void* dU, int skipChann
     const size_t bytes = wgrad_scratch_bytes();
     void* scratch = nullptr;
     I360B_TRY(dev_alloc(&scratch, bytes, s, "wgrad scratch"));
-    WgradArgs a{};
-    a.x = static_cast<const bf16*>(dX);
-    a.u = static_cast<const bf16*>(dU);
-    a.cs = skipChannels;
-    a.g = static_cast<const bf16*>(dGrad);
-    a.n = n;
-    a.h = h;
-    a.w = w;
-    a.error = dErr;
+    WgradLayer L{static_cast<const bf16*>(dX), static_cast<const bf16*>(dU), std::max(skipChannels, 0),
+                 static_cast<const bf16*>(dGrad), n, h, w, cin, cout, cout, dGradW, nullptr};
     I360B_CUDA(cudaMemsetAsync(dErr, 0, sizeof(int), s), "error flag");
-    int rc = dispatch_wgrad(cin, cout, skipChannels > 0 ? LD_CONCAT : LD_PLAIN, a, dGradW, cout, scratch, bytes, s);
+    int rc = I360B_SUCCESS;
+    void* full = nullptr;
+    if ((L.cs > 0) != (cin == 96))
+        rc = fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", cin, cout,
+                  L.cs > 0 ? LD_CONCAT : LD_PLAIN);
+    else if (cin == 96 && cout == 32 && L.cs % 32)
+    {
+        // a skip that is not whole 32-channel jobs: concatenate first
+        const long long units = (long long)n * h * w * (cin / 8);
+        rc = dev_alloc(&full, (size_t)units * 16, s, "wgrad concatenation");
+        if (rc == I360B_SUCCESS)
+        {
+            k_concat<<<elementwise_grid(units), 256, 0, s>>>(L.x, L.u, L.cs, cin, n, h, w, static_cast<bf16*>(full));
+            rc = check_launch("concatenation kernel");
+        }
+        L.x = static_cast<const bf16*>(full);
+        L.cs = 0;
+    }
+    if (rc == I360B_SUCCESS) rc = run_wgrad(&L, 1, dErr, scratch, bytes, s);
+    if (full) dev_free(full, s);
     int e = 0;
     cudaMemcpyAsync(&e, dErr, sizeof(int), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);

@@ -32,6 +32,23 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
     return d;
 }
 
+// Shared-memory matrix descriptor, MN-major, rows of C = 16, 32 or 64 bf16
+// values of the M or N dimension (32, 64 or 128 bytes, a row per K) in the
+// swizzle of that width: groups of 8 rows follow each other, the next C
+// values lie `atom` bytes further.  Addresses are multiples of 8 rows.
+template <int C>
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t atom)
+{
+    static_assert(C == 16 || C == 32 || C == 64, "swizzle width");
+    uint64_t d = 0;
+    d |= (uint64_t)((addr >> 4) & 0x3fffu);
+    d |= (uint64_t)((atom >> 4) & 0x3fffu) << 16;
+    d |= (uint64_t)((8 * C * 2) >> 4) << 32;
+    d |= (uint64_t)1 << 46;                                   // descriptor version (Blackwell)
+    d |= (uint64_t)(C == 64 ? 2 : C == 32 ? 4 : 6) << 61;     // 128-, 64-, 32-byte swizzle
+    return d;
+}
+
 // Instruction descriptor of kind::f16: BF16 x BF16 -> F32, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
 {

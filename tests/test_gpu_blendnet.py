@@ -313,3 +313,30 @@ def test_invalid_windows_are_rejected(backend):
     with pytest.raises(RuntimeError, match="INVALID_PARAM"):
         net.infer(jobs, 1, 256, 7)
     net.close()
+
+
+@pytest.mark.parametrize("cin,cout,skip", [(i, o, 32 if c else 0) for i, o, c in WGRAD_CASES] +
+                         [(96, 32, 8), (96, 32, 64)])
+@pytest.mark.parametrize("n,h,w", [(1, 2, 256), (3, 6, 256), (1, 130, 512)])
+def test_conv3x3_wgrad_tile_edges(backend, cin, cout, skip, n, h, w):
+    """Heights around the 4-row tiles (a last tile of two rows, a single one),
+    several images, more tiles than SMs, other splits of the concatenation.  fp32 sums of bf16 products in another
+    order: 1e-4 of the largest gradient, as above."""
+    import torch
+    import torch.nn.functional as F
+    from image360_b200 import blendnet as bn
+    rng = np.random.default_rng(cin * 100 + cout + h)
+    if skip:
+        x, u = _bf((n, h, w, skip), rng), _bf((n, h // 2, w // 2, cin - skip), rng)
+        full = torch.cat([x, u.repeat_interleave(2, 1).repeat_interleave(2, 2)], -1)
+    else:
+        x, u = _bf((n, h, w, cin), rng), None
+        full = x
+    g = _bf((n, h, w, cout), rng)
+    out = torch.full((cout, 3, 3, cin), float("nan"), dtype=torch.float32, device="cuda")
+    bn.conv3x3_wgrad(x, g, out, u=u, skip=skip)
+    torch.cuda.synchronize()
+    xp = F.pad(full.double(), (0, 0, 1, 1, 1, 1))
+    ref = torch.stack([torch.stack([torch.einsum("nhwo,nhwi->oi", g.double(), xp[:, ky:ky + h, kx:kx + w])
+                                    for kx in range(3)], 1) for ky in range(3)], 1)
+    assert float((out.double() - ref).abs().max()) <= 1e-4 * float(ref.abs().max())
