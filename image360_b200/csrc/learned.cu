@@ -50,7 +50,8 @@ constexpr float kInScale = 1.0f / 32768.0f;
 enum
 {
     LD_PLAIN = 0,
-    LD_CONCAT = 1
+    LD_CONCAT = 1,
+    LD_SPLIT = 2  // 96 channels of one tensor
 };
 enum
 {
@@ -73,48 +74,82 @@ struct ConvArgs
     const bf16* act;  // EP_MASK: [n][h][w][npad]
     const i360b_blend_job* jobs;  // EP_COMPOSITE: one per image
     int* error;
+    int rowSplit;  // the output map has the rows as (row % J, row / J): h is a multiple of J
 };
 
-// Tile geometry of the 3x3 convolution: TW x TH output pixels per tile, split
-// into M blocks of 8 columns x 16 rows; the input halo of (TW+2) x (TH+2)
-// pixels is kept per 8-channel chunk with row pitch kP = TW+2 pixels.
-template <int CIN, int NPAD, int TW, int TH, int STAGES, int LD, int EW = 4>
+// Tile geometry of the 3x3 convolution: TW x 16 J output pixels per tile, split
+// into M blocks of 8 columns x 16 rows that lie J apart.  The input halo of (TW+2) x (TH+2)
+// pixels is kept as rows of a pixel's channels (row pitch kP = TW+2 pixels) in
+// the swizzle of that width: all 16, 32 or 64 of them, or for 96 the first 32
+// and the other 64 in two such tiles.
+template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
 struct ConvShape
 {
     // Roles by warp: [0, EW) epilogue, EW producer, EW + 1 MMA, then (for a
     // concatenated input) 4 upsampling warps.
-    static constexpr int kEpiWarps = EW;
     static constexpr int kProducerWarp = EW, kMmaWarp = EW + 1, kExpandWarp = EW + 2;
-    static constexpr int kC8 = CIN / 8;
+    static constexpr int TH = 16 * J;
     static constexpr int kP = TW + 2;
     static constexpr int kHaloPx = (TW + 2) * (TH + 2);
-    static constexpr uint32_t kBox = kHaloPx * 16;                  // bytes of one chunk box
-    static constexpr uint32_t kChunk = (kBox + 127) / 128 * 128;    // TMA destinations 128-byte aligned
-    static constexpr uint32_t kStage = kC8 * kChunk;
-    static constexpr uint32_t kW = 9u * CIN * NPAD * 2;
-    static constexpr int kBX = TW / 8, kBY = TH / 16, kMB = kBX * kBY;
+    static constexpr int kCA = CIN == 96 ? 32 : CIN, kCB = CIN - kCA;  // channels of the two tiles
+    static constexpr uint32_t kBoxA = kHaloPx * kCA * 2, kBoxB = kHaloPx * kCB * 2;
+    static constexpr uint32_t kTileA = (kBoxA + 1023) / 1024 * 1024, kTileB = (kBoxB + 1023) / 1024 * 1024;
+    static constexpr uint32_t kW = (9u * CIN * NPAD * 2 + 1023) / 1024 * 1024;
+    static constexpr int kBX = TW / 8, kMB = kBX * J;  // block b: column b / J, row b % J
     static constexpr uint32_t kSlotCols = kMB * NPAD;
     static constexpr uint32_t kTmem = tc::tmem_cols(2 * kSlotCols);
-    static constexpr int kKSteps = 9 * CIN / 16;
     static constexpr int kThreads = 32 * (EW + 2) + (LD == LD_CONCAT ? 128 : 0);
     // Concatenated input: the half-resolution box behind a tile's halo,
-    // (TW/2+2) x (TH/2+2) pixels per 8-channel chunk, per ring stage.
+    // (TW/2+2) x (TH/2+2) pixels, per ring stage.
     static constexpr int kPh = TW / 2 + 2;
     static constexpr int kHalfPx = (TW / 2 + 2) * (TH / 2 + 2);
-    static constexpr uint32_t kHalfBox = kHalfPx * 16;
-    static constexpr uint32_t kHalfChunk = (kHalfBox + 127) / 128 * 128;
-    static constexpr uint32_t kHalfStage = LD == LD_CONCAT ? kC8 * kHalfChunk : 0;  // upper bound on chunks
+    static constexpr uint32_t kHalfBox = LD == LD_CONCAT ? kHalfPx * kCB * 2 : 0;
+    static constexpr uint32_t kStage = kTileA + kTileB + (kHalfBox + 1023) / 1024 * 1024;
+    // Outputs leave by TMA from BUFS buffers per epilogue warp, each 32
+    // pixels as NPAD / 32 swizzled tiles of 32 channels.
+    static constexpr bool kStored = EP != EP_LOGITS && EP != EP_COMPOSITE;
+    static constexpr uint32_t kOutBuf = kStored ? 32 * NPAD * 2 : 0, kOut = EW * BUFS * kOutBuf;
     static constexpr uint32_t kBars = (3 * STAGES + 4) * 8 + 16;
     static constexpr uint32_t kBias = NPAD * 4;
-    static constexpr uint32_t kSmem = 128 + kW + STAGES * (kStage + kHalfStage) + kBars + kBias;
-    static_assert(CIN % 16 == 0 && NPAD % 16 == 0 && NPAD >= 16 && NPAD <= 256, "MMA shape");
-    static_assert(TW % 8 == 0 && TH % 16 == 0 && TW + 2 <= 256 && TH + 2 <= 256, "tile shape");
+    static constexpr uint32_t kSmem = 1024 + kW + STAGES * kStage + kOut + kBars + kBias;
+    static_assert(CIN == 16 || CIN == 32 || CIN == 64 || CIN == 96, "channels as swizzled rows");
+    static_assert(NPAD == 16 || NPAD % 32 == 0, "MMA and output shape");
+    static_assert((LD == LD_PLAIN) == (CIN != 96), "loader");
+    static_assert(TW % 8 == 0 && TW + 2 <= 256 && TH + 2 <= 256, "tile shape");
+    static_assert((J < 3 ? J : 3) * NPAD <= 256, "MMA columns");
     static_assert(2 * kSlotCols <= 512, "TMEM capacity");
-    static_assert(kW % 128 == 0, "ring alignment");
-    static_assert(kChunk / 16 < (1u << 14) && kP < (1 << 14), "descriptor offset range");
     static_assert(kSmem <= 227u * 1024u, "shared memory");
     static_assert(EW == 4 || (EW == 8 && kMB % 2 == 0), "epilogue warps split the M blocks in two");
 };
+
+// The tiles that a persistent CTA takes, `stride` apart, as column, row and
+// image, stepped with carries.
+struct TileWalk
+{
+    int tilesX, tilesY, nx, ny, ni, tx, ty, img;
+    __device__ __forceinline__ TileWalk(int tilesX_, int tilesY_, int first, int stride)
+        : tilesX(tilesX_), tilesY(tilesY_), nx(stride % tilesX_), ny(stride / tilesX_ % tilesY_),
+          ni(stride / tilesX_ / tilesY_), tx(first % tilesX_), ty(first / tilesX_ % tilesY_),
+          img(first / tilesX_ / tilesY_)
+    {
+    }
+    __device__ __forceinline__ void next()
+    {
+        tx += nx;
+        ty += ny + (tx >= tilesX);
+        if (tx >= tilesX) tx -= tilesX;
+        img += ni + (ty >= tilesY);
+        if (ty >= tilesY) ty -= tilesY;
+    }
+};
+
+// Position of the 16-byte channel chunk c of pixel px in a row of C channels
+// (C * 2 bytes a pixel) under the swizzle of that width; its own inverse in c.
+template <int C>
+__device__ __forceinline__ int swizzled_chunk(int px, int c)
+{
+    return C == 64 ? c ^ (px & 7) : C == 32 ? c ^ ((px >> 1) & 3) : c ^ ((px >> 2) & 1);
+}
 
 __device__ __forceinline__ uint4 pack8_bf16(const float* v)
 {
@@ -208,40 +243,56 @@ __device__ __forceinline__ void composite_pixel(const i360b_blend_job& J, int y,
 // 3x3 convolution (forward, or backward-data with flipped transposed weights),
 // persistent and warp-specialised; CTA b handles tiles b, b + gridDim.x, ...
 //
-// The A operand of tap (dy, dx) for M block (bx, by) is the halo chunk with
-// the descriptor start moved by ((16 by + dy) kP + 8 bx + dx) * 16 bytes: the
-// 8 pixels of a block row are one core matrix (8 rows of 16 bytes) and the 16
-// block rows are core-matrix groups kP * 16 bytes apart (SBO); the two
-// 8-channel halves of a K step are one chunk apart (LBO).
+// One MMA serves three taps.  The 16 rows of M block j lie J apart, rows
+// j, j + J, ...; so the operand of its tap dy, rows j + dy, j + dy + J, ... of
+// the halo, is "set" j + dy of J + 2, and set s is the operand of blocks s - 2,
+// s - 1 and s at dy = 2, 1, 0.  Their accumulators are consecutive columns and
+// the weights of the three dy consecutive rows of B: one MMA of N = 3 NPAD per
+// set, dx and 16 channels (fewer at the first and last two sets), 3 (J + 2)
+// CIN / 16 of them instead of 9 J CIN / 16.  An MMA costs the fetch of its 4 KB
+// of A and its issue however few its columns, which bounded one MMA per tap of
+// 16..64 columns.  Sets ascend, so each accumulator still sums
+// in the order tap, channel that fixes the results' bits; the epilogue leaves
+// zeros in accumulators that it has read, as an MMA can not start one of its
+// blocks and continue two.
+//
+// The A operand of set s and dx for column block bx is the halo tile from
+// pixel (8 bx + dx, s): 8 pixels of a row are 8 swizzled rows, the 16 rows J kP
+// pixels apart (SBO), a K step 32 bytes into the row.  The swizzle is a
+// function of the address, so a window may start at any pixel.
 //
 // Roles:
-//   warp EW lane 0 TMA producer: one 4-D box (8 channels x (TW+2) x (TH+2))
-//                  per chunk into a STAGES-deep ring, zero fill outside the
-//                  image;
+//   warp EW lane 0 TMA producer: one 4-D box (channels x (TW+2) x (16J+2)) per
+//                  tile into a STAGES-deep ring, zero fill outside the image;
 //   warps EW+2..   (concatenated input only) expand the TMA-loaded
 //                  half-resolution box into the nearest-upsampled channels
 //                  of the halo (shared memory to shared memory);
-//   warp EW+1 lane 0 MMA issuer: MB x 9 CIN/16 tcgen05.mma per tile into one of
-//                  two TMEM accumulators; commits free the ring stage and
-//                  publish the accumulator;
+//   warp EW+1 lane 0 MMA issuer, into one of two sets of TMEM accumulators;
+//                  commits free the ring stage and publish the accumulators;
 //   warps 0..EW-1  epilogue (EW = 4 or 8): TMEM lanes 32q..32q+31, q = w % 4
-//                  (rows 4q..4q+3 of each M block) -> bias/ReLU, mask, raw or
-//                  blend head -> global.
+//                  (4 rows of each M block) -> bias/ReLU, mask or raw,
+//                  then by TMA from shared memory, or blend head -> global.
 // Every wait is bounded; a timeout sets the error flag and the CTA winds
 // down after its loads have landed.
+//
+// 64 windows of 256 x 256, a 32 -> 32 layer: 93 us (537 MB, 81 us at the
+// measured copy rate); with one MMA per tap, 8-channel TMA boxes and outputs
+// stored a lane's 16 bytes at a time 176 us.
 // ---------------------------------------------------------------------------
-template <int CIN, int NPAD, int TW, int TH, int STAGES, int LD, int EP, int EW>
-__global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::kThreads, 1)
-    k_conv3x3(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap tmapHalf, ConvArgs a)
+template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
+__global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW, BUFS>::kThreads, 1)
+    k_conv3x3(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+              const __grid_constant__ CUtensorMap mapOut, ConvArgs a)
 {
-    using S = ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>;
+    using S = ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW, BUFS>;
+    constexpr int TH = S::TH;
     extern __shared__ unsigned char smemRaw[];
     unsigned char* smem =
-        reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
+        reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     unsigned char* wsm = smem;
     unsigned char* ring = smem + S::kW;
-    unsigned char* halfRing = ring + STAGES * S::kStage;
-    uint64_t* full = reinterpret_cast<uint64_t*>(halfRing + STAGES * S::kHalfStage);
+    unsigned char* outBufs = ring + STAGES * S::kStage;
+    uint64_t* full = reinterpret_cast<uint64_t*>(outBufs + S::kOut);
     uint64_t* empty = full + STAGES;
     uint64_t* halfFull = empty + STAGES;
     uint64_t* accFull = halfFull + STAGES;
@@ -249,19 +300,11 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(accEmpty + 2);
     float* sBias = reinterpret_cast<float*>(tmemSlot + 4);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tilesX = (a.w + TW - 1) / TW, tilesY = (a.h + TH - 1) / TH;
     const long long nTiles = (long long)a.n * tilesX * tilesY;
     if ((long long)blockIdx.x >= nTiles) return;
     const int myTiles = (int)((nTiles - 1 - blockIdx.x) / gridDim.x) + 1;
-    auto coord = [&](int i, int& img, int& y0, int& x0) {
-        const long long t = blockIdx.x + (long long)i * gridDim.x;
-        x0 = (int)(t % tilesX) * TW;
-        const long long r = t / tilesX;
-        y0 = (int)(r % tilesY) * TH;
-        img = (int)(r / tilesY);
-    };
-    const int tmaChunks = LD == LD_CONCAT ? (a.cs >> 3) : S::kC8;
 
     if (warp == 0) tc::tmem_alloc(tmemSlot, S::kTmem);
     if (tid == 0)
@@ -280,11 +323,13 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
         tc::fence_mbar_init();
     }
     {
-        constexpr int kK8 = 9 * S::kC8;
+        // [dx][channel / 8][2 - dy][n] of 8 channels, from [n][dy][dx][channel]
+        constexpr int kC8 = CIN / 8, kK8 = 9 * kC8;
         for (int q = tid; q < NPAD * kK8; q += blockDim.x)
         {
-            const int n = q / kK8, k8 = q % kK8;
-            tc::cp_async16(wsm + k8 * (NPAD * 16) + n * 16, a.wt + (size_t)n * 9 * CIN + k8 * 8, 16);
+            const int n = q / kK8, k8 = q % kK8, tap = k8 / kC8, c8 = k8 % kC8;
+            tc::cp_async16(wsm + (((tap % 3) * kC8 + c8) * 3 + 2 - tap / 3) * (NPAD * 16) + n * 16,
+                           a.wt + (size_t)n * 9 * CIN + k8 * 8, 16);
         }
         tc::cp_async_commit();
         for (int c = tid; c < NPAD; c += blockDim.x) sBias[c] = a.bias ? a.bias[c] : 0.0f;
@@ -296,13 +341,22 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
     tc::fence_after_sync();
     const uint32_t tmem = *tmemSlot;
     bool ok = true;
+    if (warp < 4)
+    {
+        for (uint32_t c = 0; c < 2 * S::kSlotCols; c += 16) tc::tmem_zero16(tmem + ((uint32_t)(warp * 32) << 16) + c);
+        tc::tmem_wait_st();
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
 
     if (warp == S::kProducerWarp)
     {
         if (lane == 0)
         {
             int issued = 0;
-            for (int i = 0; i < myTiles; ++i)
+            TileWalk t(tilesX, tilesY, blockIdx.x, gridDim.x);
+            for (int i = 0; i < myTiles; ++i, t.next())
             {
                 const int s = i % STAGES;
                 if (!tc::mbar_wait(&empty[s], ((i / STAGES) & 1) ^ 1, kWaitSpins))
@@ -310,22 +364,18 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
                     ok = false;
                     break;
                 }
-                int img, y0, x0;
-                coord(i, img, y0, x0);
+                const int x0 = t.tx * TW, y0 = t.ty * TH;
                 unsigned char* st = ring + s * S::kStage;
                 if (LD == LD_CONCAT)
                 {
                     // half-resolution rows/columns y0/2 - 1 .. (y0 + TH)/2 (x0, y0 even)
-                    unsigned char* hs = halfRing + s * S::kHalfStage;
-                    const int nu8 = S::kC8 - tmaChunks;
-                    tc::mbar_arrive_expect_tx(&halfFull[s], (uint32_t)nu8 * S::kHalfBox);
-                    for (int c = 0; c < nu8; ++c)
-                        tc::tma_load_4d(hs + c * S::kHalfChunk, &tmapHalf, c * 8, (x0 >> 1) - 1, (y0 >> 1) - 1, img,
-                                        &halfFull[s]);
+                    tc::mbar_arrive_expect_tx(&halfFull[s], S::kHalfBox);
+                    tc::tma_load_4d(st + S::kTileA + S::kTileB, &mapB, 0, (x0 >> 1) - 1, (y0 >> 1) - 1, t.img,
+                                    &halfFull[s]);
                 }
-                tc::mbar_arrive_expect_tx(&full[s], (uint32_t)tmaChunks * S::kBox);
-                for (int c = 0; c < tmaChunks; ++c)
-                    tc::tma_load_4d(st + c * S::kChunk, &tmap, c * 8, x0 - 1, y0 - 1, img, &full[s]);
+                tc::mbar_arrive_expect_tx(&full[s], S::kBoxA + (LD == LD_SPLIT ? S::kBoxB : 0u));
+                tc::tma_load_4d(st, &mapA, 0, x0 - 1, y0 - 1, t.img, &full[s]);
+                if (LD == LD_SPLIT) tc::tma_load_4d(st + S::kTileA, &mapB, S::kCA, x0 - 1, y0 - 1, t.img, &full[s]);
                 issued = i + 1;
             }
             // The last loads must land before the CTA may exit.
@@ -338,30 +388,32 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
     }
     else if (LD == LD_CONCAT && warp >= S::kExpandWarp)
     {
-        // Nearest 2x upsample of the half-resolution box into the halo chunks
-        // after the skip channels: halo pixel (hx, hy) reads box pixel
-        // ((hx - 1) >> 1) + 1, ((hy - 1) >> 1) + 1 (tile origin even).
-        const int ptid = tid - 32 * S::kExpandWarp;
-        const int sc8 = a.cs >> 3, nu8 = S::kC8 - sc8;
+        // Nearest 2x upsample of the half-resolution box: its pixel (lx, ly)
+        // is halo columns 2 lx - 1, 2 lx and rows 2 ly - 1, 2 ly (tile origin
+        // even), those of them that there are.
+        const int c = tid & 7;
         for (int i = 0; i < myTiles; ++i)
         {
             const int s = i % STAGES;
-            bool got = tc::mbar_wait(&halfFull[s], (i / STAGES) & 1, kWaitSpins);
-            if (!got)
+            if (!tc::mbar_wait(&halfFull[s], (i / STAGES) & 1, kWaitSpins))
             {
                 ok = false;
                 break;
             }
-            const unsigned char* hs = halfRing + s * S::kHalfStage;
-            unsigned char* st = ring + s * S::kStage;
-            const int nq = nu8 * S::kHaloPx;
-            for (int q = ptid; q < nq; q += 128)
+            unsigned char* up = ring + s * S::kStage + S::kTileA;
+            const unsigned char* half = up + S::kTileB;
+            for (int hp = (tid - 32 * S::kExpandWarp) >> 3; hp < S::kHalfPx; hp += 16)
             {
-                const int cu = q / S::kHaloPx, px = q - cu * S::kHaloPx;
-                const int hy = px / S::kP, hx = px - hy * S::kP;
-                const int ly = ((hy - 1) >> 1) + 1, lx = ((hx - 1) >> 1) + 1;
-                *reinterpret_cast<uint4*>(st + (sc8 + cu) * S::kChunk + px * 16) =
-                    *reinterpret_cast<const uint4*>(hs + cu * S::kHalfChunk + (ly * S::kPh + lx) * 16);
+                const int ly = hp / S::kPh, lx = hp - ly * S::kPh;
+                const uint4 v = *reinterpret_cast<const uint4*>(half + hp * 128 + swizzled_chunk<64>(hp, c) * 16);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    const int hy = 2 * ly - 1 + (k >> 1), hx = 2 * lx - 1 + (k & 1);
+                    if (hy < 0 || hy > TH + 1 || hx < 0 || hx > TW + 1) continue;
+                    const int px = hy * S::kP + hx;
+                    *reinterpret_cast<uint4*>(up + px * 128 + swizzled_chunk<64>(px, c) * 16) = v;
+                }
             }
             tc::fence_proxy_async();  // generic smem writes -> tensor core
             tc::mbar_arrive(&full[s]);
@@ -369,15 +421,19 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
     }
     else if (warp == S::kMmaWarp)
     {
-        if (lane == 0)
+        // The whole warp runs the loop and one thread of it issues: operands
+        // then stay in uniform registers.  From one thread's branch each MMA
+        // took 70 cycles to issue, whatever its size.
         {
-            constexpr uint32_t idesc = tc::idesc_bf16_f32(128, NPAD);
-            const uint64_t bBase = tc::smem_desc(tc::smem_u32(wsm), NPAD * 16, 128);
+            const bool leader = tc::elect_one();
+            const uint32_t tmemU = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint64_t bBase = tc::smem_desc(tc::smem_u32(wsm), 3 * NPAD * 16, 128);
             for (int i = 0; i < myTiles; ++i)
             {
                 const int s = i % STAGES, acc = i & 1;
-                if (!tc::mbar_wait(&full[s], (i / STAGES) & 1, kWaitSpins) ||
-                    !tc::mbar_wait(&accEmpty[acc], ((i >> 1) & 1) ^ 1, kWaitSpins))
+                const bool ready = tc::mbar_wait(&full[s], (i / STAGES) & 1, kWaitSpins) &&
+                                   tc::mbar_wait(&accEmpty[acc], ((i >> 1) & 1) ^ 1, kWaitSpins);
+                if (!__all_sync(0xffffffffu, ready))
                 {
                     ok = false;
                     break;
@@ -385,24 +441,34 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
                 tc::fence_after_sync();
                 // Descriptors differ only in their start-address field: add
                 // the (compile-time) offset in 16-byte units to a base.
-                const uint64_t aBase = tc::smem_desc(tc::smem_u32(ring + s * S::kStage), S::kChunk, S::kP * 16);
+                const uint32_t st = tc::smem_u32(ring + s * S::kStage);
+                const uint64_t aBase = tc::smem_desc_k<S::kCA>(st, J * S::kP * S::kCA * 2);
+                const uint64_t a2Base = tc::smem_desc_k<64>(st + S::kTileA, J * S::kP * 64 * 2);
 #pragma unroll
-                for (int b = 0; b < S::kMB; ++b)
-                {
-                    const int bx = b % S::kBX, by = b / S::kBX;
-                    const uint32_t d = tmem + acc * S::kSlotCols + b * NPAD;
+                for (int bx = 0; bx < S::kBX; ++bx)
 #pragma unroll
-                    for (int ks = 0; ks < S::kKSteps; ++ks)
+                    for (int set = 0; set < J + 2; ++set)
                     {
-                        const int k0 = ks * 16, tap = k0 / CIN, c8 = (k0 % CIN) >> 3;
-                        const int dy = tap / 3, dx = tap % 3;
-                        const uint32_t aOff = (c8 * S::kChunk + ((by * 16 + dy) * S::kP + bx * 8 + dx) * 16) >> 4;
-                        const uint32_t bOff = (2 * ks * (NPAD * 16)) >> 4;
-                        tc::mma_bf16(d, aBase + aOff, bBase + bOff, idesc, ks > 0 ? 1u : 0u);
+                        const int j0 = set > 2 ? set - 2 : 0, j1 = set < J ? set : J - 1;  // blocks of the set
+                        const uint32_t d = tmemU + acc * S::kSlotCols + (bx * J + j0) * NPAD;
+                        const uint32_t idesc = tc::idesc_bf16_f32(128, (j1 - j0 + 1) * NPAD);
+#pragma unroll
+                        for (int k0 = 0; k0 < 3 * CIN; k0 += 16)
+                        {
+                            const int dx = k0 / CIN, c = k0 % CIN;
+                            const uint32_t px = set * S::kP + bx * 8 + dx;
+                            const uint64_t aDesc = c < S::kCA ? aBase + ((px * S::kCA * 2 + c * 2) >> 4)
+                                                              : a2Base + ((px * 128 + (c - S::kCA) * 2) >> 4);
+                            const uint32_t bRow = (k0 / 8) * 3 * NPAD + (2 - (set - j0)) * NPAD;
+                            if (leader) tc::mma_bf16(d, aDesc, bBase + bRow, idesc, 1u);
+                        }
                     }
+                if (leader)
+                {
+                    tc::mma_commit(&empty[s]);
+                    tc::mma_commit(&accFull[acc]);
                 }
-                tc::mma_commit(&empty[s]);
-                tc::mma_commit(&accFull[acc]);
+                __syncwarp();
             }
         }
     }
@@ -411,29 +477,21 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
         // Warp w reads TMEM lane quadrant w % 4; with 8 epilogue warps the
         // two warps of a quadrant take alternate M blocks.
         const int quad = warp & 3, half = warp >> 2;
-        for (int i = 0; i < myTiles; ++i)
+        unsigned char* buf = outBufs + warp * (BUFS * S::kOutBuf);
+        int next = 0;  // output buffer
+        TileWalk t(tilesX, tilesY, blockIdx.x, gridDim.x);
+        for (int i = 0; i < myTiles && ok; ++i, t.next())
         {
-            const int acc = i & 1;
-            bool done = tc::mbar_wait(&accFull[acc], (i >> 1) & 1, kWaitSpins);
-            done = __all_sync(0xffffffffu, done);
-            if (!done)
-            {
-                ok = false;
-                break;
-            }
-            tc::fence_after_sync();
-            int img, y0, x0;
-            coord(i, img, y0, x0);
+            const int acc = i & 1, img = t.img;
             const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + acc * S::kSlotCols;
             for (int b = (EW == 8 ? half : 0); b < S::kMB; b += EW / 4)
             {
-                const int bx = b % S::kBX, by = b / S::kBX;
-                const int y = y0 + by * 16 + quad * 4 + (lane >> 3);
-                const int x = x0 + bx * 8 + (lane & 7);
+                const int yq = t.ty * TH + b % J + 4 * J * quad, xq = t.tx * TW + b / J * 8;
+                const int y = yq + J * (lane >> 3), x = xq + (lane & 7);
                 const bool valid = y < a.h && x < a.w;
                 const size_t pix = ((size_t)img * a.h + y) * a.w + x;
                 // Global inputs of the epilogue first, so their latency
-                // overlaps the TMEM loads.
+                // overlaps the wait and the TMEM loads.
                 float vv[4][3];
                 bool inJob = false;
                 if (EP == EP_COMPOSITE)
@@ -449,6 +507,16 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
 #pragma unroll
                     for (int q = 0; q < NPAD / 8; ++q) mk[q] = ap[q];
                 }
+                if (b < EW / 4)
+                {
+                    const bool done = tc::mbar_wait(&accFull[acc], (i >> 1) & 1, kWaitSpins);
+                    if (!__all_sync(0xffffffffu, done))
+                    {
+                        ok = false;
+                        break;
+                    }
+                    tc::fence_after_sync();
+                }
                 constexpr int kCols = (EP == EP_LOGITS || EP == EP_COMPOSITE) ? 16 : NPAD;
                 uint32_t r[kCols];
 #pragma unroll
@@ -456,7 +524,15 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
                 tc::tmem_wait_ld();
 #pragma unroll
                 for (int cb = 0; cb < kCols / 16; ++cb) tc::tmem_reg_fence16(r + cb * 16);
-                if (!valid) continue;
+#pragma unroll
+                for (int cb = 0; cb < NPAD / 16; ++cb) tc::tmem_zero16(base + b * NPAD + cb * 16);
+                tc::tmem_wait_st();
+                if (b + EW / 4 >= S::kMB)
+                {
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive(&accEmpty[acc]);
+                }
                 if (EP == EP_LOGITS || EP == EP_COMPOSITE)
                 {
                     float l[4];
@@ -464,7 +540,7 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
                     for (int j = 0; j < 4; ++j) l[j] = __uint_as_float(r[j]) + sBias[j];
                     if (EP == EP_LOGITS)
                     {
-                        reinterpret_cast<float4*>(a.out)[pix] = make_float4(l[0], l[1], l[2], l[3]);
+                        if (valid) reinterpret_cast<float4*>(a.out)[pix] = make_float4(l[0], l[1], l[2], l[3]);
                     }
                     else if (inJob)
                     {
@@ -481,35 +557,49 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>::
                 }
                 else
                 {
+                    unsigned char* ob = buf + next * S::kOutBuf;
+                    if (BUFS > 1) next = next + 1 == BUFS ? 0 : next + 1;
+                    if (lane == 0) tc::bulk_wait_read<BUFS - 1>();
+                    __syncwarp();
 #pragma unroll
-                    for (int cb = 0; cb < NPAD / 16; ++cb)
+                    for (int c8 = 0; c8 < NPAD / 8; ++c8)
                     {
-                        float v[16];
+                        float v[8];
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[cb * 16 + j]);
+                        for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[c8 * 8 + j]);
                         if (EP == EP_RELU)
                         {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j] + sBias[cb * 16 + j], 0.0f);
+                            for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j] + sBias[c8 * 8 + j], 0.0f);
                         }
                         if (EP == EP_MASK)
                         {
-                            float m[16];
-                            unpack8_bf16(mk[2 * cb], m);
-                            unpack8_bf16(mk[2 * cb + 1], m + 8);
+                            float m[8];
+                            unpack8_bf16(mk[c8], m);
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = m[j] > 0.0f ? v[j] : 0.0f;
+                            for (int j = 0; j < 8; ++j) v[j] = m[j] > 0.0f ? v[j] : 0.0f;
                         }
-                        uint4* op = reinterpret_cast<uint4*>(static_cast<bf16*>(a.out) + pix * NPAD + cb * 16);
-                        op[0] = pack8_bf16(v);
-                        op[1] = pack8_bf16(v + 8);
+                        *reinterpret_cast<uint4*>(ob + (c8 >> 2) * 2048 + lane * 64 +
+                                                  swizzled_chunk<32>(lane, c8 & 3) * 16) = pack8_bf16(v);
                     }
+                    tc::fence_proxy_async();  // generic smem writes -> TMA
+                    __syncwarp();
+                    if (lane == 0 && yq < a.h && xq < a.w)
+                    {
+                        for (int u = 0; u < NPAD / 32; ++u)
+                        {
+                            if (a.rowSplit)  // 4 rows J apart as rows / J of the map
+                                tc::tma_store_5d(&mapOut, ob + u * 2048, u * 32, xq, yq % J, yq / J, img);
+                            else
+                                for (int k = 0; k < 4 && yq + J * k < a.h; ++k)
+                                    tc::tma_store_5d(&mapOut, ob + u * 2048 + k * 512, u * 32, xq, yq + J * k, 0, img);
+                        }
+                    }
+                    if (lane == 0) tc::bulk_commit();
                 }
             }
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&accEmpty[acc]);
         }
+        if (S::kStored && lane == 0) tc::bulk_wait_all();
     }
     if (!ok) atomicOr(a.error, 1);
     tc::fence_before_sync();
@@ -619,14 +709,6 @@ struct WgradShape
     static_assert(kStages >= 2 && kSmem <= 227u * 1024u, "shared memory");
 };
 
-// Position of the 16-byte channel chunk c of pixel px in a row of C channels
-// (C * 2 bytes a pixel) under the swizzle of that width; its own inverse in c.
-template <int C>
-__device__ __forceinline__ int swizzled_chunk(int px, int c)
-{
-    return C == 64 ? c ^ (px & 7) : C == 32 ? c ^ ((px >> 1) & 3) : c ^ ((px >> 2) & 1);
-}
-
 template <int CX, int COUT, bool UP>
 __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float (&sBias)[128][9], int* error)
 {
@@ -639,7 +721,7 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
     uint64_t* halfFull = empty + S::kStages;
     uint64_t* done = halfFull + S::kStages;
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(done + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tilesX = a.w / kWgTW, tilesY = (a.h + kWgRows - 1) / kWgRows;
     const long long nTiles = (long long)a.n * tilesX * tilesY;  // >= a.slices
     const int myTiles = (int)((nTiles - 1 - slice) / a.slices) + 1;
@@ -669,10 +751,7 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
         if (lane == 0)
         {
             int issued = 0;
-            // Tile (tx, ty, img), stepped by a.slices tiles with carries: this
-            // one thread's divisions per tile took longer than its copies.
-            const int nx = a.slices % tilesX, ny = a.slices / tilesX % tilesY, ni = a.slices / tilesX / tilesY;
-            int tx = slice % tilesX, ty = slice / tilesX % tilesY, img = slice / tilesX / tilesY;
+            TileWalk t(tilesX, tilesY, slice, a.slices);
             int s = -1;
             uint32_t phase = 0;  // of the empty barrier: one before the first use
             for (int i = 0; i < myTiles; ++i)
@@ -684,22 +763,18 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
                     ok = false;
                     break;
                 }
-                const int x0 = tx * kWgTW, y0 = ty * kWgRows;
+                const int x0 = t.tx * kWgTW, y0 = t.ty * kWgRows;
                 unsigned char* st = smem + s * S::kStage;
                 if (UP)
                 {
                     tc::mbar_arrive_expect_tx(&halfFull[s], S::kHalf);
-                    tc::tma_load_4d(st + S::kX + S::kG, &a.mapX, a.xc0, x0 >> 1, (y0 >> 1) - 1, img, &halfFull[s]);
+                    tc::tma_load_4d(st + S::kX + S::kG, &a.mapX, a.xc0, x0 >> 1, (y0 >> 1) - 1, t.img, &halfFull[s]);
                 }
                 tc::mbar_arrive_expect_tx(&full[s], (UP ? 0u : S::kXRows * S::kXRow) + 3 * S::kGCopy);
-                if (!UP) tc::tma_load_4d(st, &a.mapX, a.xc0, x0, y0 - 1, img, &full[s]);
+                if (!UP) tc::tma_load_4d(st, &a.mapX, a.xc0, x0, y0 - 1, t.img, &full[s]);
                 for (int dx = 0; dx < 3; ++dx)
-                    tc::tma_load_4d(st + S::kX + dx * S::kGCopy, &a.mapG, 0, x0 - (dx - 1), y0, img, &full[s]);
-                tx += nx;
-                ty += ny + (tx >= tilesX);
-                if (tx >= tilesX) tx -= tilesX;
-                img += ni + (ty >= tilesY);
-                if (ty >= tilesY) ty -= tilesY;
+                    tc::tma_load_4d(st + S::kX + dx * S::kGCopy, &a.mapG, 0, x0 - (dx - 1), y0, t.img, &full[s]);
+                t.next();
                 issued = i + 1;
             }
             // The last loads must land before the CTA may exit.
@@ -713,13 +788,16 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
     }
     else if (warp == 5)
     {
-        if (lane == 0)
+        // (the whole warp, so that operands stay in uniform registers)
         {
+            const bool leader = tc::elect_one();
+            const uint32_t tmemU = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t idesc = tc::idesc_bf16_f32(128, S::kN) | (1u << 15) | (1u << 16);  // A, B MN-major
             for (int i = 0; i < myTiles; ++i)
             {
                 const int s = i % S::kStages;
-                if (!tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins))
+                const bool ready = tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins);
+                if (!__all_sync(0xffffffffu, ready))
                 {
                     ok = false;
                     break;
@@ -732,12 +810,14 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
                 for (int r = 0; r < kWgRows; ++r)
 #pragma unroll
                     for (int k = 0; k < kWgTW / 16; ++k)
-                        tc::mma_bf16(tmem, aBase + ((r * S::kXRow + k * 16 * CX * 2) >> 4),
-                                     bBase + ((r * S::kGRow + k * 16 * COUT * 2) >> 4), idesc,
-                                     (i > 0 || r > 0 || k > 0) ? 1u : 0u);
-                tc::mma_commit(&empty[s]);
+                        if (leader)
+                            tc::mma_bf16(tmemU, aBase + ((r * S::kXRow + k * 16 * CX * 2) >> 4),
+                                         bBase + ((r * S::kGRow + k * 16 * COUT * 2) >> 4), idesc,
+                                         (i > 0 || r > 0 || k > 0) ? 1u : 0u);
+                if (leader) tc::mma_commit(&empty[s]);
+                __syncwarp();
             }
-            tc::mma_commit(done);
+            if (leader) tc::mma_commit(done);
         }
     }
     else if (helpers)
@@ -1205,12 +1285,13 @@ int elementwise_grid(long long n, int block = 256)
     return (int)std::max<long long>(1, std::min<long long>((n + block - 1) / block, (long long)sm_count() * 16));
 }
 
-// Tensor map of an NHWC bf16 tensor as (C, W, H, N) with a box of boxC
-// channels x boxW x boxH x 1 (zero fill outside) under a shared-memory
-// swizzle.  The encoder comes from the driver through the runtime (no link
-// against the driver library).
-int make_tile_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxC, int boxW, int boxH,
-                  CUtensorMapSwizzle swizzle)
+// Tensor map of bf16 values (zero fill outside) under a shared-memory swizzle;
+// dims[0] is the contiguous one, stride[i] that of dims[i + 1] in values.  The
+// encoder comes from the driver through the runtime (no link against the
+// driver library).
+template <int RANK>
+int make_map(CUtensorMap* m, const bf16* base, const long long (&dims)[RANK], const long long (&stride)[RANK - 1],
+             const int (&box)[RANK], CUtensorMapSwizzle swizzle)
 {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     static std::once_flag once;
@@ -1222,81 +1303,42 @@ int make_tile_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, 
         if (err == cudaSuccess && q != cudaDriverEntryPointSuccess) err = cudaErrorSymbolNotFound;
     });
     if (err != cudaSuccess || !encode) return cuda_fail(err, "cuTensorMapEncodeTiled entry point");
-    if ((reinterpret_cast<uintptr_t>(base) & 15) || c % 8)
-        return fail(I360B_INVALID_PARAM, "conv3x3 input must be 16-byte aligned with channels a multiple of 8");
-    const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
-    const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
-    const cuuint32_t box[4] = {(cuuint32_t)boxC, (cuuint32_t)boxW, (cuuint32_t)boxH, 1};
-    const cuuint32_t es[4] = {1, 1, 1, 1};
-    CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(base), dims, strides, box, es,
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || dims[0] % 8)
+        return fail(I360B_INVALID_PARAM, "conv3x3 tensors must be 16-byte aligned with channels a multiple of 8");
+    cuuint64_t d[RANK], st[RANK - 1];
+    cuuint32_t bx[RANK], es[RANK];
+    for (int i = 0; i < RANK; ++i)
+    {
+        d[i] = (cuuint64_t)dims[i];
+        bx[i] = (cuuint32_t)box[i];
+        es[i] = 1;
+        if (i + 1 < RANK) st[i] = (cuuint64_t)stride[i] * sizeof(bf16);
+    }
+    CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, RANK, const_cast<bf16*>(base), d, st, bx, es,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(I360B_CUDA_ERROR, "cuTensorMapEncodeTiled failed (%d)", (int)r);
     return I360B_SUCCESS;
 }
 
-// The convolutions' 8-channel boxes.
-int make_input_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxW, int boxH)
+// An NHWC tensor as (C, W, H, N) with boxes of boxC x boxW x boxH x 1.
+int make_tile_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxC, int boxW, int boxH,
+                  CUtensorMapSwizzle swizzle)
 {
-    return make_tile_map(m, base, c, n, h, w, 8, boxW, boxH, CU_TENSOR_MAP_SWIZZLE_NONE);
+    const long long row = (long long)w * c;
+    return make_map<4>(m, base, {c, w, h, n}, {c, row, h * row}, {boxC, boxW, boxH, 1}, swizzle);
 }
 
-template <int CIN, int NPAD, int TW, int TH, int STAGES, int LD, int EP, int EW>
-int run_conv(const ConvArgs& a, cudaStream_t s)
+// A convolution's output, 32 channels of 8 x 4 pixels at a time: rows
+// split > 0 apart as (C, W, split, H / split, N), or (split = 0) a row at a
+// time as (C, W, H, 1, N).
+int make_output_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int split)
 {
-    using S = ConvShape<CIN, NPAD, TW, TH, STAGES, LD, EW>;
-    static std::once_flag once;
-    static int perSm = 1;
-    static cudaError_t attrErr = cudaSuccess;
-    std::call_once(once, [] {
-        auto* k = k_conv3x3<CIN, NPAD, TW, TH, STAGES, LD, EP, EW>;
-        attrErr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
-        int occ = 1;
-        if (attrErr == cudaSuccess)
-            attrErr = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, S::kThreads, S::kSmem);
-        perSm = std::max(1, std::min<int>(occ, 512 / (int)S::kTmem));
-    });
-    if (attrErr != cudaSuccess) return cuda_fail(attrErr, "conv3x3 attributes");
-    const long long tiles = (long long)a.n * ((a.h + TH - 1) / TH) * ((a.w + TW - 1) / TW);
-    if (tiles == 0) return I360B_SUCCESS;
-    CUtensorMap tm, th;
-    I360B_TRY(make_input_map(&tm, a.x, LD == LD_CONCAT ? a.cs : CIN, a.n, a.h, a.w, TW + 2, TH + 2));
-    if (LD == LD_CONCAT)
-    {
-        if (a.cs % 8 || a.h % 2 || a.w % 2 || CIN - a.cs > 8 * S::kC8)
-            return fail(I360B_INVALID_PARAM, "concatenated conv3x3 input: even sizes and 8-channel groups");
-        I360B_TRY(make_input_map(&th, a.u, CIN - a.cs, a.n, a.h / 2, a.w / 2, TW / 2 + 2, TH / 2 + 2));
-    }
-    else
-        th = tm;
-    k_conv3x3<CIN, NPAD, TW, TH, STAGES, LD, EP, EW><<<grid_for(tiles, perSm), S::kThreads, S::kSmem, s>>>(tm, th, a);
-    return check_launch("conv3x3 kernel");
-}
-
-// The (cin, npad) shapes the network uses, forward and backward, with their
-// tile shape and ring depth.
-int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cudaStream_t s)
-{
-#define I360B_CONV(CI, NP, TW, TH, ST, LD, EP_, EW)             \
-    if (cin == CI && npad == NP && loader == LD && ep == EP_) \
-        return run_conv<CI, NP, TW, TH, ST, LD, EP_, EW>(a, s);
-    // forward
-    I360B_CONV(16, 32, 32, 32, 3, LD_PLAIN, EP_RELU, 8)
-    I360B_CONV(32, 32, 16, 32, 3, LD_PLAIN, EP_RELU, 8)
-    I360B_CONV(32, 64, 16, 32, 3, LD_PLAIN, EP_RELU, 8)
-    I360B_CONV(64, 64, 16, 16, 3, LD_PLAIN, EP_RELU, 8)
-    I360B_CONV(96, 32, 16, 16, 2, LD_CONCAT, EP_RELU, 8)
-    I360B_CONV(32, 16, 32, 32, 2, LD_PLAIN, EP_LOGITS, 8)
-    I360B_CONV(32, 16, 32, 32, 2, LD_PLAIN, EP_COMPOSITE, 8)
-    // backward data
-    I360B_CONV(16, 32, 32, 32, 3, LD_PLAIN, EP_MASK, 8)
-    I360B_CONV(32, 32, 16, 32, 3, LD_PLAIN, EP_MASK, 8)
-    I360B_CONV(32, 96, 16, 16, 3, LD_PLAIN, EP_RAW, 8)
-    I360B_CONV(64, 64, 16, 16, 3, LD_PLAIN, EP_MASK, 8)
-    I360B_CONV(64, 32, 16, 16, 3, LD_PLAIN, EP_RAW, 8)
-#undef I360B_CONV
-    return fail(I360B_NOT_SUPPORTED, "conv3x3: no kernel for cin=%d cout=%d loader=%d epilogue=%d", cin, npad, loader,
-                ep);
+    const long long row = (long long)w * c;
+    return split > 0 ? make_map<5>(m, base, {c, w, split, h / split, n}, {c, row, split * row, h * row}, {32, 8, 1, 4, 1},
+                                   CU_TENSOR_MAP_SWIZZLE_64B)
+                     : make_map<5>(m, base, {c, w, h, 1, n}, {c, row, h * row, h * row}, {32, 8, 1, 1, 1},
+                                   CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 constexpr CUtensorMapSwizzle swizzle_of(int channels)
@@ -1304,6 +1346,62 @@ constexpr CUtensorMapSwizzle swizzle_of(int channels)
     return channels == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
            : channels == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
                             : CU_TENSOR_MAP_SWIZZLE_32B;
+}
+
+template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
+int run_conv(ConvArgs a, cudaStream_t s)
+{
+    using S = ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW, BUFS>;
+    auto* k = k_conv3x3<CIN, NPAD, TW, J, STAGES, LD, EP, EW, BUFS>;
+    static std::once_flag once;
+    static cudaError_t attrErr = cudaSuccess;
+    std::call_once(once, [&] {
+        attrErr = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem);
+    });
+    if (attrErr != cudaSuccess) return cuda_fail(attrErr, "conv3x3 attributes");
+    constexpr int TH = S::TH;
+    const long long tiles = (long long)a.n * ((a.h + TH - 1) / TH) * ((a.w + TW - 1) / TW);
+    if (tiles == 0) return I360B_SUCCESS;
+    CUtensorMap ma, mb, mo;
+    I360B_TRY(make_tile_map(&ma, a.x, LD == LD_CONCAT ? a.cs : CIN, a.n, a.h, a.w, S::kCA, TW + 2, TH + 2,
+                            swizzle_of(S::kCA)));
+    mb = mo = ma;
+    if (LD == LD_CONCAT)
+        I360B_TRY(make_tile_map(&mb, a.u, S::kCB, a.n, a.h / 2, a.w / 2, S::kCB, TW / 2 + 2, TH / 2 + 2,
+                                swizzle_of(S::kCB)));
+    if (LD == LD_SPLIT)
+        I360B_TRY(make_tile_map(&mb, a.x, CIN, a.n, a.h, a.w, S::kCB, TW + 2, TH + 2, swizzle_of(S::kCB)));
+    a.rowSplit = a.h % J == 0;
+    if (S::kStored)
+        I360B_TRY(make_output_map(&mo, static_cast<const bf16*>(a.out), NPAD, a.n, a.h, a.w, a.rowSplit ? J : 0));
+    k<<<grid_for(tiles, 1), S::kThreads, S::kSmem, s>>>(ma, mb, mo, a);
+    return check_launch("conv3x3 kernel");
+}
+
+// The (cin, npad) shapes the network uses, forward and backward, with their
+// tile shape and ring depth.
+int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cudaStream_t s)
+{
+#define I360B_CONV(CI, NP, TW, J, ST, LD, EP_, EW, BUFS)      \
+    if (cin == CI && npad == NP && loader == LD && ep == EP_) \
+        return run_conv<CI, NP, TW, J, ST, LD, EP_, EW, BUFS>(a, s);
+    I360B_CONV(16, 32, 16, 4, 3, LD_PLAIN, EP_RELU, 8, 2)
+    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_RELU, 8, 2)
+    I360B_CONV(32, 64, 8, 4, 3, LD_PLAIN, EP_RELU, 8, 1)
+    I360B_CONV(64, 64, 8, 2, 2, LD_PLAIN, EP_RELU, 8, 1)
+    I360B_CONV(96, 32, 8, 2, 2, LD_CONCAT, EP_RELU, 4, 1)
+    I360B_CONV(96, 32, 8, 2, 2, LD_SPLIT, EP_RELU, 4, 1)
+    I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_LOGITS, 8, 1)
+    I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_COMPOSITE, 8, 1)
+    // backward data
+    I360B_CONV(16, 32, 16, 4, 3, LD_PLAIN, EP_MASK, 8, 2)
+    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_MASK, 8, 2)
+    I360B_CONV(32, 96, 8, 2, 3, LD_PLAIN, EP_RAW, 8, 1)
+    I360B_CONV(64, 64, 8, 2, 2, LD_PLAIN, EP_MASK, 8, 1)
+    I360B_CONV(64, 32, 8, 4, 2, LD_PLAIN, EP_RAW, 8, 1)
+#undef I360B_CONV
+    return fail(I360B_NOT_SUPPORTED, "conv3x3: no kernel for cin=%d cout=%d loader=%d epilogue=%d", cin, npad, loader,
+                ep);
 }
 
 // Slices of a layer's sums at most: one 128-row block of (tap, cin) per SM.
@@ -1399,6 +1497,21 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
     I360B_TRY(check_launch("wgrad kernel"));
     k_wgrad_reduce<<<reduceBlocks, 128, 0, s>>>(r);
     return check_launch("wgrad reduce kernel");
+}
+
+// The concatenation as a tensor of its own (dev_free it on `s`).
+int concatenate(const bf16* x, const bf16* u, int cs, int cin, int n, int h, int w, void** out, cudaStream_t s)
+{
+    const long long units = (long long)n * h * w * (cin / 8);
+    I360B_TRY(dev_alloc(out, (size_t)units * 16, s, "concatenated input"));
+    k_concat<<<elementwise_grid(units), 256, 0, s>>>(x, u, cs, cin, n, h, w, static_cast<bf16*>(*out));
+    const int rc = check_launch("concatenation kernel");
+    if (rc != I360B_SUCCESS)
+    {
+        dev_free(*out, s);
+        *out = nullptr;
+    }
+    return rc;
 }
 
 int check_window(int n, int w, int h)
@@ -2022,7 +2135,18 @@ extern "C" int i360b_conv3x3_forward(const void* dX, const void* dU, int skipCha
     a.error = dErr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     I360B_CUDA(cudaMemsetAsync(dErr, 0, sizeof(int), s), "error flag");
-    I360B_TRY(dispatch_conv(cin, cout, skipChannels > 0 ? LD_CONCAT : LD_PLAIN, epilogue, a, s));
+    int loader = skipChannels > 0 ? LD_CONCAT : LD_PLAIN;
+    void* full = nullptr;
+    if (loader == LD_CONCAT && cin == 96 && cout == 32 && epilogue == EP_RELU && skipChannels != 32)
+    {
+        // a skip other than the first tile's 32 channels: concatenate first
+        I360B_TRY(concatenate(a.x, a.u, skipChannels, cin, n, h, w, &full, s));
+        a.x = static_cast<const bf16*>(full);
+        loader = LD_SPLIT;
+    }
+    const int rc = dispatch_conv(cin, cout, loader, epilogue, a, s);
+    if (full) dev_free(full, s);
+    if (rc != I360B_SUCCESS) return rc;
     int e = 0;
     I360B_CUDA(cudaMemcpyAsync(&e, dErr, sizeof(int), cudaMemcpyDeviceToHost, s), "error flag");
     I360B_CUDA(cudaStreamSynchronize(s), "conv3x3");
@@ -2057,13 +2181,7 @@ extern "C" int i360b_conv3x3_wgrad(const void* dX, const void* dU, int skipChann
     else if (cin == 96 && cout == 32 && L.cs % 32)
     {
         // a skip that is not whole 32-channel jobs: concatenate first
-        const long long units = (long long)n * h * w * (cin / 8);
-        rc = dev_alloc(&full, (size_t)units * 16, s, "wgrad concatenation");
-        if (rc == I360B_SUCCESS)
-        {
-            k_concat<<<elementwise_grid(units), 256, 0, s>>>(L.x, L.u, L.cs, cin, n, h, w, static_cast<bf16*>(full));
-            rc = check_launch("concatenation kernel");
-        }
+        rc = concatenate(L.x, L.u, L.cs, cin, n, h, w, &full, s);
         L.x = static_cast<const bf16*>(full);
         L.cs = 0;
     }

@@ -49,6 +49,23 @@ __device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr, uint32_t atom)
     return d;
 }
 
+// Shared-memory matrix descriptor, K-major, rows of C = 16, 32 or 64 bf16
+// values of K in the swizzle of that width: 8 rows follow each other, the next
+// 8 lie sbo bytes further.  The swizzle is a function of the address (pattern
+// aligned to 8 rows), so the start may be any row, and any 32 bytes in it.
+template <int C>
+__device__ __forceinline__ uint64_t smem_desc_k(uint32_t addr, uint32_t sbo)
+{
+    static_assert(C == 16 || C == 32 || C == 64, "swizzle width");
+    uint64_t d = 0;
+    d |= (uint64_t)((addr >> 4) & 0x3fffu);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)((sbo >> 4) & 0x3fffu) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)(C == 64 ? 2 : C == 32 ? 4 : 6) << 61;
+    return d;
+}
+
 // Instruction descriptor of kind::f16: BF16 x BF16 -> F32, both K-major.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N)
 {
@@ -79,6 +96,20 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, one thread.
+// True in one thread of the (converged) warp.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t p;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ void mma_bf16(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accum)
 {
     asm volatile(
@@ -156,6 +187,17 @@ __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* r)
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
+// Zeros into 16 consecutive TMEM columns of this warp's 32 lanes.
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr)
+{
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::
+            "r"(taddr),
+        "r"(0u)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Ties 16 registers written by tmem_ld16_nowait to a preceding tmem_wait_ld():
 // an empty statement that "modifies" them, so no use can be scheduled before
@@ -216,6 +258,25 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0,
 }
 
 // TMEM allocation size: a power of two of at least 32 columns.
+// One tiled TMA store of a box (bulk group of the issuing thread; parts
+// outside the tensor are left out).
+__device__ __forceinline__ void tma_store_5d(const void* tmap, const void* src, int c0, int c1, int c2, int c3, int c4)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5, %6}], [%1];\n" ::"l"(
+            reinterpret_cast<uint64_t>(tmap)),
+        "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+        : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Until at most N of this thread's groups still read shared memory.
+template <int N>
+__device__ __forceinline__ void bulk_wait_read()
+{
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 __host__ __device__ constexpr uint32_t tmem_cols(uint32_t n)
 {
     return n <= 32 ? 32u : n <= 64 ? 64u : n <= 128 ? 128u : n <= 256 ? 256u : 512u;

@@ -340,3 +340,39 @@ def test_conv3x3_wgrad_tile_edges(backend, cin, cout, skip, n, h, w):
     ref = torch.stack([torch.stack([torch.einsum("nhwo,nhwi->oi", g.double(), xp[:, ky:ky + h, kx:kx + w])
                                     for kx in range(3)], 1) for ky in range(3)], 1)
     assert float((out.double() - ref).abs().max()) <= 1e-4 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("cin,cout,ep,skip", [(i, o, e, 32 if c else 0) for i, o, e, c in CONV_CASES] +
+                         [(96, 32, 0, 8), (96, 32, 0, 64)])
+@pytest.mark.parametrize("n,h,w", [(1, 2, 256), (2, 66, 256), (1, 130, 512), (3, 37, 24)])
+def test_conv3x3_forward_tile_edges(backend, cin, cout, ep, skip, n, h, w):
+    """Heights and widths around the 32- and 64-row tiles, heights that are not
+    a multiple of the rows' interleave, other splits of the concatenation.
+    Bounds as above."""
+    import torch
+    from image360_b200 import blendnet as bn
+    if skip and (h % 2 or w % 256):
+        pytest.skip("concatenated inputs have even heights and whole windows")
+    rng = np.random.default_rng(cin * 1000 + cout * 10 + ep + h)
+    if skip:
+        x, u = _bf((n, h, w, skip), rng), _bf((n, h // 2, w // 2, cin - skip), rng)
+        full = torch.cat([x, u.repeat_interleave(2, 1).repeat_interleave(2, 2)], -1)
+    else:
+        x, u = _bf((n, h, w, cin), rng), None
+        full = x
+    W = _bf((cout, 3, 3, cin), rng, 1.0 / np.sqrt(9 * cin))
+    b = _t(rng.standard_normal(cout).astype(np.float32) * 0.1)
+    act = _bf((n, h, w, cout), rng) if ep == 2 else None
+    out = torch.full((n, h, w, 4 if ep == 1 else cout), float("nan"),
+                     dtype=torch.float32 if ep == 1 else torch.bfloat16, device="cuda")
+    bn.conv3x3_forward(x, W, b, cout, ep, out, u=u, skip=skip, act=act)
+    torch.cuda.synchronize()
+    ref = _torch_conv(full, W)
+    if ep < 2:
+        ref = (ref + b)[..., :out.shape[3]]
+    if ep == 0:
+        ref = torch.relu(ref)
+    if ep == 2:
+        ref = torch.where(act.float() > 0, ref, torch.zeros_like(ref))
+    tol = (1e-4 if ep == 1 else 2 ** -8) * ref.abs() + 1e-4 * ref.abs().max()
+    assert bool(((out.float() - ref).abs() <= tol).all())
