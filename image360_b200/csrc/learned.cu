@@ -59,7 +59,9 @@ enum
     EP_LOGITS = I360B_CONV_LOGITS,
     EP_MASK = I360B_CONV_MASK,
     EP_RAW = I360B_CONV_RAW,
-    EP_COMPOSITE = 4
+    EP_COMPOSITE = 4,
+    EP_RELU_POOL = 5,  // EP_RELU, and its 2x2 averages
+    EP_RAW_UP = 6      // the first 32 channels raw, 2x2 sums of the others masked
 };
 
 struct ConvArgs
@@ -71,9 +73,10 @@ struct ConvArgs
     const bf16* wt;     // [npad][9 * cin], k = tap * cin + c
     const float* bias;  // [npad]
     void* out;
-    const bf16* act;  // EP_MASK: [n][h][w][npad]
+    const bf16* act;  // EP_MASK: [n][h][w][npad]; EP_RAW_UP: [n][h/2][w/2][npad - 32]
     const i360b_blend_job* jobs;  // EP_COMPOSITE: one per image
     int* error;
+    bf16* half;          // EP_RELU_POOL: [n][h/2][w/2][npad]; EP_RAW_UP: [n][h/2][w/2][npad - 32]
     int rowSplit;  // the output map has the rows as (row % J, row / J): h is a multiple of J
 };
 
@@ -85,41 +88,48 @@ struct ConvArgs
 template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
 struct ConvShape
 {
-    // Roles by warp: [0, EW) epilogue, EW producer, EW + 1 MMA, then (for a
-    // concatenated input) 4 upsampling warps.
-    static constexpr int kProducerWarp = EW, kMmaWarp = EW + 1, kExpandWarp = EW + 2;
+    // Roles by warp: [0, EW) epilogue, EW producer, EW + 1 MMA.
+    static constexpr int kProducerWarp = EW, kMmaWarp = EW + 1, kThreads = 32 * (EW + 2);
     static constexpr int TH = 16 * J;
-    static constexpr int kP = TW + 2;
-    static constexpr int kHaloPx = (TW + 2) * (TH + 2);
     static constexpr int kCA = CIN == 96 ? 32 : CIN, kCB = CIN - kCA;  // channels of the two tiles
-    static constexpr uint32_t kBoxA = kHaloPx * kCA * 2, kBoxB = kHaloPx * kCB * 2;
-    static constexpr uint32_t kTileA = (kBoxA + 1023) / 1024 * 1024, kTileB = (kBoxB + 1023) / 1024 * 1024;
+    // With an upsampled second tile the two blocks of a row band take the even
+    // and the odd columns: a tap then reads 8 successive half-resolution
+    // pixels, and the first tile is kept as its odd and even columns.
+    static constexpr bool kParity = LD == LD_CONCAT;
+    static constexpr int kPA = kParity ? TW / 2 + 1 : TW + 2, kPB = kParity ? TW / 2 + 2 : TW + 2;  // row pitches, pixels
+    static constexpr uint32_t kBoxA = kPA * (TH + 2) * kCA * 2, kPlane = (kBoxA + 1023) / 1024 * 1024;
+    static constexpr uint32_t kBoxB = kPB * (kParity ? TH / 2 + 2 : TH + 2) * kCB * 2;
+    static constexpr uint32_t kTileA = (kParity ? 2 : 1) * kPlane, kTileB = (kBoxB + 1023) / 1024 * 1024;
+    static constexpr uint32_t kStage = kTileA + kTileB;
     static constexpr uint32_t kW = (9u * CIN * NPAD * 2 + 1023) / 1024 * 1024;
     static constexpr int kBX = TW / 8, kMB = kBX * J;  // block b: column b / J, row b % J
     static constexpr uint32_t kSlotCols = kMB * NPAD;
     static constexpr uint32_t kTmem = tc::tmem_cols(2 * kSlotCols);
-    static constexpr int kThreads = 32 * (EW + 2) + (LD == LD_CONCAT ? 128 : 0);
-    // Concatenated input: the half-resolution box behind a tile's halo,
-    // (TW/2+2) x (TH/2+2) pixels, per ring stage.
-    static constexpr int kPh = TW / 2 + 2;
-    static constexpr int kHalfPx = (TW / 2 + 2) * (TH / 2 + 2);
-    static constexpr uint32_t kHalfBox = LD == LD_CONCAT ? kHalfPx * kCB * 2 : 0;
-    static constexpr uint32_t kStage = kTileA + kTileB + (kHalfBox + 1023) / 1024 * 1024;
-    // Outputs leave by TMA from BUFS buffers per epilogue warp, each 32
-    // pixels as NPAD / 32 swizzled tiles of 32 channels.
+    // The epilogue's unit is kBatch blocks by kGroup channels: two rows (or the
+    // two parities of a row), which hide each other's latencies, where the
+    // accumulators then fit registers.
+    // With 8 warps the upper four take the upper half of the J rows.
+    static constexpr int kPer = kMB * 4 / EW;  // blocks of a warp, one column after the other
+    static constexpr int kGroup = EP == EP_RAW_UP ? 32 : NPAD, kBatch = EP == EP_COMPOSITE                                ? kPer
+                                  : kGroup <= 32 && (kParity || J * 4 / EW >= 2) ? 2
+                                                                                 : 1;
+    // Outputs leave by TMA from BUFS buffers per epilogue warp, each a unit as
+    // swizzled tiles of 32 pixels and channels.
     static constexpr bool kStored = EP != EP_LOGITS && EP != EP_COMPOSITE;
-    static constexpr uint32_t kOutBuf = kStored ? 32 * NPAD * 2 : 0, kOut = EW * BUFS * kOutBuf;
-    static constexpr uint32_t kBars = (3 * STAGES + 4) * 8 + 16;
+    static constexpr uint32_t kOutBuf = kStored ? kBatch * 32 * kGroup * 2 : 0, kOut = EW * BUFS * kOutBuf;
+    static constexpr uint32_t kBars = ((2 * STAGES + 4) * 8 + 16 + 15) / 16 * 16;
     static constexpr uint32_t kBias = NPAD * 4;
     static constexpr uint32_t kSmem = 1024 + kW + STAGES * kStage + kOut + kBars + kBias;
     static_assert(CIN == 16 || CIN == 32 || CIN == 64 || CIN == 96, "channels as swizzled rows");
     static_assert(NPAD == 16 || NPAD % 32 == 0, "MMA and output shape");
     static_assert((LD == LD_PLAIN) == (CIN != 96), "loader");
-    static_assert(TW % 8 == 0 && TW + 2 <= 256 && TH + 2 <= 256, "tile shape");
+    static_assert(TW % 8 == 0 && TW + 2 <= 256 && TH + 2 <= 256 && TH % 16 == 0, "tile shape");
     static_assert((J < 3 ? J : 3) * NPAD <= 256, "MMA columns");
     static_assert(2 * kSlotCols <= 512, "TMEM capacity");
     static_assert(kSmem <= 227u * 1024u, "shared memory");
-    static_assert(EW == 4 || (EW == 8 && kMB % 2 == 0), "epilogue warps split the M blocks in two");
+    static_assert(EW == 4 || (EW == 8 && J % 2 == 0), "epilogue warps split the rows in two");
+    static_assert(!kParity || (TW == 16 && J == 2 && EW == 8 && kStored), "parities of a row in one unit");
+    static_assert((EP != EP_RELU_POOL && EP != EP_RAW_UP) || kBatch == 2, "2x2 sums take two rows");
 };
 
 // The tiles that a persistent CTA takes, `stride` apart, as column, row and
@@ -165,6 +175,12 @@ __device__ __forceinline__ uint4 pack8_bf16(const float* v)
     return r;
 }
 
+// All ones in each half of a bf16 pair that is > 0.
+__device__ __forceinline__ uint32_t positive2(uint32_t v)
+{
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&v), __nv_bfloat162(__nv_bfloat16_raw{0}, __nv_bfloat16_raw{0}));
+}
+
 __device__ __forceinline__ void unpack8_bf16(uint4 q, float* v)
 {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
@@ -179,6 +195,22 @@ __device__ __forceinline__ void unpack8_bf16(uint4 q, float* v)
 }
 
 // Softmax-weighted composite of a pixel's covered layers (the network head).
+// The pixel's layer values (0 where a slot is absent), as (r | g << 16, b).
+__device__ __forceinline__ void load_slots_raw(const i360b_blend_job& J, int y, int x, uint2 (&v)[kSlots])
+{
+    const long long at = (long long)y * J.rowStride + (long long)x * J.pixStride;
+#pragma unroll
+    for (int i = 0; i < kSlots; ++i)
+    {
+        v[i] = make_uint2(0, 0);
+        if (J.slot[i])
+        {
+            const unsigned short* p = J.slot[i] + at;
+            v[i] = make_uint2(__ldg(p) | (uint32_t)__ldg(p + 1) << 16, __ldg(p + 2));
+        }
+    }
+}
+
 // The pixel's layer values (0 where a slot is absent).
 __device__ __forceinline__ void load_slots(const i360b_blend_job& J, int y, int x, float (*v)[3])
 {
@@ -259,14 +291,14 @@ __device__ __forceinline__ void composite_pixel(const i360b_blend_job& J, int y,
 // The A operand of set s and dx for column block bx is the halo tile from
 // pixel (8 bx + dx, s): 8 pixels of a row are 8 swizzled rows, the 16 rows J kP
 // pixels apart (SBO), a K step 32 bytes into the row.  The swizzle is a
-// function of the address, so a window may start at any pixel.
+// function of the address, so a window may start at any pixel.  An upsampled
+// half of the input is read where it lies, at half resolution: of the two
+// blocks of a row one takes the even, one the odd columns, so that tap's 8
+// pixels are successive there, and two rows' taps the same row.
 //
 // Roles:
 //   warp EW lane 0 TMA producer: one 4-D box (channels x (TW+2) x (16J+2)) per
 //                  tile into a STAGES-deep ring, zero fill outside the image;
-//   warps EW+2..   (concatenated input only) expand the TMA-loaded
-//                  half-resolution box into the nearest-upsampled channels
-//                  of the halo (shared memory to shared memory);
 //   warp EW+1 lane 0 MMA issuer, into one of two sets of TMEM accumulators;
 //                  commits free the ring stage and publish the accumulators;
 //   warps 0..EW-1  epilogue (EW = 4 or 8): TMEM lanes 32q..32q+31, q = w % 4
@@ -275,9 +307,12 @@ __device__ __forceinline__ void composite_pixel(const i360b_blend_job& J, int y,
 // Every wait is bounded; a timeout sets the error flag and the CTA winds
 // down after its loads have landed.
 //
-// 64 windows of 256 x 256, a 32 -> 32 layer: 93 us (537 MB, 81 us at the
-// measured copy rate); with one MMA per tap, 8-channel TMA boxes and outputs
-// stored a lane's 16 bytes at a time 176 us.
+// 64 windows of 256 x 256, a 32 -> 32 layer: 89 us (537 MB, 81 us at the
+// measured copy rate), and with the 2x2 averages 109; with one MMA per tap,
+// 8-channel TMA boxes and outputs stored a lane's 16 bytes at a time 176 us
+// and 55 for a kernel that averaged.  The 96-channel layer 0.22 ms (MMA issue
+// and operand fetch; 0.49 with the upsample expanded by warps), its backward
+// with the upsample's sums 0.22 (0.47 and 0.17 apart).
 // ---------------------------------------------------------------------------
 template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
 __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW, BUFS>::kThreads, 1)
@@ -294,11 +329,10 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
     unsigned char* outBufs = ring + STAGES * S::kStage;
     uint64_t* full = reinterpret_cast<uint64_t*>(outBufs + S::kOut);
     uint64_t* empty = full + STAGES;
-    uint64_t* halfFull = empty + STAGES;
-    uint64_t* accFull = halfFull + STAGES;
+    uint64_t* accFull = empty + STAGES;
     uint64_t* accEmpty = accFull + 2;
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(accEmpty + 2);
-    float* sBias = reinterpret_cast<float*>(tmemSlot + 4);
+    float* sBias = reinterpret_cast<float*>(outBufs + S::kOut + S::kBars);
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tilesX = (a.w + TW - 1) / TW, tilesY = (a.h + TH - 1) / TH;
@@ -311,9 +345,8 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
     {
         for (int s = 0; s < STAGES; ++s)
         {
-            tc::mbar_init(&full[s], LD == LD_CONCAT ? 1 + 128 : 1);
+            tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], 1);
-            tc::mbar_init(&halfFull[s], 1);
         }
         for (int k = 0; k < 2; ++k)
         {
@@ -366,57 +399,24 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
                 }
                 const int x0 = t.tx * TW, y0 = t.ty * TH;
                 unsigned char* st = ring + s * S::kStage;
-                if (LD == LD_CONCAT)
+                tc::mbar_arrive_expect_tx(&full[s], (S::kParity ? 2 : 1) * S::kBoxA + S::kBoxB);
+                if (S::kParity)
                 {
-                    // half-resolution rows/columns y0/2 - 1 .. (y0 + TH)/2 (x0, y0 even)
-                    tc::mbar_arrive_expect_tx(&halfFull[s], S::kHalfBox);
-                    tc::tma_load_4d(st + S::kTileA + S::kTileB, &mapB, 0, (x0 >> 1) - 1, (y0 >> 1) - 1, t.img,
-                                    &halfFull[s]);
+                    // columns x0 - 1, x0 + 1, ... and x0, x0 + 2, ... (x0 even)
+                    tc::tma_load_5d(st, &mapA, 0, 1, (x0 >> 1) - 1, y0 - 1, t.img, &full[s]);
+                    tc::tma_load_5d(st + S::kPlane, &mapA, 0, 0, x0 >> 1, y0 - 1, t.img, &full[s]);
+                    tc::tma_load_4d(st + S::kTileA, &mapB, 0, (x0 >> 1) - 1, (y0 >> 1) - 1, t.img, &full[s]);
                 }
-                tc::mbar_arrive_expect_tx(&full[s], S::kBoxA + (LD == LD_SPLIT ? S::kBoxB : 0u));
-                tc::tma_load_4d(st, &mapA, 0, x0 - 1, y0 - 1, t.img, &full[s]);
-                if (LD == LD_SPLIT) tc::tma_load_4d(st + S::kTileA, &mapB, S::kCA, x0 - 1, y0 - 1, t.img, &full[s]);
+                else
+                {
+                    tc::tma_load_4d(st, &mapA, 0, x0 - 1, y0 - 1, t.img, &full[s]);
+                    if (LD == LD_SPLIT) tc::tma_load_4d(st + S::kTileA, &mapB, S::kCA, x0 - 1, y0 - 1, t.img, &full[s]);
+                }
                 issued = i + 1;
             }
             // The last loads must land before the CTA may exit.
             for (int j = max(0, issued - STAGES); j < issued; ++j)
-            {
                 if (!tc::mbar_wait(&full[j % STAGES], (j / STAGES) & 1, kWaitSpins)) ok = false;
-                if (LD == LD_CONCAT && !tc::mbar_wait(&halfFull[j % STAGES], (j / STAGES) & 1, kWaitSpins)) ok = false;
-            }
-        }
-    }
-    else if (LD == LD_CONCAT && warp >= S::kExpandWarp)
-    {
-        // Nearest 2x upsample of the half-resolution box: its pixel (lx, ly)
-        // is halo columns 2 lx - 1, 2 lx and rows 2 ly - 1, 2 ly (tile origin
-        // even), those of them that there are.
-        const int c = tid & 7;
-        for (int i = 0; i < myTiles; ++i)
-        {
-            const int s = i % STAGES;
-            if (!tc::mbar_wait(&halfFull[s], (i / STAGES) & 1, kWaitSpins))
-            {
-                ok = false;
-                break;
-            }
-            unsigned char* up = ring + s * S::kStage + S::kTileA;
-            const unsigned char* half = up + S::kTileB;
-            for (int hp = (tid - 32 * S::kExpandWarp) >> 3; hp < S::kHalfPx; hp += 16)
-            {
-                const int ly = hp / S::kPh, lx = hp - ly * S::kPh;
-                const uint4 v = *reinterpret_cast<const uint4*>(half + hp * 128 + swizzled_chunk<64>(hp, c) * 16);
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-                {
-                    const int hy = 2 * ly - 1 + (k >> 1), hx = 2 * lx - 1 + (k & 1);
-                    if (hy < 0 || hy > TH + 1 || hx < 0 || hx > TW + 1) continue;
-                    const int px = hy * S::kP + hx;
-                    *reinterpret_cast<uint4*>(up + px * 128 + swizzled_chunk<64>(px, c) * 16) = v;
-                }
-            }
-            tc::fence_proxy_async();  // generic smem writes -> tensor core
-            tc::mbar_arrive(&full[s]);
         }
     }
     else if (warp == S::kMmaWarp)
@@ -442,8 +442,8 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
                 // Descriptors differ only in their start-address field: add
                 // the (compile-time) offset in 16-byte units to a base.
                 const uint32_t st = tc::smem_u32(ring + s * S::kStage);
-                const uint64_t aBase = tc::smem_desc_k<S::kCA>(st, J * S::kP * S::kCA * 2);
-                const uint64_t a2Base = tc::smem_desc_k<64>(st + S::kTileA, J * S::kP * 64 * 2);
+                const uint64_t aBase = tc::smem_desc_k<S::kCA>(st, J * S::kPA * S::kCA * 2);
+                const uint64_t a2Base = tc::smem_desc_k<64>(st + S::kTileA, (S::kParity ? J / 2 : J) * S::kPB * 64 * 2);
 #pragma unroll
                 for (int bx = 0; bx < S::kBX; ++bx)
 #pragma unroll
@@ -456,9 +456,12 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
                         for (int k0 = 0; k0 < 3 * CIN; k0 += 16)
                         {
                             const int dx = k0 / CIN, c = k0 % CIN;
-                            const uint32_t px = set * S::kP + bx * 8 + dx;
-                            const uint64_t aDesc = c < S::kCA ? aBase + ((px * S::kCA * 2 + c * 2) >> 4)
-                                                              : a2Base + ((px * 128 + (c - S::kCA) * 2) >> 4);
+                            // first pixel of the operand in either tile
+                            const int px = S::kParity ? set * S::kPA + (bx + dx) / 2 : set * S::kPA + bx * 8 + dx;
+                            const int px2 = S::kParity ? (set + 1) / 2 * S::kPB + (bx + dx + 1) / 2 : px;
+                            const uint32_t plane = S::kParity ? (bx + dx) % 2 * S::kPlane : 0;
+                            const uint64_t aDesc = c < S::kCA ? aBase + ((plane + px * S::kCA * 2 + c * 2) >> 4)
+                                                              : a2Base + ((px2 * 128 + (c - S::kCA) * 2) >> 4);
                             const uint32_t bRow = (k0 / 8) * 3 * NPAD + (2 - (set - j0)) * NPAD;
                             if (leader) tc::mma_bf16(d, aDesc, bBase + bRow, idesc, 1u);
                         }
@@ -474,130 +477,276 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
     }
     else if (warp < EW)
     {
-        // Warp w reads TMEM lane quadrant w % 4; with 8 epilogue warps the
-        // two warps of a quadrant take alternate M blocks.
-        const int quad = warp & 3, half = warp >> 2;
+        // Warp w reads TMEM lane quadrant w % 4, of rows `firstRow` on.
+        const int quad = warp & 3, firstRow = (warp >> 2) * (J * 4 / EW);
         unsigned char* buf = outBufs + warp * (BUFS * S::kOutBuf);
         int next = 0;  // output buffer
-        TileWalk t(tilesX, tilesY, blockIdx.x, gridDim.x);
-        for (int i = 0; i < myTiles && ok; ++i, t.next())
+        constexpr int kRows = S::kPer / S::kBX;  // rows of a column that this warp takes
+        constexpr int kBatch = S::kBatch, kGroup = S::kGroup;
+        // Pixel of this lane in the n-th block of tile t.
+        struct Px
         {
-            const int acc = i & 1, img = t.img;
-            const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + acc * S::kSlotCols;
-            for (int b = (EW == 8 ? half : 0); b < S::kMB; b += EW / 4)
+            int y, x;
+        };
+        auto pixel = [&](const TileWalk& t, int n) {
+            return Px{t.ty * TH + firstRow + n % kRows + J * (4 * quad + (lane >> 3)),
+                      t.tx * TW + (S::kParity ? n / kRows + 2 * (lane & 7) : n / kRows * 8 + (lane & 7))};
+        };
+        // Global inputs of a unit are loaded while the one before it is
+        // finished.
+        uint2 vv[EP == EP_COMPOSITE ? kBatch : 1][kSlots];
+        bool inJob[kBatch];
+        uint4 mk[EP == EP_MASK ? kBatch * kGroup / 8 : EP == EP_RAW_UP ? 2 : 1];
+        auto load_inputs = [&](const TileWalk& t, int n, int group) {
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k)
             {
-                const int yq = t.ty * TH + b % J + 4 * J * quad, xq = t.tx * TW + b / J * 8;
-                const int y = yq + J * (lane >> 3), x = xq + (lane & 7);
-                const bool valid = y < a.h && x < a.w;
-                const size_t pix = ((size_t)img * a.h + y) * a.w + x;
-                // Global inputs of the epilogue first, so their latency
-                // overlaps the wait and the TMEM loads.
-                float vv[4][3];
-                bool inJob = false;
+                const Px p = pixel(t, n + k);
+                const bool valid = p.y < a.h && p.x < a.w;
+                const size_t pix = ((size_t)t.img * a.h + p.y) * a.w + p.x;
                 if (EP == EP_COMPOSITE)
                 {
-                    const i360b_blend_job& J = a.jobs[img];
-                    inJob = valid && x < J.width && y < J.height;
-                    if (inJob) load_slots(J, y, x, vv);
+                    const i360b_blend_job& Jb = a.jobs[t.img];
+                    inJob[k] = valid && p.x < Jb.width && p.y < Jb.height;
+                    if (inJob[k]) load_slots_raw(Jb, p.y, p.x, vv[EP == EP_COMPOSITE ? k : 0]);
                 }
-                uint4 mk[EP == EP_MASK ? NPAD / 8 : 1];
                 if (EP == EP_MASK && valid)
                 {
                     const uint4* ap = reinterpret_cast<const uint4*>(a.act + pix * NPAD);
 #pragma unroll
-                    for (int q = 0; q < NPAD / 8; ++q) mk[q] = ap[q];
+                    for (int q = 0; q < kGroup / 8; ++q) mk[EP == EP_MASK ? k * (kGroup / 8) + q : 0] = ap[q];
                 }
-                if (b < EW / 4)
+                if (EP == EP_RAW_UP && k == 0 && group > 0 && valid)
                 {
-                    const bool done = tc::mbar_wait(&accFull[acc], (i >> 1) & 1, kWaitSpins);
-                    if (!__all_sync(0xffffffffu, done))
-                    {
-                        ok = false;
-                        break;
-                    }
-                    tc::fence_after_sync();
-                }
-                constexpr int kCols = (EP == EP_LOGITS || EP == EP_COMPOSITE) ? 16 : NPAD;
-                uint32_t r[kCols];
-#pragma unroll
-                for (int cb = 0; cb < kCols / 16; ++cb) tc::tmem_ld16_nowait(base + b * NPAD + cb * 16, r + cb * 16);
-                tc::tmem_wait_ld();
-#pragma unroll
-                for (int cb = 0; cb < kCols / 16; ++cb) tc::tmem_reg_fence16(r + cb * 16);
-#pragma unroll
-                for (int cb = 0; cb < NPAD / 16; ++cb) tc::tmem_zero16(base + b * NPAD + cb * 16);
-                tc::tmem_wait_st();
-                if (b + EW / 4 >= S::kMB)
-                {
-                    tc::fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) tc::mbar_arrive(&accEmpty[acc]);
-                }
-                if (EP == EP_LOGITS || EP == EP_COMPOSITE)
-                {
-                    float l[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) l[j] = __uint_as_float(r[j]) + sBias[j];
-                    if (EP == EP_LOGITS)
-                    {
-                        if (valid) reinterpret_cast<float4*>(a.out)[pix] = make_float4(l[0], l[1], l[2], l[3]);
-                    }
-                    else if (inJob)
-                    {
-                        const i360b_blend_job& J = a.jobs[img];
-                        float o[3], wts[4];
-                        bool cov[4];
-                        int nCov;
-                        blend_slots(l, vv, o, wts, cov, nCov);
-                        unsigned short* q = J.out + (long long)y * J.outRowStride + (long long)x * 3;
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-                            q[c] = (unsigned short)__float2uint_rn(fminf(fmaxf(o[c], 0.0f), 65535.0f));
-                    }
-                }
-                else
-                {
-                    unsigned char* ob = buf + next * S::kOutBuf;
-                    if (BUFS > 1) next = next + 1 == BUFS ? 0 : next + 1;
-                    if (lane == 0) tc::bulk_wait_read<BUFS - 1>();
-                    __syncwarp();
-#pragma unroll
-                    for (int c8 = 0; c8 < NPAD / 8; ++c8)
-                    {
-                        float v[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[c8 * 8 + j]);
-                        if (EP == EP_RELU)
-                        {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j] + sBias[c8 * 8 + j], 0.0f);
-                        }
-                        if (EP == EP_MASK)
-                        {
-                            float m[8];
-                            unpack8_bf16(mk[c8], m);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) v[j] = m[j] > 0.0f ? v[j] : 0.0f;
-                        }
-                        *reinterpret_cast<uint4*>(ob + (c8 >> 2) * 2048 + lane * 64 +
-                                                  swizzled_chunk<32>(lane, c8 & 3) * 16) = pack8_bf16(v);
-                    }
-                    tc::fence_proxy_async();  // generic smem writes -> TMA
-                    __syncwarp();
-                    if (lane == 0 && yq < a.h && xq < a.w)
-                    {
-                        for (int u = 0; u < NPAD / 32; ++u)
-                        {
-                            if (a.rowSplit)  // 4 rows J apart as rows / J of the map
-                                tc::tma_store_5d(&mapOut, ob + u * 2048, u * 32, xq, yq % J, yq / J, img);
-                            else
-                                for (int k = 0; k < 4 && yq + J * k < a.h; ++k)
-                                    tc::tma_store_5d(&mapOut, ob + u * 2048 + k * 512, u * 32, xq, yq + J * k, 0, img);
-                        }
-                    }
-                    if (lane == 0) tc::bulk_commit();
+                    const size_t hp = ((size_t)t.img * (a.h >> 1) + (p.y >> 1)) * (a.w >> 1) + (p.x >> 1);
+                    const uint4* ap = reinterpret_cast<const uint4*>(a.act + hp * (NPAD - 32) + (group - 1) * 32 +
+                                                                     (lane & 1) * 16);
+                    mk[0] = ap[0];
+                    mk[EP == EP_RAW_UP ? 1 : 0] = ap[1];
                 }
             }
+        };
+        TileWalk t(tilesX, tilesY, blockIdx.x, gridDim.x);
+        load_inputs(t, 0, 0);
+        for (int i = 0; i < myTiles && ok; ++i)
+        {
+            const int acc = i & 1, img = t.img;
+            const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + acc * S::kSlotCols;
+            TileWalk following = t;
+            following.next();
+            const bool done = tc::mbar_wait(&accFull[acc], (i >> 1) & 1, kWaitSpins);
+            if (!__all_sync(0xffffffffu, done))
+            {
+                ok = false;
+                break;
+            }
+            tc::fence_after_sync();
+#pragma unroll 1
+            for (int n = 0; n < S::kPer; n += kBatch)
+#pragma unroll 1
+                for (int group = 0; group < NPAD / kGroup; ++group)
+                {
+                    auto at = [&](int k) {  // accumulators of the unit's k-th block
+                        return base + ((n + k) / kRows * J + firstRow + (n + k) % kRows) * NPAD + group * kGroup;
+                    };
+                    uint32_t r[kBatch][kGroup];
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+                        for (int cb = 0; cb < kGroup / 16; ++cb)
+                            tc::tmem_ld16_nowait(at(k) + cb * 16, r[k] + cb * 16);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+                        for (int cb = 0; cb < kGroup / 16; ++cb) tc::tmem_reg_fence16(r[k] + cb * 16);
+#pragma unroll
+                    for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+                        for (int cb = 0; cb < kGroup / 16; ++cb) tc::tmem_zero16(at(k) + cb * 16);
+                    const bool lastGroup = group + 1 == NPAD / kGroup, last = lastGroup && n + kBatch >= S::kPer;
+                    if (last)
+                    {
+                        tc::tmem_wait_st();
+                        tc::fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) tc::mbar_arrive(&accEmpty[acc]);
+                    }
+                    const Px p = pixel(t, n);
+                    const bool valid = p.y < a.h && p.x < a.w;  // of the batch's first row
+                    uint4 pk[kBatch][S::kStored ? kGroup / 8 : 1];
+                    if (S::kStored)
+                    {
+#pragma unroll
+                        for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+                            for (int c8 = 0; c8 < kGroup / 8; ++c8)
+                            {
+                                uint32_t w[4];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j)
+                                {
+                                    const uint32_t* v = r[k] + c8 * 8 + 2 * j;
+                                    f32x2 f = pack2(__uint_as_float(v[0]), __uint_as_float(v[1]));
+                                    if (EP == EP_RELU || EP == EP_RELU_POOL)
+                                        f = add2(f, *reinterpret_cast<const f32x2*>(sBias + c8 * 8 + 2 * j));
+                                    __nv_bfloat162 h = __floats2bfloat162_rn(lo2(f), hi2(f));
+                                    if (EP == EP_RELU || EP == EP_RELU_POOL)
+                                        h = __hmax2(h, __nv_bfloat162(__nv_bfloat16_raw{0}, __nv_bfloat16_raw{0}));
+                                    w[j] = *reinterpret_cast<uint32_t*>(&h);
+                                }
+                                if (EP == EP_MASK)
+                                {
+                                    const uint4 m = mk[EP == EP_MASK ? k * (kGroup / 8) + c8 : 0];
+                                    w[0] &= positive2(m.x);
+                                    w[1] &= positive2(m.y);
+                                    w[2] &= positive2(m.z);
+                                    w[3] &= positive2(m.w);
+                                }
+                                pk[k][S::kStored ? c8 : 0] = make_uint4(w[0], w[1], w[2], w[3]);
+                            }
+                    }
+                    if (EP == EP_LOGITS || EP == EP_COMPOSITE)
+                    {
+#pragma unroll
+                        for (int k = 0; k < kBatch; ++k)
+                        {
+                            const Px q = pixel(t, n + k);
+                            float l[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) l[j] = __uint_as_float(r[k][j]) + sBias[j];
+                            if (EP == EP_LOGITS)
+                            {
+                                if (q.y < a.h && q.x < a.w)
+                                    reinterpret_cast<float4*>(a.out)[((size_t)img * a.h + q.y) * a.w + q.x] =
+                                        make_float4(l[0], l[1], l[2], l[3]);
+                            }
+                            else if (inJob[k])
+                            {
+                                const i360b_blend_job& Jb = a.jobs[img];
+                                float o[3], wts[4];
+                                bool cov[4];
+                                int nCov;
+                                float v[kSlots][3];
+#pragma unroll
+                                for (int m = 0; m < kSlots; ++m)
+                                {
+                                    const uint2 raw = vv[EP == EP_COMPOSITE ? k : 0][m];
+                                    v[m][0] = raw.x & 0xffff;
+                                    v[m][1] = raw.x >> 16;
+                                    v[m][2] = raw.y;
+                                }
+                                blend_slots(l, v, o, wts, cov, nCov);
+                                unsigned short* op = Jb.out + (long long)q.y * Jb.outRowStride + (long long)q.x * 3;
+#pragma unroll
+                                for (int c = 0; c < 3; ++c)
+                                    op[c] = (unsigned short)__float2uint_rn(fminf(fmaxf(o[c], 0.0f), 65535.0f));
+                            }
+                        }
+                    }
+                    if (EP == EP_RELU_POOL || (EP == EP_RAW_UP && group > 0))
+                    {
+                        // 2x2 sums of the rounded outputs, left to right, upper
+                        // row first; of 32 channels the left lane of a pair
+                        // takes the first half, the right lane the second.
+                        const bool right = lane & 1;
+                        float sum[16];
+#pragma unroll
+                        for (int c = 0; c < 16; ++c) sum[c] = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+                            for (int q = 0; q < 2; ++q)
+                            {
+                                const uint4 lo = pk[k][S::kStored ? q : 0], hi = pk[k][S::kStored ? 2 + q : 0];
+                                uint4 own = right ? hi : lo, other = right ? lo : hi;
+                                other.x = __shfl_xor_sync(0xffffffffu, other.x, 1);
+                                other.y = __shfl_xor_sync(0xffffffffu, other.y, 1);
+                                other.z = __shfl_xor_sync(0xffffffffu, other.z, 1);
+                                other.w = __shfl_xor_sync(0xffffffffu, other.w, 1);
+                                float first[8], second[8];
+                                unpack8_bf16(right ? other : own, first);
+                                unpack8_bf16(right ? own : other, second);
+#pragma unroll
+                                for (int c = 0; c < 8; ++c) sum[q * 8 + c] = (sum[q * 8 + c] + first[c]) + second[c];
+                            }
+                        uint4 o[2];
+                        if (EP == EP_RELU_POOL)
+                        {
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) sum[c] *= 0.25f;
+                        }
+                        o[0] = pack8_bf16(sum);
+                        o[1] = pack8_bf16(sum + 8);
+                        if (EP == EP_RAW_UP)
+                        {
+#pragma unroll
+                            for (int q = 0; q < 2; ++q)
+                            {
+                                const uint4 m = mk[EP == EP_RAW_UP ? q : 0];
+                                o[q].x &= positive2(m.x);
+                                o[q].y &= positive2(m.y);
+                                o[q].z &= positive2(m.z);
+                                o[q].w &= positive2(m.w);
+                            }
+                        }
+                        if (valid)
+                        {
+                            constexpr int kC = EP == EP_RAW_UP ? NPAD - 32 : NPAD;
+                            const size_t hp = ((size_t)img * (a.h >> 1) + (p.y >> 1)) * (a.w >> 1) + (p.x >> 1);
+                            uint4* op = reinterpret_cast<uint4*>(a.half + hp * kC +
+                                                                 (EP == EP_RAW_UP ? (group - 1) * 32 : 0) + right * 16);
+                            op[0] = o[0];
+                            op[1] = o[1];
+                        }
+                    }
+                    // inputs of the unit after this one
+                    if (!lastGroup) load_inputs(t, n, group + 1);
+                    else if (!last) load_inputs(t, n + kBatch, 0);
+                    else if (i + 1 < myTiles) load_inputs(following, 0, 0);
+                    if (S::kStored && (EP != EP_RAW_UP || group == 0))
+                    {
+                        unsigned char* ob = buf + next * S::kOutBuf;
+                        if (BUFS > 1) next = next + 1 == BUFS ? 0 : next + 1;
+                        if (lane == 0) tc::bulk_wait_read<BUFS - 1>();
+                        __syncwarp();
+#pragma unroll
+                        for (int k = 0; k < kBatch; ++k)
+#pragma unroll
+                            for (int c8 = 0; c8 < kGroup / 8; ++c8)
+                            {
+                                // parities: one tile of 16 x 4 pixels
+                                const int px = S::kParity ? 2 * lane + k : lane;
+                                *reinterpret_cast<uint4*>(
+                                    ob + (S::kParity ? 0 : (k * (kGroup / 32) + (c8 >> 2)) * 2048) + px * 64 +
+                                    swizzled_chunk<32>(px, c8 & 3) * 16) = pk[k][S::kStored ? c8 : 0];
+                            }
+                        tc::fence_proxy_async();  // generic smem writes -> TMA
+                        __syncwarp();
+                        if (lane == 0)
+                        {
+#pragma unroll
+                            for (int k = 0; k < (S::kParity ? 1 : kBatch); ++k)
+                            {
+                                const Px q = pixel(t, n + k);  // lane 0: the block's first
+                                if (q.y >= a.h || q.x >= a.w) continue;
+#pragma unroll
+                                for (int u = 0; u < kGroup / 32; ++u)
+                                {
+                                    const unsigned char* tile = ob + (k * (kGroup / 32) + u) * 2048;
+                                    constexpr int kRow = S::kParity ? 1024 : 512;  // bytes of a pixel row
+                                    if (a.rowSplit)  // 4 rows J apart as rows / J of the map
+                                        tc::tma_store_5d(&mapOut, tile, u * 32, q.x, q.y % J, q.y / J, img);
+                                    else
+                                        for (int v = 0; v < 4 && q.y + J * v < a.h; ++v)
+                                            tc::tma_store_5d(&mapOut, tile + v * kRow, u * 32, q.x, q.y + J * v, 0, img);
+                                }
+                            }
+                            tc::bulk_commit();
+                        }
+                    }
+                }
+            t = following;
         }
         if (S::kStored && lane == 0) tc::bulk_wait_all();
     }
@@ -618,13 +767,17 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
 // summed over image rows y and pixels q (K, 16 per MMA), accumulators in TMEM
 // over the CTA's whole share.  Both operands are MN-major: a pixel's CX = 16
 // or 32 input channels, or its output channels, are rows of 32, 64 or 128
-// bytes in the swizzle of that width, as TMA writes them.  X lies in shared
-// memory as [row][pixel][CX], so the operand of output row y is 128 / CX
+// bytes in the swizzle of that width, as TMA writes them.  An MMA's 16 pixels
+// are those of one column parity, kept as planes.  X lies in shared memory as
+// [parity][row][pixel][CX], so the operand of output row y is 128 / CX
 // successive rows from y on: the three dy, then rows whose accumulators are
-// not looked at.  G is loaded three times, a pixel further each time, so its
-// dx are a copy apart.  One MMA per tap would have N = cout = 16..64 columns,
-// and fetching the 4 KB of A takes several times such a multiplication; here
-// N = 3 cout.  A layer of more than 32 input channels is a job per 32.
+// not looked at.  G is kept as the four planes of columns + 2, + 1, + 0 and
+// - 1: the dx of even pixels are the last three, of odd ones the first three,
+// a plane apart.  Of an upsampled input both parities are the same
+// half-resolution pixels, and rows y - 1 .. y + 4 three boxes of two.
+// One MMA per tap would have N = cout = 16..64 columns, and fetching the 4 KB
+// of A takes several times such a multiplication; here N = 3 cout.  A layer of
+// more than 32 input channels is a job per 32.
 //
 // How far a sum is cut into slices (a CTA's share of the tiles) is not free:
 // the tensor core truncates as it adds to an accumulator, so a sum comes out
@@ -634,26 +787,23 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
 // results have always come from: gradients of a batch of 64 windows agree
 // with those to 8e-7, and one slice per SM is 1.3e-4 away.
 //
-// That leaves two thirds of the SMs idle, so one launch takes the jobs of
-// several layers, longest first, a CTA per (job, slice).  CTA `b` of a job
+// That leaves two thirds of the SMs idle, so one launch takes the jobs of all
+// layers, longest first, a CTA per (job, slice).  CTA `b` of a job
 // handles tiles b, b + slices, ... of 32 x 4 pixels.
 //   warp 4     lane 0 loads a tile's X and G by TMA (zero fill outside the
 //              image) into a ring of stages;
-//   warp 5     lane 0 issues the MMAs; a commit frees the stage;
-//   warps 0-3  sum G for the bias gradient (where asked for); with an
-//              upsampled input expand the half-resolution box into the
-//              stage's X; at the end write the accumulators as this slice's
-//              partial sums.
+//   warp 5     issues the MMAs; a commit frees the stage;
+//   warps 0-3  sum G for the bias gradient (where asked for); at the end write
+//              the accumulators as this slice's partial sums.
 // Every wait is bounded; a timeout sets the error flag and the CTA winds down
 // after its loads have landed.
 //
-// What bounds it is shared memory: a 32 -> 32 tile takes 718 cycles, of which
-// TMA writes 37 KB (288 cycles at 128 B, and 580 at the 64 B/clk that L2
-// gives an SM) and the MMAs read 56 KB (448).
-// 64 windows of 256 x 256, all eight layers with their bias gradients: 0.95 ms
-// (2.5 ms with a launch per layer), and 0.06 for the reduction; one 128-row
-// chunk of (tap, cin) per CTA gathered by cp.async, N = cout and a kernel of
-// its own for the bias took 10.9 + 0.29 ms.
+// 64 windows of 256 x 256, all eight layers with their bias gradients: 0.70
+// ms for 3.3 GB of X and G (0.50 at the measured copy rate); the longest jobs,
+// the 96-channel layer's 63 CTAs, set the end.  With a launch per layer 1.9 ms;
+// with the pixels of an MMA successive (three full copies of G and an upsample
+// by the warps) 0.77; one 128-row chunk of (tap, cin) per CTA gathered by
+// cp.async, N = cout and a kernel of its own for the bias 10.9 + 0.29 ms.
 // ---------------------------------------------------------------------------
 enum WgradKind
 {
@@ -675,7 +825,7 @@ struct WgradJob
     float* partial;  // per slice [3 cin][3 COUT], then [COUT] sums of g
 };
 
-constexpr int kWgJobs = 9;  // a 96-, two 64- and two 32-channel layers
+constexpr int kWgJobs = 12;  // the network's eight layers
 
 struct WgradBatch
 {
@@ -689,17 +839,14 @@ constexpr int kWgRows = 4, kWgTW = 32;  // pixels of a tile
 template <int CX, int COUT, bool UP>
 struct WgradShape
 {
-    static constexpr int kAtoms = 128 / CX;     // rows of X in an MMA
-    static constexpr int kXRows = kWgRows + 2;  // rows loaded
-    static constexpr uint32_t kXRow = kWgTW * CX * 2, kGRow = kWgTW * COUT * 2;
-    static constexpr uint32_t kX = ((kWgRows - 1 + kAtoms) * kXRow + 1023) / 1024 * 1024;
-    static constexpr uint32_t kGCopy = kWgRows * kGRow;
-    static constexpr uint32_t kG = (3 * kGCopy + 1023) / 1024 * 1024;
-    // Upsampled input: the half-resolution box behind a tile's X rows.
-    static constexpr int kHalfRows = kWgRows / 2 + 2;
-    static constexpr uint32_t kHalfRow = kWgTW / 2 * CX * 2, kHalf = UP ? kHalfRows * kHalfRow : 0;
-    static constexpr uint32_t kStage = kX + kG + (kHalf + 1023) / 1024 * 1024;
-    static constexpr int kStages = 214 * 1024 / kStage > 6 ? 6 : 214 * 1024 / kStage;
+    static constexpr int kXRows = kWgRows + 2, kHalfW = kWgTW / 2;
+    static constexpr uint32_t kXRow = kHalfW * CX * 2, kGRow = kHalfW * COUT * 2;
+    static constexpr uint32_t kXPlane = kXRows * kXRow, kGPlane = kWgRows * kGRow;
+    static constexpr uint32_t kX = ((UP ? 1 : 2) * kXPlane + 1023) / 1024 * 1024, kG = 4 * kGPlane;
+    static constexpr uint32_t kStage = kX + kG;
+    // The last row's operand is 128 / CX rows from row 3 of the last plane on.
+    static_assert(kXPlane + (kWgRows - 1 + 128 / CX) * kXRow <= kStage, "operands within the stage");
+    static constexpr int kStages = 214 * 1024 / kStage > 8 ? 8 : 214 * 1024 / kStage;
     static constexpr uint32_t kSmem = 1024 + kStages * kStage + 256;
     static constexpr int kN = 3 * COUT;
     static constexpr uint32_t kTmem = tc::tmem_cols(kN);
@@ -718,24 +865,21 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
         reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::kStages * S::kStage);
     uint64_t* empty = full + S::kStages;
-    uint64_t* halfFull = empty + S::kStages;
-    uint64_t* done = halfFull + S::kStages;
+    uint64_t* done = empty + S::kStages;
     uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(done + 1);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int tilesX = a.w / kWgTW, tilesY = (a.h + kWgRows - 1) / kWgRows;
     const long long nTiles = (long long)a.n * tilesX * tilesY;  // >= a.slices
     const int myTiles = (int)((nTiles - 1 - slice) / a.slices) + 1;
     const bool bias = !UP && a.bias;
-    const bool helpers = UP || bias;  // warps 0-3 take part in every tile
 
     if (warp == 0) tc::tmem_alloc(tmemSlot, S::kTmem);
     if (tid == 0)
     {
         for (int s = 0; s < S::kStages; ++s)
         {
-            tc::mbar_init(&full[s], UP ? 1 + 128 : 1);
+            tc::mbar_init(&full[s], 1);
             tc::mbar_init(&empty[s], bias ? 1 + 4 : 1);
-            tc::mbar_init(&halfFull[s], 1);
         }
         tc::mbar_init(done, 1);
         tc::fence_mbar_init();
@@ -765,15 +909,17 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
                 }
                 const int x0 = t.tx * kWgTW, y0 = t.ty * kWgRows;
                 unsigned char* st = smem + s * S::kStage;
+                const int xh = x0 >> 1;
+                tc::mbar_arrive_expect_tx(&full[s], 2 * S::kXPlane / (UP ? 2 : 1) + S::kG);
                 if (UP)
-                {
-                    tc::mbar_arrive_expect_tx(&halfFull[s], S::kHalf);
-                    tc::tma_load_4d(st + S::kX + S::kG, &a.mapX, a.xc0, x0 >> 1, (y0 >> 1) - 1, t.img, &halfFull[s]);
-                }
-                tc::mbar_arrive_expect_tx(&full[s], (UP ? 0u : S::kXRows * S::kXRow) + 3 * S::kGCopy);
-                if (!UP) tc::tma_load_4d(st, &a.mapX, a.xc0, x0, y0 - 1, t.img, &full[s]);
-                for (int dx = 0; dx < 3; ++dx)
-                    tc::tma_load_4d(st + S::kX + dx * S::kGCopy, &a.mapG, 0, x0 - (dx - 1), y0, t.img, &full[s]);
+                    for (int k = 0; k < 3; ++k)
+                        tc::tma_load_4d(st + 2 * k * S::kXRow, &a.mapX, a.xc0, xh, (y0 >> 1) - 1 + k, t.img, &full[s]);
+                else
+                    for (int k = 0; k < 2; ++k)
+                        tc::tma_load_5d(st + k * S::kXPlane, &a.mapX, a.xc0, k, xh, y0 - 1, t.img, &full[s]);
+                for (int k = 0; k < 4; ++k)  // columns x0 + 2 - k, x0 + 4 - k, ...
+                    tc::tma_load_5d(st + S::kX + k * S::kGPlane, &a.mapG, 0, k & 1, xh + (2 - k - (k & 1)) / 2, y0,
+                                    t.img, &full[s]);
                 t.next();
                 issued = i + 1;
             }
@@ -781,7 +927,6 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
             for (int j = max(0, issued - S::kStages); j < issued; ++j)
             {
                 const int s = j % S::kStages;
-                if (UP && !tc::mbar_wait(&halfFull[s], (j / S::kStages) & 1, kWaitSpins)) ok = false;
                 if (!tc::mbar_wait(&full[s], (j / S::kStages) & 1, kWaitSpins)) ok = false;
             }
         }
@@ -805,75 +950,49 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
                 tc::fence_after_sync();
                 const uint32_t xa = tc::smem_u32(smem + s * S::kStage);
                 const uint64_t aBase = tc::smem_desc_mn<CX>(xa, S::kXRow),
-                               bBase = tc::smem_desc_mn<COUT>(xa + S::kX, S::kGCopy);
+                               bBase = tc::smem_desc_mn<COUT>(xa + S::kX, S::kGPlane);
 #pragma unroll
                 for (int r = 0; r < kWgRows; ++r)
 #pragma unroll
-                    for (int k = 0; k < kWgTW / 16; ++k)
+                    for (int p = 0; p < 2; ++p)  // column parity
                         if (leader)
-                            tc::mma_bf16(tmemU, aBase + ((r * S::kXRow + k * 16 * CX * 2) >> 4),
-                                         bBase + ((r * S::kGRow + k * 16 * COUT * 2) >> 4), idesc,
-                                         (i > 0 || r > 0 || k > 0) ? 1u : 0u);
+                            tc::mma_bf16(tmemU, aBase + (((UP ? 0 : p) * S::kXPlane + r * S::kXRow) >> 4),
+                                         bBase + (((1 - p) * S::kGPlane + r * S::kGRow) >> 4), idesc,
+                                         (i > 0 || r > 0 || p > 0) ? 1u : 0u);
                 if (leader) tc::mma_commit(&empty[s]);
                 __syncwarp();
             }
             if (leader) tc::mma_commit(done);
         }
     }
-    else if (helpers)
+    else if (bias)
     {
-        // Bias: this thread's chunk position and pixels of the copy dx = 1,
-        // rows of 32 pixels with COUT / 8 chunks; the pixels it sees keep the
-        // chunk's place in the swizzle, so its channels are fixed.
+        // This thread's chunk position and pixels of the planes + 1 and + 0,
+        // 128 rows of COUT / 8 chunks; the pixels it sees keep the chunk's
+        // place in the swizzle, so its channels are fixed.
         constexpr int kO8 = COUT / 8;
         const int pos = tid % kO8, px0 = tid / kO8;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int i = 0; i < myTiles; ++i)
         {
             const int s = i % S::kStages;
-            unsigned char* st = smem + s * S::kStage;
-            if (UP)
+            if (!tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins))
             {
-                if (!tc::mbar_wait(&halfFull[s], (i / S::kStages) & 1, kWaitSpins))
-                {
-                    ok = false;
-                    break;
-                }
-                // X row j is image row y0 - 1 + j, y0 a multiple of 4: row
-                // (j + 1) / 2 of the box
-                const unsigned char* half = st + S::kX + S::kG;
-#pragma unroll
-                for (int k = 0; k < S::kXRows * kWgTW * 4 / 128; ++k)
-                {
-                    const int c = tid & 3, px = tid >> 2, j = k;
-                    const int hr = (j + 1) >> 1, hp = px >> 1;
-                    *reinterpret_cast<uint4*>(st + j * S::kXRow + px * 64 + swizzled_chunk<32>(px, c) * 16) =
-                        *reinterpret_cast<const uint4*>(half + hr * S::kHalfRow + hp * 64 +
-                                                        swizzled_chunk<32>(hp, c) * 16);
-                }
-                tc::fence_proxy_async();  // generic smem writes -> tensor core
-                tc::mbar_arrive(&full[s]);
+                ok = false;
+                break;
             }
-            else
+            const unsigned char* g = smem + s * S::kStage + S::kX + S::kGPlane;
+#pragma unroll
+            for (int k = 0; k < kWgRows * kWgTW * kO8 / 128; ++k)
             {
-                if (!tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins))
-                {
-                    ok = false;
-                    break;
-                }
-                const unsigned char* g = st + S::kX + S::kGCopy;
+                const int p = px0 + k * (128 / kO8);
+                float v[8];
+                unpack8_bf16(*reinterpret_cast<const uint4*>(g + p * COUT * 2 + pos * 16), v);
 #pragma unroll
-                for (int k = 0; k < kWgRows * kWgTW * kO8 / 128; ++k)
-                {
-                    const int p = px0 + k * (128 / kO8);  // pixel of the tile, rows of 32
-                    float v[8];
-                    unpack8_bf16(*reinterpret_cast<const uint4*>(g + p * COUT * 2 + pos * 16), v);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] += v[j];
-                }
-                __syncwarp();
-                if (lane == 0) tc::mbar_arrive(&empty[s]);
+                for (int j = 0; j < 8; ++j) acc[j] += v[j];
             }
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&empty[s]);
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) sBias[tid][j] = acc[j];
@@ -1058,68 +1177,6 @@ __global__ void k_pack_input(const i360b_blend_job* __restrict__ jobs, int n, in
         uint4* o = reinterpret_cast<uint4*>(x0 + idx * 16);
         o[0] = pack8_bf16(ch);
         o[1] = pack8_bf16(ch + 8);
-    }
-}
-
-// 2x2 average pool of [n][h][w][C] (C = 8 * c8n) into [n][h/2][w/2][C].
-__global__ void k_pool2(const bf16* __restrict__ in, int n, int h, int w, int c8n, bf16* __restrict__ out)
-{
-    const int hh = h >> 1, wh = w >> 1;
-    const long long total = (long long)n * hh * wh * c8n;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x)
-    {
-        const int c8 = (int)(idx % c8n);
-        long long r = idx / c8n;
-        const int xh = (int)(r % wh);
-        r /= wh;
-        const int yh = (int)(r % hh), img = (int)(r / hh);
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx)
-            {
-                float v[8];
-                const size_t p = ((size_t)img * h + 2 * yh + dy) * w + 2 * xh + dx;
-                unpack8_bf16(reinterpret_cast<const uint4*>(in + p * c8n * 8)[c8], v);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] += v[j];
-            }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] *= 0.25f;
-        reinterpret_cast<uint4*>(out + idx * 8)[0] = pack8_bf16(acc);
-    }
-}
-
-// Gradient of the upsampled half of the concatenation: g5 = (sum over the 2x2
-// children of du[..., skip: skip+C]) * (a5 > 0), at half resolution.
-__global__ void k_upsample_grad(const bf16* __restrict__ du, int duC, int skip, const bf16* __restrict__ act, int n,
-                                int h, int w, int c8n, bf16* __restrict__ g)
-{
-    const int hh = h >> 1, wh = w >> 1;
-    const long long total = (long long)n * hh * wh * c8n;
-    for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
-         idx += (long long)gridDim.x * blockDim.x)
-    {
-        const int c8 = (int)(idx % c8n);
-        long long r = idx / c8n;
-        const int xh = (int)(r % wh);
-        r /= wh;
-        const int yh = (int)(r % hh), img = (int)(r / hh);
-        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int dy = 0; dy < 2; ++dy)
-            for (int dx = 0; dx < 2; ++dx)
-            {
-                float v[8];
-                const size_t p = ((size_t)img * h + 2 * yh + dy) * w + 2 * xh + dx;
-                unpack8_bf16(*reinterpret_cast<const uint4*>(du + p * duC + skip + c8 * 8), v);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] += v[j];
-            }
-        float m[8];
-        unpack8_bf16(reinterpret_cast<const uint4*>(act)[idx], m);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] = m[j] > 0.0f ? acc[j] : 0.0f;
-        reinterpret_cast<uint4*>(g)[idx] = pack8_bf16(acc);
     }
 }
 
@@ -1329,23 +1386,32 @@ int make_tile_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, 
     return make_map<4>(m, base, {c, w, h, n}, {c, row, h * row}, {boxC, boxW, boxH, 1}, swizzle);
 }
 
-// A convolution's output, 32 channels of 8 x 4 pixels at a time: rows
-// split > 0 apart as (C, W, split, H / split, N), or (split = 0) a row at a
-// time as (C, W, H, 1, N).
-int make_output_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int split)
-{
-    const long long row = (long long)w * c;
-    return split > 0 ? make_map<5>(m, base, {c, w, split, h / split, n}, {c, row, split * row, h * row}, {32, 8, 1, 4, 1},
-                                   CU_TENSOR_MAP_SWIZZLE_64B)
-                     : make_map<5>(m, base, {c, w, h, 1, n}, {c, row, h * row, h * row}, {32, 8, 1, 1, 1},
-                                   CU_TENSOR_MAP_SWIZZLE_64B);
-}
-
 constexpr CUtensorMapSwizzle swizzle_of(int channels)
 {
     return channels == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
            : channels == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
                             : CU_TENSOR_MAP_SWIZZLE_32B;
+}
+
+// The columns by parity, as (C, W % 2, W / 2, H, N) with boxes of boxC x 1 x
+// boxW x boxH x 1 (w even).
+int make_parity_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int boxC, int boxW, int boxH)
+{
+    const long long row = (long long)w * c;
+    return make_map<5>(m, base, {c, 2, w / 2, h, n}, {c, 2 * c, row, h * row}, {boxC, 1, boxW, boxH, 1},
+                       swizzle_of(boxC));
+}
+
+// A convolution's output, 32 channels of boxW x 4 pixels at a time: rows
+// split > 0 apart as (C, W, split, H / split, N), or (split = 0) a row at a
+// time as (C, W, H, 1, N).
+int make_output_map(CUtensorMap* m, const bf16* base, int c, int n, int h, int w, int split, int boxW)
+{
+    const long long row = (long long)w * c;
+    return split > 0 ? make_map<5>(m, base, {c, w, split, h / split, n}, {c, row, split * row, h * row}, {32, boxW, 1, 4, 1},
+                                   CU_TENSOR_MAP_SWIZZLE_64B)
+                     : make_map<5>(m, base, {c, w, h, 1, n}, {c, row, h * row, h * row}, {32, boxW, 1, 1, 1},
+                                   CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
@@ -1363,17 +1429,23 @@ int run_conv(ConvArgs a, cudaStream_t s)
     const long long tiles = (long long)a.n * ((a.h + TH - 1) / TH) * ((a.w + TW - 1) / TW);
     if (tiles == 0) return I360B_SUCCESS;
     CUtensorMap ma, mb, mo;
-    I360B_TRY(make_tile_map(&ma, a.x, LD == LD_CONCAT ? a.cs : CIN, a.n, a.h, a.w, S::kCA, TW + 2, TH + 2,
-                            swizzle_of(S::kCA)));
-    mb = mo = ma;
     if (LD == LD_CONCAT)
-        I360B_TRY(make_tile_map(&mb, a.u, S::kCB, a.n, a.h / 2, a.w / 2, S::kCB, TW / 2 + 2, TH / 2 + 2,
-                                swizzle_of(S::kCB)));
-    if (LD == LD_SPLIT)
-        I360B_TRY(make_tile_map(&mb, a.x, CIN, a.n, a.h, a.w, S::kCB, TW + 2, TH + 2, swizzle_of(S::kCB)));
+    {
+        I360B_TRY(make_parity_map(&ma, a.x, S::kCA, a.n, a.h, a.w, S::kCA, S::kPA, TH + 2));
+        I360B_TRY(make_tile_map(&mb, a.u, S::kCB, a.n, a.h / 2, a.w / 2, S::kCB, S::kPB, TH / 2 + 2, swizzle_of(S::kCB)));
+    }
+    else
+    {
+        I360B_TRY(make_tile_map(&ma, a.x, CIN, a.n, a.h, a.w, S::kCA, S::kPA, TH + 2, swizzle_of(S::kCA)));
+        mb = ma;
+        if (LD == LD_SPLIT)
+            I360B_TRY(make_tile_map(&mb, a.x, CIN, a.n, a.h, a.w, S::kCB, S::kPB, TH + 2, swizzle_of(S::kCB)));
+    }
+    mo = ma;
     a.rowSplit = a.h % J == 0;
     if (S::kStored)
-        I360B_TRY(make_output_map(&mo, static_cast<const bf16*>(a.out), NPAD, a.n, a.h, a.w, a.rowSplit ? J : 0));
+        I360B_TRY(make_output_map(&mo, static_cast<const bf16*>(a.out), EP == EP_RAW_UP ? 32 : NPAD, a.n, a.h, a.w,
+                                  a.rowSplit ? J : 0, S::kParity ? 16 : 8));
     k<<<grid_for(tiles, 1), S::kThreads, S::kSmem, s>>>(ma, mb, mo, a);
     return check_launch("conv3x3 kernel");
 }
@@ -1386,19 +1458,21 @@ int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cuda
     if (cin == CI && npad == NP && loader == LD && ep == EP_) \
         return run_conv<CI, NP, TW, J, ST, LD, EP_, EW, BUFS>(a, s);
     I360B_CONV(16, 32, 16, 4, 3, LD_PLAIN, EP_RELU, 8, 2)
-    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_RELU, 8, 2)
+    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_RELU, 8, 1)
+    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_RELU_POOL, 8, 1)
     I360B_CONV(32, 64, 8, 4, 3, LD_PLAIN, EP_RELU, 8, 1)
     I360B_CONV(64, 64, 8, 2, 2, LD_PLAIN, EP_RELU, 8, 1)
-    I360B_CONV(96, 32, 8, 2, 2, LD_CONCAT, EP_RELU, 4, 1)
-    I360B_CONV(96, 32, 8, 2, 2, LD_SPLIT, EP_RELU, 4, 1)
+    I360B_CONV(96, 32, 16, 2, 2, LD_CONCAT, EP_RELU, 8, 1)
+    I360B_CONV(96, 32, 8, 2, 2, LD_SPLIT, EP_RELU, 8, 1)
     I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_LOGITS, 8, 1)
     I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_COMPOSITE, 8, 1)
     // backward data
     I360B_CONV(16, 32, 16, 4, 3, LD_PLAIN, EP_MASK, 8, 2)
-    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_MASK, 8, 2)
+    I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_MASK, 8, 1)
     I360B_CONV(32, 96, 8, 2, 3, LD_PLAIN, EP_RAW, 8, 1)
+    I360B_CONV(32, 96, 8, 2, 3, LD_PLAIN, EP_RAW_UP, 4, 2)
     I360B_CONV(64, 64, 8, 2, 2, LD_PLAIN, EP_MASK, 8, 1)
-    I360B_CONV(64, 32, 8, 4, 2, LD_PLAIN, EP_RAW, 8, 1)
+    I360B_CONV(64, 32, 8, 4, 2, LD_PLAIN, EP_RAW, 4, 1)
 #undef I360B_CONV
     return fail(I360B_NOT_SUPPORTED, "conv3x3: no kernel for cin=%d cout=%d loader=%d epilogue=%d", cin, npad, loader,
                 ep);
@@ -1425,10 +1499,10 @@ struct WgradLayer
     size_t partials() const { return (size_t)slices() * (9 * cin * cout + cout); }
 };
 
-// Partial sums of the network's layers 3..7 in one batch, the most at a time.
+// Partial sums of the network's layers in one batch, the most at a time.
 size_t wgrad_scratch_bytes()
 {
-    constexpr int shapes[][2] = {{32, 32}, {32, 16}, {64, 64}, {64, 64}, {96, 32}};
+    constexpr int shapes[][2] = {{16, 32}, {32, 32}, {32, 64}, {64, 64}, {64, 64}, {96, 32}, {32, 32}, {32, 16}};
     size_t floats = 0;
     for (const auto& c : shapes) floats += (size_t)(9 * c[0] * c[1] + c[1]) * wgrad_slices(c[0]);
     return floats * sizeof(float);
@@ -1481,12 +1555,12 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
             j.bias = L.db && c == 0;
             j.partial = part;
             if (up)
-                I360B_TRY(make_tile_map(&j.mapX, L.u, L.cin - L.cs, L.n, L.h / 2, L.w / 2, cx, kWgTW / 2,
-                                        kWgRows / 2 + 2, swizzle_of(cx)));
-            else
-                I360B_TRY(make_tile_map(&j.mapX, L.x, L.cs > 0 ? L.cs : L.cin, L.n, L.h, L.w, cx, kWgTW, kWgRows + 2,
+                I360B_TRY(make_tile_map(&j.mapX, L.u, L.cin - L.cs, L.n, L.h / 2, L.w / 2, cx, kWgTW / 2, 2,
                                         swizzle_of(cx)));
-            I360B_TRY(make_tile_map(&j.mapG, L.g, L.cout, L.n, L.h, L.w, L.cout, kWgTW, kWgRows, swizzle_of(L.cout)));
+            else
+                I360B_TRY(make_parity_map(&j.mapX, L.x, L.cs > 0 ? L.cs : L.cin, L.n, L.h, L.w, cx, kWgTW / 2,
+                                          kWgRows + 2));
+            I360B_TRY(make_parity_map(&j.mapG, L.g, L.cout, L.n, L.h, L.w, L.cout, kWgTW / 2, kWgRows));
             blocks += j.slices;
         }
         r.layer[r.layers++] = {part, L.slices(), L.cin, L.cout, L.coutReal, reduceBlocks, L.dw, L.db};
@@ -1549,7 +1623,8 @@ struct BlendNet
     bf16 *x0 = nullptr, *a1 = nullptr, *a2 = nullptr, *p2 = nullptr, *a3 = nullptr, *a4 = nullptr, *a5 = nullptr,
          *a6 = nullptr, *a7 = nullptr;
     float* logits = nullptr;
-    bf16 *g8 = nullptr, *gA = nullptr, *gB = nullptr, *du = nullptr, *gh1 = nullptr, *gh2 = nullptr, *dp = nullptr;
+    bf16 *g8 = nullptr, *gA = nullptr, *gB = nullptr, *du = nullptr, *gh1 = nullptr, *gh2 = nullptr, *dp = nullptr,
+         *gC = nullptr, *gh3 = nullptr;
     void* wgScratch = nullptr;
     size_t wgBytes = 0;
     double* dLoss = nullptr;
@@ -1689,8 +1764,8 @@ struct BlendNet
         // bf16 element counts of every buffer, then the fp32 logits.
         const size_t counts[] = {pix * 16,       pix * 32,       pix * 32,       half * 32,      half * 64,
                                  half * 64,      half * 64,      pix * 32,       pix * 32,       tr * pix * 16,
-                                 tr * pix * 32,  tr * pix * 32,  tr * pix * 96,  tr * half * 64, tr * half * 64,
-                                 tr * half * 32};
+                                 tr * pix * 32,  tr * pix * 32,  tr * pix * 32,  tr * half * 64, tr * half * 64,
+                                 tr * half * 32, tr * pix * 32,  tr * half * 64};
         size_t total = 0;
         for (size_t c : counts) total += (c * sizeof(bf16) + 255) / 256 * 256;
         total += pix * 4 * sizeof(float);
@@ -1702,7 +1777,7 @@ struct BlendNet
             return fail(I360B_OUT_OF_MEMORY, "blend network: %zu bytes of activations for %d windows of %dx%d", total,
                         n, w, h);
         }
-        bf16** slots[] = {&x0, &a1, &a2, &p2, &a3, &a4, &a5, &a6, &a7, &g8, &gA, &gB, &du, &gh1, &gh2, &dp};
+        bf16** slots[] = {&x0, &a1, &a2, &p2, &a3, &a4, &a5, &a6, &a7, &g8, &gA, &gB, &du, &gh1, &gh2, &dp, &gC, &gh3};
         size_t o = 0;
         for (size_t i = 0; i < sizeof(counts) / sizeof(counts[0]); ++i)
         {
@@ -1773,11 +1848,11 @@ struct BlendNet
         mark(1);
         I360B_TRY(dispatch_conv(16, 32, LD_PLAIN, EP_RELU, conv(x0, n, w, h, 0, a1, jobs), s));
         mark(2);
-        I360B_TRY(dispatch_conv(32, 32, LD_PLAIN, EP_RELU, conv(a1, n, w, h, 1, a2, jobs), s));
+        ConvArgs c2 = conv(a1, n, w, h, 1, a2, jobs);
+        c2.half = p2;
+        I360B_TRY(dispatch_conv(32, 32, LD_PLAIN, EP_RELU_POOL, c2, s));
         mark(3);
-        k_pool2<<<elementwise_grid((long long)n * hw * hh * 4), 256, 0, s>>>(a2, n, h, w, 4, p2);
-        I360B_TRY(check_launch("pool kernel"));
-        mark(4);
+        mark(4);  // the pool, a part of conv2
         I360B_TRY(dispatch_conv(32, 64, LD_PLAIN, EP_RELU, conv(p2, n, hw, hh, 2, a3, jobs), s));
         mark(5);
         I360B_TRY(dispatch_conv(64, 64, LD_PLAIN, EP_RELU, conv(a3, n, hw, hh, 3, a4, jobs), s));
@@ -1798,7 +1873,8 @@ struct BlendNet
     }
 
     // Backward data through layer l (flipped, transposed weights).
-    int dgrad(int l, const bf16* g, int n, int w, int h, const bf16* actMask, void* out, int ep, cudaStream_t s)
+    int dgrad(int l, const bf16* g, int n, int w, int h, const bf16* actMask, void* out, int ep, cudaStream_t s,
+              bf16* half = nullptr)
     {
         ConvArgs a{};
         a.x = g;
@@ -1808,6 +1884,7 @@ struct BlendNet
         a.wt = dgW[l];
         a.out = out;
         a.act = actMask;
+        a.half = half;
         a.error = dError;
         return dispatch_conv(pad16(kNet[l].cout), kNet[l].cin, LD_PLAIN, ep, a, s);
     }
@@ -1817,9 +1894,9 @@ struct BlendNet
         return {x, u, cs, g, n, h, w, kNet[l].cin, pad16(kNet[l].cout), kNet[l].cout, grads + wOff[l], grads + bOff[l]};
     }
 
-    // Loss, then every parameter gradient into `grads`.  The weight gradients
-    // are taken in two batches, each once the next step would overwrite an
-    // output gradient that they read.
+    // Loss, then every parameter gradient into `grads`: the output gradients
+    // of all layers first, g1 .. g8 from the last down, then the layers' weight
+    // gradients in one batch.
     int backward(int n, int w, int h, cudaStream_t s)
     {
         const int hw = w / 2, hh = h / 2;
@@ -1833,27 +1910,23 @@ struct BlendNet
         // layer 7 (32 -> 32): input a6
         I360B_TRY(dgrad(6, gA, n, w, h, a6, gB, EP_MASK, s));  // gB = g6
         // layer 6 (96 -> 32): input concat(a2, up(a5))
-        I360B_TRY(dgrad(5, gB, n, w, h, nullptr, du, EP_RAW, s));
-        k_upsample_grad<<<elementwise_grid((long long)n * hw * hh * 8), 256, 0, s>>>(du, 96, 32, a5, n, h, w, 8, gh1);
-        I360B_TRY(check_launch("upsample gradient kernel"));  // gh1 = g5
+        I360B_TRY(dgrad(5, gB, n, w, h, a5, du, EP_RAW_UP, s, gh1));  // du of the skip, gh1 = g5
         // layer 5 (64 -> 64): input a4
         I360B_TRY(dgrad(4, gh1, n, hw, hh, a4, gh2, EP_MASK, s));  // gh2 = g4
-        const WgradLayer late[] = {wgrad(5, a2, gB, n, w, h, a5, 32), wgrad(6, a6, gA, n, w, h),
-                                   wgrad(7, a7, g8, n, w, h), wgrad(4, a4, gh1, n, hw, hh),
-                                   wgrad(3, a3, gh2, n, hw, hh)};
-        I360B_TRY(run_wgrad(late, 5, dError, wgScratch, wgBytes, s));
         // layer 4 (64 -> 64): input a3
-        I360B_TRY(dgrad(3, gh2, n, hw, hh, a3, gh1, EP_MASK, s));  // gh1 = g3
+        I360B_TRY(dgrad(3, gh2, n, hw, hh, a3, gh3, EP_MASK, s));  // gh3 = g3
         // layer 3 (32 -> 64): input p2
-        I360B_TRY(dgrad(2, gh1, n, hw, hh, nullptr, dp, EP_RAW, s));  // dp = d(pool)
-        k_skip_grad<<<elementwise_grid(pix * 4), 256, 0, s>>>(du, 96, dp, a2, n, h, w, 4, gA);
-        I360B_TRY(check_launch("skip gradient kernel"));  // gA = g2
-        // layer 2 (32 -> 32): input a1
-        I360B_TRY(dgrad(1, gA, n, w, h, a1, gB, EP_MASK, s));  // gB = g1
-        // layer 1 (16 -> 32): input x0
-        const WgradLayer early[] = {wgrad(1, a1, gA, n, w, h), wgrad(0, x0, gB, n, w, h),
-                                    wgrad(2, p2, gh1, n, hw, hh)};
-        return run_wgrad(early, 3, dError, wgScratch, wgBytes, s);
+        I360B_TRY(dgrad(2, gh3, n, hw, hh, nullptr, dp, EP_RAW, s));  // dp = d(pool)
+        k_skip_grad<<<elementwise_grid(pix * 4), 256, 0, s>>>(du, 32, dp, a2, n, h, w, 4, gC);
+        I360B_TRY(check_launch("skip gradient kernel"));  // gC = g2
+        // layer 2 (32 -> 32): input a1; layer 1 (16 -> 32): input x0
+        I360B_TRY(dgrad(1, gC, n, w, h, a1, du, EP_MASK, s));  // du = g1
+        const WgradLayer layers[] = {
+            wgrad(5, a2, gB, n, w, h, a5, 32), wgrad(1, a1, gC, n, w, h),     wgrad(6, a6, gA, n, w, h),
+            wgrad(7, a7, g8, n, w, h),         wgrad(0, x0, du, n, w, h),     wgrad(4, a4, gh1, n, hw, hh),
+            wgrad(3, a3, gh2, n, hw, hh),      wgrad(2, p2, gh3, n, hw, hh),
+        };
+        return run_wgrad(layers, kNumLayers, dError, wgScratch, wgBytes, s);
     }
 
     int adam(float lr, cudaStream_t s)

@@ -258,6 +258,16 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0,
 }
 
 // TMEM allocation size: a power of two of at least 32 columns.
+__device__ __forceinline__ void tma_load_5d(void* dst, const void* tmap, int c0, int c1, int c2, int c3, int c4,
+                                            uint64_t* mbar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
+        "%6}], [%7];" ::"r"(smem_u32(dst)),
+        "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(mbar))
+        : "memory");
+}
+
 // One tiled TMA store of a box (bulk group of the issuing thread; parts
 // outside the tensor are left out).
 __device__ __forceinline__ void tma_store_5d(const void* tmap, const void* src, int c0, int c1, int c2, int c3, int c4)
