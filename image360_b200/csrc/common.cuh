@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstddef>
+#include <cstring>
 
 #include "../../include/image360_b200.h"
 
@@ -83,6 +84,19 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
+__device__ __forceinline__ f32x2 fma2_rz(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// The pair (v, v), on the host.
+inline f32x2 pair_of(float v)
+{
+    uint32_t b;
+    std::memcpy(&b, &v, sizeof(b));
+    return f32x2{(unsigned long long)b << 32 | b};
+}
 // a * b, rounded once per half; `nz` is neg_zero2().
 __device__ __forceinline__ f32x2 mulx2(f32x2 a, f32x2 b, f32x2 nz) { return fma2(a, b, nz); }
 static __constant__ float2 g_negZero2 = {-0.0f, -0.0f};
@@ -97,6 +111,13 @@ __device__ __forceinline__ unsigned short clamp_trunc_u16(float v)
     v = v > 0.0f ? v : 0.0f;  // NaN -> 0
     v = v < 65535.0f ? v : 65535.0f;
     return static_cast<unsigned short>(f2u_floor(v));  // truncation = floor on [0, 65535]
+}
+
+// v within [0, 65535] (NaN -> 0).
+__device__ __forceinline__ float clamp_u16f(float v)
+{
+    v = v > 0.0f ? v : 0.0f;
+    return v < 65535.0f ? v : 65535.0f;
 }
 
 // (float)clamp_trunc_u16(v) without the round trip through an integer: on
