@@ -1008,8 +1008,8 @@ __global__ void __launch_bounds__(256) k_owner(BlendArgs a, const Unit* __restri
     const int W = T.w;
     const long long full = (long long)W * T.h;
     const float kInf = (float)(W + T.h);
-    const int row0 = u.by * a.bandRows;
-    const int rows = min(a.bandRows, T.h - row0);
+    const int row0 = u.by * u.rows;
+    const int rows = min(u.rows, T.h - row0);
     // Four pixels per thread: 16-byte reads of d and one 4-byte owner store
     // when rows are 4-pixel aligned.  A contributor with no covered pixel, or
     // whose covered box misses the pixels, has d == 0 there and cannot win
@@ -2472,8 +2472,8 @@ __global__ void __launch_bounds__(256, 3) k_blend_level(BlendArgs a, const Unit*
     const int K = T.numItems;
     const int lw = T.lw[level], lh = T.lh[level];
     const bool top = level == T.bands - 1;
-    const int row0 = u.by * a.bandRows;
-    const int rows = min(a.bandRows, lh - row0);
+    const int row0 = u.by * u.rows;
+    const int rows = min(u.rows, lh - row0);
     const int qpr = (lw + 3) >> 2;
     const int nq = rows * qpr;
     for (int qi = threadIdx.x; qi < nq; qi += blockDim.x)
@@ -2500,8 +2500,8 @@ __global__ void __launch_bounds__(256) k_collapse(BlendArgs a, const Unit* __res
     const int lw = T.lw[level], lh = T.lh[level];
     const int uw = T.lw[level + 1], uh = T.lh[level + 1];
     const float* r = T.blend + T.loff[level + 1] * 3;
-    const long long base = (long long)u.by * a.bandRows * lw;
-    const long long n = min((long long)a.bandRows * lw, (long long)lw * lh - base);
+    const long long base = (long long)u.by * u.rows * lw;
+    const long long n = min((long long)u.rows * lw, (long long)lw * lh - base);
     for (long long q = threadIdx.x; q < n; q += blockDim.x)
     {
         const long long pl = base + q;
@@ -2686,8 +2686,8 @@ __global__ void __launch_bounds__(256) k_final0(BlendArgs a, const Unit* __restr
     const int W = T.w, H = T.h;
     const int uw = T.lw[1], uh = T.lh[1];
     const float* rc = T.blend + T.loff[1] * 3;
-    const int row0 = u.by * a.bandRows;
-    const int rows = min(a.bandRows, H - row0);
+    const int row0 = u.by * u.rows;
+    const int rows = min(u.rows, H - row0);
     const int qpr = (W + 3) >> 2;  // quads per row
     const int nq = rows * qpr;
     const signed char* owner = T.owner;

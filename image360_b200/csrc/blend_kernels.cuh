@@ -9,6 +9,7 @@ namespace i360b
 {
 constexpr int kMaxBands = 8;
 constexpr int kBandRows = 16;  // default rows per CTA of the per-pixel band kernels
+constexpr int kBandThreads = 256;  // of their CTAs
 constexpr int kSeamRadius = 24;                 // SeamBlend.cpp:319
 constexpr int kSeamBand = 2 * kSeamRadius + 1;  // candidates per line
 constexpr float kSeamSmooth = 2.0f;             // SeamBlend.cpp:309
@@ -64,7 +65,7 @@ struct Unit
     int id;
     int bx;
     int by;
-    int level;
+    int rows;  // of a band
 };
 
 // Default limit of every bounded device wait, in SM cycles (~1 s at B200

@@ -123,6 +123,7 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
                 cudaStream_t stream, bool oneShot)
 {
     render = renderPath;
+    oneChunk = oneShot && !extArena;  // (a caller's arena holds the default work lists)
     nTiles = (int)specs.size();
     if (numBands < 1) return fail(I360B_INVALID_PARAM, "numBands must be >= 1.");
     bandsReq = std::min(numBands, kMaxBands);
@@ -374,7 +375,18 @@ void Plan::make_units(int rows, std::vector<Unit>& units)
     units.clear();
     // Band units: `rows` full-width rows each (per-pixel kernels).
     auto addBands = [&](int id, int h) {
-        for (int by = 0; by < (h + rows - 1) / rows; ++by) units.push_back(Unit{id, 0, by, 0});
+        for (int by = 0; by < (h + rows - 1) / rows; ++by) units.push_back(Unit{id, 0, by, rows});
+    };
+    // Bands of a tile's output and levels.  One chunk alone has too few bands
+    // of 16 rows to fill the GPU (a 2048 x 2048 chunk 128, its level 1 64):
+    // there bands of fewer rows, down to a quad of pixels per thread.
+    // 2048 x 2048 x 4: level blends 223 -> 61 us, output 153 -> 71, collapse
+    // 70 -> 20, ownership 59 -> 17.
+    auto addTileBands = [&](int id, int w, int h) {
+        const int quads = (w + 3) / 4;
+        const int fill = std::max(h / (4 * sm_count()), (kBandThreads + quads - 1) / quads);
+        const int r = oneChunk ? std::max(1, std::min(rows, fill)) : rows;
+        for (int by = 0; by < (h + r - 1) / r; ++by) units.push_back(Unit{id, 0, by, r});
     };
     // Block units of the pyramid down kernels: bw x 16 outputs each (64 wide
     // for the level-0 step, whose lanes make two columns each; 32 above).
@@ -406,11 +418,11 @@ void Plan::make_units(int rows, std::vector<Unit>& units)
         endList(s);
         s = beginList();  // 1: ownership
         for (int t = 0; t < nTiles; ++t)
-            if (inT(t)) addBands(t, tiles[t].h);
+            if (inT(t)) addTileBands(t, tiles[t].w, tiles[t].h);
         endList(s);
         s = beginList();  // 2: level 0 output
         for (int t = 0; t < nTiles; ++t)
-            if (inT(t)) addBands(t, tiles[t].h);
+            if (inT(t)) addTileBands(t, tiles[t].w, tiles[t].h);
         endList(s);
         for (int l = 0; l < kMaxBands - 1; ++l)  // 3 + l: down from level l
         {
@@ -427,7 +439,7 @@ void Plan::make_units(int rows, std::vector<Unit>& units)
             s = beginList();
             if (l >= 1)
                 for (int t = 0; t < nTiles; ++t)
-                    if (inT(t) && tiles[t].bands > l) addBands(t, tiles[t].lh[l]);
+                    if (inT(t) && tiles[t].bands > l) addTileBands(t, tiles[t].lw[l], tiles[t].lh[l]);
             endList(s);
         }
         for (int l = 0; l < kMaxBands; ++l)  // 3 + 2*kMaxBands - 1 + l: collapse at level l (1 <= l <= bands-2)
@@ -435,7 +447,7 @@ void Plan::make_units(int rows, std::vector<Unit>& units)
             s = beginList();
             if (l >= 1)
                 for (int t = 0; t < nTiles; ++t)
-                    if (inT(t) && tiles[t].bands > l + 1) addBands(t, tiles[t].lh[l]);
+                    if (inT(t) && tiles[t].bands > l + 1) addTileBands(t, tiles[t].lw[l], tiles[t].lh[l]);
             endList(s);
         }
         s = beginList();  // kListBase2: level-2 blocks of every contributor of a tile with >= 3 bands

@@ -59,6 +59,7 @@ struct Plan
     // Tuning: rows per band unit of the per-pixel kernels (8, 16, 32 or 64)
     // and ring slots of the chamfer transform (0 = as many as fit).
     int bandRows = kBandRows, dtSlots = 0;
+    bool oneChunk = false;  // built for one blend of one chunk
     // Pyramid levels computed on chip (level-fusion depth): 2 = levels 0 and
     // 1 fused (k_base2 + k_fine, only levels >= 2 in memory), 1 = level 1
     // materialised by k_down0s and read by k_fine (the level-1 blend,
