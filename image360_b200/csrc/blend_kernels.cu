@@ -27,6 +27,9 @@ __device__ __forceinline__ bool cov_bit(const uint32_t* cov, int covWords, int x
 // the inclusive bounding box of covered pixels (SeamBlend.cpp:263-280).
 // A CTA owns a band of a.bandRows full-width rows of one contributor; each warp
 // walks its rows 32 pixels at a time, so one ballot is one coverage word.
+// Rows of whole 16-byte words are taken 256 pixels at a time, 8 to a lane: a
+// warp then has 1.5 KB in flight instead of 192 bytes, which is what bounds
+// it (four 2048 x 2048 images 26 us, 80 us 32 pixels at a time).
 // ---------------------------------------------------------------------------
 struct BoxAcc
 {
@@ -90,10 +93,45 @@ __global__ void __launch_bounds__(256) k_coverage(BlendArgs a, const Unit* __res
     const int W = T.w, H = T.h, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     BoxAcc box;
     const int rowsPerWarp = a.bandRows >> 3;
+    const bool wide = (W & 7) == 0 && (reinterpret_cast<uintptr_t>(it.img) & 15) == 0;
     for (int r = 0; r < rowsPerWarp; ++r)
     {
         const int y = u.by * a.bandRows + warp * rowsPerWarp + r;
         if (y >= H) break;
+        if (wide)
+        {
+            const uint4* row = reinterpret_cast<const uint4*>(it.img + (size_t)y * W * 3);
+#pragma unroll 2
+            for (int x0 = 0; x0 < W; x0 += 256)
+            {
+                const int x = x0 + 8 * lane;
+                uint32_t bits = 0;
+                if (x < W)
+                {
+                    const uint4 q0 = row[x / 8 * 3], q1 = row[x / 8 * 3 + 1], q2 = row[x / 8 * 3 + 2];
+                    const uint32_t v[12] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)  // two pixels in three words
+                    {
+                        if ((v[3 * k] | (v[3 * k + 1] & 0xffffu)) != 0) bits |= 1u << (2 * k);
+                        if (((v[3 * k + 1] >> 16) | v[3 * k + 2]) != 0) bits |= 2u << (2 * k);
+                    }
+                }
+                uint32_t word = bits << (8 * (lane & 3));
+                word |= __shfl_xor_sync(kFull, word, 1);
+                word |= __shfl_xor_sync(kFull, word, 2);
+                if ((lane & 3) == 0 && x < W) it.cov[(size_t)y * T.covWords + (x >> 5)] = word;
+                if (bits)
+                {
+                    box.n += __popc(bits);
+                    box.x0 = min(box.x0, x + __ffs(bits) - 1);
+                    box.x1 = max(box.x1, x + 31 - __clz(bits));
+                    box.y0 = min(box.y0, y);
+                    box.y1 = max(box.y1, y);
+                }
+            }
+            continue;
+        }
         for (int x0 = 0; x0 < W; x0 += 32)
         {
             const int x = x0 + lane;

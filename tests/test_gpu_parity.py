@@ -346,3 +346,23 @@ def test_demosaic_strip_edges(backend, oracle_c, filters, w, h):
         assert backend.launch_demosaic(d_in.data_ptr(), w, h, black, cm, rc, filters, d_out.data_ptr()) == 0
         torch.cuda.synchronize()
         assert np.array_equal(d_out.cpu().numpy().view(np.uint16), oracle_c.demosaic(cfa, black, cm, rc, filters))
+
+
+@pytest.mark.parametrize("w", [8, 16, 40, 248, 256, 264, 520])
+def test_blend_coverage_words(backend, oracle_c, w):
+    """Rows of whole 16-byte words, whose coverage is read 8 pixels a lane:
+    covered by any one channel, sparse, and with empty columns at either end."""
+    rng = np.random.default_rng(w)
+    h = 21
+    bufs = []
+    for k in range(3):
+        b = np.zeros((h, w, 3), np.uint16)
+        one = rng.integers(0, 3, (h, w))
+        on = rng.random((h, w)) < (0.03, 0.5, 0.95)[k]
+        on[:, :k] = False
+        on[:, w - 2 * k:] = False
+        np.put_along_axis(b, one[..., None], np.where(on, rng.integers(1, 65536, (h, w)), 0)[..., None].astype(np.uint16), 2)
+        bufs.append(b)
+    out = np.zeros((h, w, 3), np.uint16)
+    assert backend.blend_chunk_contributors(bufs, w, h, out, 4) == ComputeResult.SUCCESS, backend.get_last_error()
+    assert np.array_equal(out, oracle_c.blend(bufs, 4))
