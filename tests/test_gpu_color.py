@@ -148,3 +148,31 @@ def test_invalid_arguments(backend):
     assert backend.launch_color_correct([], [], [], 0) == bad
     assert backend.launch_lab_stats([t.data_ptr()] * 65, [4] * 65, [4] * 65, t.data_ptr()) == bad
     assert backend.launch_reinhard([t.data_ptr()], [4], [0], t.data_ptr(), t.data_ptr()) == bad
+
+
+@pytest.mark.parametrize("spread", [1.0, 0.05, 40.0])
+def test_transfer_pairs_equal_single_pixels(backend, spread):
+    """Whole chunks (two pixels at a time, the encode by table) give the bits
+    that an image at an address that is not 16-byte aligned gives one pixel at
+    a time: noise, ramps of every code, blacks and whites, and statistics that
+    push values out of range on either side."""
+    import torch
+    rng = np.random.default_rng(int(spread * 100))
+    h, w = 97, 2048
+    img = rng.integers(0, 65536, (h, w, 3)).astype(np.uint16)
+    img[:32] = np.arange(65536, dtype=np.uint16).reshape(32, w, 1)
+    img[32:64, :, 1:] = (np.arange(65536).reshape(32, w, 1) // 37).astype(np.uint16)
+    img[64:70] = 0
+    img[70:74] = 65535
+    src = torch.tensor([48.0, 3.0, -7.5, 21.0, 9.0, 14.0], dtype=torch.float64, device="cuda")
+    ref = torch.tensor([55.0, -6.0, 11.0, 21.0 * spread, 9.0 * spread, 14.0 * spread], dtype=torch.float64,
+                       device="cuda")
+    got = []
+    for shift in (0, 1):
+        buf = torch.zeros(h * w * 3 + 8, dtype=torch.int16, device="cuda")
+        view = buf[shift:shift + h * w * 3]
+        view.copy_(torch.from_numpy(img.reshape(-1).view(np.int16)))
+        assert backend.launch_reinhard([buf.data_ptr() + 2 * shift], [w], [h], src.data_ptr(), ref.data_ptr()) == 0
+        torch.cuda.synchronize()
+        got.append(view.cpu().numpy())
+    assert np.array_equal(got[0], got[1])
