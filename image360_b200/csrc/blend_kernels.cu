@@ -1981,6 +1981,15 @@ __device__ __forceinline__ UpCoef up_coef_s(float sx, float sy, int sw, int sh, 
     return c;
 }
 
+// The same on taps held as pairs (row 0, row 1): ix = (1 - wx) and wx twice,
+// w = (1 - wy, wy).  Every half is rounded as up_mix rounds it; 5 instructions
+// instead of 9.
+__device__ __forceinline__ float up_mix2(f32x2 left, f32x2 right, f32x2 ix, f32x2 wx, f32x2 w, f32x2 nz)
+{
+    const f32x2 m = mulx2(w, add2(mulx2(ix, left, nz), mulx2(wx, right, nz)), nz);
+    return fadd(lo2(m), hi2(m));
+}
+__device__ __forceinline__ f32x2 row_weights(float wy) { return pack2(fsub(1.0f, wy), wy); }
 __device__ __forceinline__ float up_mix(float v00, float v10, float v01, float v11, float wx, float wy)
 {
     float ix = fsub(1.0f, wx), iy = fsub(1.0f, wy);
@@ -2529,30 +2538,97 @@ __global__ void __launch_bounds__(256, 3) k_blend_level(BlendArgs a, const Unit*
     }
 }
 
+// A column of the coarser level's reconstruction at rows y0 and y1, as pairs.
+__device__ __forceinline__ void recon_column(const float* r, int uw, int y0, int y1, int col, f32x2 (&t)[3])
+{
+    const float* a = r + ((size_t)y0 * uw + col) * 3;
+    const float* b = r + ((size_t)y1 * uw + col) * 3;
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch) t[ch] = pack2(a[ch], b[ch]);
+}
+
 // Collapse one level in place: recon_l = blended_l + Up(recon_l+1)
-// (SeamBlend.cpp:514-525).
+// (SeamBlend.cpp:514-525).  A thread makes four pixels of a row; as in
+// final_quad their taps are a window of two columns that slides by at most one
+// column per pixel.  A thread per pixel with its
+// own four taps and a 64-bit division took 0.75 ms on a 24-frame panorama, this
+// 0.54 (a 2048 x 2048 chunk 20 -> 16 us).
 __global__ void __launch_bounds__(256) k_collapse(BlendArgs a, const Unit* __restrict__ units, int level)
 {
     const Unit u = units[blockIdx.x];
     const TileDev& T = a.tiles[u.id];
     const int lw = T.lw[level], lh = T.lh[level];
     const int uw = T.lw[level + 1], uh = T.lh[level + 1];
+    const float sx = T.usx[level], sy = T.usy[level];
     const float* r = T.blend + T.loff[level + 1] * 3;
-    const long long base = (long long)u.by * u.rows * lw;
-    const long long n = min((long long)u.rows * lw, (long long)lw * lh - base);
-    for (long long q = threadIdx.x; q < n; q += blockDim.x)
+    float* band = T.blend + T.loff[level] * 3;
+    const f32x2 nz = neg_zero2();
+    const int row0 = u.by * u.rows;
+    const int rows = min(u.rows, lh - row0);
+    const int qpr = (lw + 3) >> 2;
+    const int nq = rows * qpr;
+    for (int qi = threadIdx.x; qi < nq; qi += blockDim.x)
     {
-        const long long pl = base + q;
-        const int y = (int)(pl / lw), x = (int)(pl - (long long)y * lw);
-        UpCoef c = up_coef_s(T.usx[level], T.usy[level], uw, uh, x, y);
-        float* b = T.blend + (T.loff[level] + pl) * 3;
-#pragma unroll
-        for (int ch = 0; ch < 3; ++ch)
+        const int y = row0 + qi / qpr, x = (qi - (qi / qpr) * qpr) * 4;
+        const int cnt = min(4, lw - x);
+        float* b = band + ((size_t)y * lw + x) * 3;
+        float v[12];
+        const bool vec = cnt == 4 && (reinterpret_cast<uintptr_t>(b) & 15) == 0;
+        if (vec)
         {
-            float v = up_mix(r[((size_t)c.y0 * uw + c.x0) * 3 + ch], r[((size_t)c.y0 * uw + c.x1) * 3 + ch],
-                             r[((size_t)c.y1 * uw + c.x0) * 3 + ch], r[((size_t)c.y1 * uw + c.x1) * 3 + ch], c.wx,
-                             c.wy);
-            b[ch] = fadd(b[ch], v);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                const float4 q = reinterpret_cast<const float4*>(b)[k];
+                v[4 * k] = q.x;
+                v[4 * k + 1] = q.y;
+                v[4 * k + 2] = q.z;
+                v[4 * k + 3] = q.w;
+            }
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 12; ++k) v[k] = k < 3 * cnt ? b[k] : 0.0f;
+        }
+        const UpCoef c = up_coef_s(sx, sy, uw, uh, x, y);
+        const f32x2 wyy = row_weights(c.wy);
+        int cur = c.x0;
+        f32x2 L[3], R[3];
+        recon_column(r, uw, c.y0, c.y1, cur, L);
+        recon_column(r, uw, c.y0, c.y1, c.x1, R);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            float wx = c.wx;
+            if (i > 0)
+            {
+                int x0;
+                up_coef_x(sx, uw, x + i, x0, wx);
+                if (x0 != cur)  // advanced by one column
+                {
+                    cur = x0;
+#pragma unroll
+                    for (int ch = 0; ch < 3; ++ch) L[ch] = R[ch];
+                    recon_column(r, uw, c.y0, c.y1, min(x0 + 1, uw - 1), R);
+                }
+            }
+            const f32x2 ix2 = dup2(fsub(1.0f, wx)), wx2 = dup2(wx);
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch)
+                v[3 * i + ch] = fadd(v[3 * i + ch], up_mix2(L[ch], R[ch], ix2, wx2, wyy, nz));
+        }
+        if (vec)
+        {
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                reinterpret_cast<float4*>(b)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 12; ++k)
+                if (k < 3 * cnt) b[k] = v[k];
         }
     }
 }
