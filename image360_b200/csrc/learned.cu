@@ -108,11 +108,11 @@ struct ConvShape
     // The epilogue's unit is kBatch blocks by kGroup channels: two rows (or the
     // two parities of a row), which hide each other's latencies, where the
     // accumulators then fit registers.
-    // With 8 warps the upper four take the upper half of the J rows.
-    static constexpr int kPer = kMB * 4 / EW;  // blocks of a warp, one column after the other
-    static constexpr int kGroup = EP == EP_RAW_UP ? 32 : NPAD, kBatch = EP == EP_COMPOSITE                                ? kPer
-                                  : kGroup <= 32 && (kParity || J * 4 / EW >= 2) ? 2
-                                                                                 : 1;
+    // Every four warps take the next J * 4 / EW of the rows (for EP_RAW_UP,
+    // which needs both, every second or only group of 32 channels instead).
+    static constexpr int kGroup = EP == EP_RAW_UP ? 32 : NPAD, kGroupStep = EP == EP_RAW_UP ? EW / 4 : 1;
+    static constexpr int kRows = EP == EP_RAW_UP ? J : J * 4 / EW, kPer = kRows * kBX;  // blocks of a warp, by columns
+    static constexpr int kBatch = EP == EP_COMPOSITE ? kPer : kGroup <= 32 && (kParity || kRows >= 2) ? 2 : 1;
     // Outputs leave by TMA from BUFS buffers per epilogue warp, each a unit as
     // swizzled tiles of 32 pixels and channels.
     static constexpr bool kStored = EP != EP_LOGITS && EP != EP_COMPOSITE;
@@ -127,7 +127,7 @@ struct ConvShape
     static_assert((J < 3 ? J : 3) * NPAD <= 256, "MMA columns");
     static_assert(2 * kSlotCols <= 512, "TMEM capacity");
     static_assert(kSmem <= 227u * 1024u, "shared memory");
-    static_assert(EW == 4 || (EW == 8 && J % 2 == 0), "epilogue warps split the rows in two");
+    static_assert(EW % 4 == 0 && kRows >= 1 && kPer % kBatch == 0, "epilogue warps split the rows");
     static_assert(!kParity || (TW == 16 && J == 2 && EW == 8 && kStored), "parities of a row in one unit");
     static_assert((EP != EP_RELU_POOL && EP != EP_RAW_UP) || kBatch == 2, "2x2 sums take two rows");
 };
@@ -312,7 +312,7 @@ __device__ __forceinline__ void composite_pixel(const i360b_blend_job& J, int y,
 // 8-channel TMA boxes and outputs stored a lane's 16 bytes at a time 176 us
 // and 55 for a kernel that averaged.  The 96-channel layer 0.22 ms (MMA issue
 // and operand fetch; 0.49 with the upsample expanded by warps), its backward
-// with the upsample's sums 0.22 (0.47 and 0.17 apart).
+// with the upsample's sums 0.21 (0.47 and 0.17 apart).
 // ---------------------------------------------------------------------------
 template <int CIN, int NPAD, int TW, int J, int STAGES, int LD, int EP, int EW, int BUFS>
 __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW, BUFS>::kThreads, 1)
@@ -477,11 +477,13 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
     }
     else if (warp < EW)
     {
-        // Warp w reads TMEM lane quadrant w % 4, of rows `firstRow` on.
-        const int quad = warp & 3, firstRow = (warp >> 2) * (J * 4 / EW);
+        // Warp w reads TMEM lane quadrant w % 4, of rows `firstRow` and groups
+        // `firstGroup` on.
+        constexpr int kRows = S::kRows;
+        const int quad = warp & 3, firstRow = EP == EP_RAW_UP ? 0 : (warp >> 2) * kRows,
+                  firstGroup = EP == EP_RAW_UP ? warp >> 2 : 0;
         unsigned char* buf = outBufs + warp * (BUFS * S::kOutBuf);
         int next = 0;  // output buffer
-        constexpr int kRows = S::kPer / S::kBX;  // rows of a column that this warp takes
         constexpr int kBatch = S::kBatch, kGroup = S::kGroup;
         // Pixel of this lane in the n-th block of tile t.
         struct Px
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
             }
         };
         TileWalk t(tilesX, tilesY, blockIdx.x, gridDim.x);
-        load_inputs(t, 0, 0);
+        load_inputs(t, 0, firstGroup);
         for (int i = 0; i < myTiles && ok; ++i)
         {
             const int acc = i & 1, img = t.img;
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
 #pragma unroll 1
             for (int n = 0; n < S::kPer; n += kBatch)
 #pragma unroll 1
-                for (int group = 0; group < NPAD / kGroup; ++group)
+                for (int group = firstGroup; group < NPAD / kGroup; group += S::kGroupStep)
                 {
                     auto at = [&](int k) {  // accumulators of the unit's k-th block
                         return base + ((n + k) / kRows * J + firstRow + (n + k) % kRows) * NPAD + group * kGroup;
@@ -564,7 +566,7 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
                     for (int k = 0; k < kBatch; ++k)
 #pragma unroll
                         for (int cb = 0; cb < kGroup / 16; ++cb) tc::tmem_zero16(at(k) + cb * 16);
-                    const bool lastGroup = group + 1 == NPAD / kGroup, last = lastGroup && n + kBatch >= S::kPer;
+                    const bool lastGroup = group + S::kGroupStep >= NPAD / kGroup, last = lastGroup && n + kBatch >= S::kPer;
                     if (last)
                     {
                         tc::tmem_wait_st();
@@ -701,9 +703,9 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
                         }
                     }
                     // inputs of the unit after this one
-                    if (!lastGroup) load_inputs(t, n, group + 1);
-                    else if (!last) load_inputs(t, n + kBatch, 0);
-                    else if (i + 1 < myTiles) load_inputs(following, 0, 0);
+                    if (!lastGroup) load_inputs(t, n, group + S::kGroupStep);
+                    else if (!last) load_inputs(t, n + kBatch, firstGroup);
+                    else if (i + 1 < myTiles) load_inputs(following, 0, firstGroup);
                     if (S::kStored && (EP != EP_RAW_UP || group == 0))
                     {
                         unsigned char* ob = buf + next * S::kOutBuf;
@@ -1146,6 +1148,9 @@ __device__ __forceinline__ float feathered_mask(const float* e, float x, float y
     return 0.25f + 0.75f * fminf(1.0f, sqrtf(d2) / kFeather);
 }
 
+// The network's input: each slot's scaled values and feathered mask.  Bound by
+// load latency: 64 windows of 256 x 256 70 us (235 MB, 36 us at the measured
+// copy rate); 91 us with each slot's loads behind the test of the one before.
 __global__ void k_pack_input(const i360b_blend_job* __restrict__ jobs, int n, int h, int w, bf16* __restrict__ x0)
 {
     const long long total = (long long)n * h * w;
@@ -1161,16 +1166,15 @@ __global__ void k_pack_input(const i360b_blend_job* __restrict__ jobs, int n, in
         for (int i = 0; i < 16; ++i) ch[i] = 0.0f;
         if (x < J.width && y < J.height)
         {
+            uint2 v[kSlots];
+            load_slots_raw(J, y, x, v);  // all loads before the first value is needed
 #pragma unroll
             for (int i = 0; i < kSlots; ++i)
             {
-                if (!J.slot[i]) continue;
-                const unsigned short* p = J.slot[i] + (long long)y * J.rowStride + (long long)x * J.pixStride;
-                const unsigned short r = p[0], g = p[1], b = p[2];
-                if ((r | g | b) == 0) continue;
-                ch[4 * i] = r * kInScale;
-                ch[4 * i + 1] = g * kInScale;
-                ch[4 * i + 2] = b * kInScale;
+                if ((v[i].x | v[i].y) == 0) continue;
+                ch[4 * i] = (unsigned short)v[i].x * kInScale;
+                ch[4 * i + 1] = (unsigned short)(v[i].x >> 16) * kInScale;
+                ch[4 * i + 2] = (unsigned short)v[i].y * kInScale;
                 ch[4 * i + 3] = feathered_mask(J.edges[i], (float)x, (float)y);
             }
         }
@@ -1450,8 +1454,15 @@ int run_conv(ConvArgs a, cudaStream_t s)
     return check_launch("conv3x3 kernel");
 }
 
-// The (cin, npad) shapes the network uses, forward and backward, with their
-// tile shape and ring depth.
+// The (cin, npad) shapes the network uses, forward and backward, with tile
+// width, rows' interleave J, ring depth, epilogue warps and output buffers.
+// J = 4 where the halos fit twice beside the weights (half the MMAs of one per
+// tap), else 2 (two thirds); 64 windows of 256 x 256:
+//   * 16 epilogue warps for the blend head, whose layer loads it must cover:
+//     90 us, 129 with 8; the others are the same with 8 and 16;
+//   * 8 for EP_RAW_UP: 206 us, 224 with 4;
+//   * the 64-channel layers with a third ring slot and 4 warps: 75 us, 62 so;
+//   * the 96-channel layer with J = 4 and one slot: 0.42 ms, 0.22 so.
 int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cudaStream_t s)
 {
 #define I360B_CONV(CI, NP, TW, J, ST, LD, EP_, EW, BUFS)      \
@@ -1465,12 +1476,12 @@ int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cuda
     I360B_CONV(96, 32, 16, 2, 2, LD_CONCAT, EP_RELU, 8, 1)
     I360B_CONV(96, 32, 8, 2, 2, LD_SPLIT, EP_RELU, 8, 1)
     I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_LOGITS, 8, 1)
-    I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_COMPOSITE, 8, 1)
+    I360B_CONV(32, 16, 16, 4, 2, LD_PLAIN, EP_COMPOSITE, 16, 1)
     // backward data
     I360B_CONV(16, 32, 16, 4, 3, LD_PLAIN, EP_MASK, 8, 2)
     I360B_CONV(32, 32, 16, 4, 2, LD_PLAIN, EP_MASK, 8, 1)
     I360B_CONV(32, 96, 8, 2, 3, LD_PLAIN, EP_RAW, 8, 1)
-    I360B_CONV(32, 96, 8, 2, 3, LD_PLAIN, EP_RAW_UP, 4, 2)
+    I360B_CONV(32, 96, 8, 2, 3, LD_PLAIN, EP_RAW_UP, 8, 2)
     I360B_CONV(64, 64, 8, 2, 2, LD_PLAIN, EP_MASK, 8, 1)
     I360B_CONV(64, 32, 8, 4, 2, LD_PLAIN, EP_RAW, 4, 1)
 #undef I360B_CONV
