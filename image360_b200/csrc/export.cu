@@ -60,10 +60,9 @@ __global__ void k_export_source_table(float scale, int n, int* tab)
 // A warp writes kExportWords x 32 aligned 4-byte words of one placement row,
 // a word per lane at a time, so its stores are whole 128-byte lines; the
 // row's first and last bytes, which may share a word with a neighbouring
-// placement, are stored by the byte.  Bound by HBM: at scale 1 (IDENTITY)
-// the source samples of a word are four consecutive u16, read as two or three
-// words (the samples of a row lie at one phase of the word grid); at any
-// other scale each byte looks its source pixel up.  `clear`: a pixel without
+// placement, are stored by the byte.  Scale 1: the source samples of a word
+// are four consecutive u16, read as two or three words (the samples of a row
+// lie at one phase of the word grid).  Bound by HBM.  `clear`: a pixel without
 // a source (rounding at the placement's edge) is written as 0 here - the
 // placements do not overlap and cover the canvas, which is then not cleared
 // beforehand.  Else such pixels are left alone.
@@ -71,10 +70,8 @@ __global__ void k_export_source_table(float scale, int n, int* tab)
 // per thread (2-byte loads, 1-byte stores) took 735 us and the clearing 83 us.
 constexpr int kExportWords = 8;
 
-template <bool IDENTITY>
 __global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restrict__ tiles, int t0, float scale,
-                                                      int ow, int oh, const int* __restrict__ srcOf, bool clear,
-                                                      unsigned char* __restrict__ out)
+                                                      int ow, int oh, bool clear, unsigned char* __restrict__ out)
 {
     const ExportTile T = tiles[t0 + blockIdx.z];
     int p[4];
@@ -86,8 +83,8 @@ __global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restri
     const long long x0 = p[0] < 0 ? -(long long)p[0] : 0;
     const long long x1 = (long long)p[0] + p[2] > ow ? (long long)ow - p[0] : p[2];
     if (x0 >= x1) return;
-    const int sy = IDENTITY ? dy : srcOf[dy];
-    const bool rowIn = sy >= 0 && sy < T.h;
+    const int sy = dy;  // int(d / 1.0f) = d while the float holds d exactly
+    const bool rowIn = sy < T.h;
     if (!rowIn && !clear) return;
     // bytes [b0, b1) of the placement row, at o + b
     const long long b0 = x0 * 3, b1 = x1 * 3;
@@ -103,7 +100,7 @@ __global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restri
     // Samples [e0, e1) of the row may be read as words: the words that hold
     // samples b .. b + 3 hold b - 1 .. b + 4 at most, inside the chunk.
     const long long e0 = firstElem > 0 ? 0 : 1, e1 = firstElem + rowElems < chunkElems ? rowElems : rowElems - 1;
-    if (IDENTITY && rowIn && base >= b0 && base >= e0 && base + (kExportWords - 1) * 128 + 4 <= b1 &&
+    if (rowIn && base >= b0 && base >= e0 && base + (kExportWords - 1) * 128 + 4 <= b1 &&
         base + (kExportWords - 1) * 128 + 4 <= e1)
     {
         const uint32_t* w = reinterpret_cast<const uint32_t*>(src + base - (odd ? 1 : 0));
@@ -126,7 +123,7 @@ __global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restri
         for (int j = 0; j < kExportWords; ++j) d[j * 32] = r[j];
         return;
     }
-    // the ends of a row, and any other scale
+    // the ends of a row
     for (int j = 0; j < kExportWords; ++j)
     {
         const long long b = base + j * 128;
@@ -139,10 +136,8 @@ __global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restri
         {
             const long long e = b + i;
             if (!rowIn || e < b0 || e >= b1) continue;
-            const int dx = (int)(e / 3);
-            const int sx = IDENTITY ? dx : srcOf[dx];
-            if (sx < 0 || sx >= T.w) continue;
-            v |= (uint32_t)(__ldg(src + (size_t)sx * 3 + (int)(e - (long long)dx * 3)) >> 8) << (8 * i);
+            if (e >= rowElems) continue;
+            v |= (uint32_t)(__ldg(src + e) >> 8) << (8 * i);
             have |= 1u << i;
         }
         if (whole && (have == 15u || clear))
@@ -153,6 +148,51 @@ __global__ void __launch_bounds__(256) k_export_place(const ExportTile* __restri
             for (int i = 0; i < 4; ++i)
                 if (b + i >= b0 && b + i < b1 && (clear || ((have >> i) & 1u))) o[b + i] = (unsigned char)(v >> (8 * i));
         }
+    }
+}
+
+// The same at any other scale: kExportPx pixels of a row per thread, 32 apart,
+// each from the source pixel that the table gives.  Bound by load latency: the
+// pixels' lookups and samples are in flight together.  16000 x 9000 into 9000 x
+// 5062: 148 us; one pixel per thread 231 and the clearing 24; a word per lane,
+// each byte looked up by itself, slower than either on small previews.
+constexpr int kExportPx = 4;
+
+__global__ void __launch_bounds__(256) k_export_scaled(const ExportTile* __restrict__ tiles, int t0, float scale,
+                                                       int ow, int oh, const int* __restrict__ srcOf, bool clear,
+                                                       unsigned char* __restrict__ out)
+{
+    const ExportTile T = tiles[t0 + blockIdx.z];
+    int p[4];
+    placement(T, scale, p);
+    const int dx0 = blockIdx.x * (32 * kExportPx) + threadIdx.x, dy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (dx0 >= p[2] || dy >= p[3]) return;
+    const int oy = p[1] + dy;
+    if (oy < 0 || oy >= oh) return;
+    const int sy = __ldg(srcOf + dy);
+    const bool rowIn = sy >= 0 && sy < T.h;
+    if (!rowIn && !clear) return;
+    int sx[kExportPx];
+#pragma unroll
+    for (int k = 0; k < kExportPx; ++k) sx[k] = dx0 + 32 * k < p[2] ? __ldg(srcOf + dx0 + 32 * k) : -1;
+    unsigned short v[kExportPx][3];
+    const unsigned short* row = T.src + (size_t)(rowIn ? sy : 0) * T.w * 3;
+#pragma unroll
+    for (int k = 0; k < kExportPx; ++k)
+    {
+        const bool in = rowIn && sx[k] >= 0 && sx[k] < T.w;
+        if (!in) sx[k] = -1;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) v[k][c] = in ? __ldg(row + (size_t)sx[k] * 3 + c) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kExportPx; ++k)
+    {
+        const int dx = dx0 + 32 * k, ox = p[0] + dx;
+        if (dx >= p[2] || ox < 0 || ox >= ow || (sx[k] < 0 && !clear)) continue;
+        unsigned char* o = out + ((size_t)oy * ow + ox) * 3;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[c] = (unsigned char)(v[k][c] >> 8);
     }
 }
 
@@ -232,24 +272,28 @@ int export_preview(const std::vector<ExportTile>& tiles, int totalW, int totalH,
     desc.s = tab.s = s;
     const int tabN = std::max(maxW, maxH);
     I360B_TRY(dev_alloc(&desc.p, tiles.size() * sizeof(ExportTile), s, "preview export"));
-    I360B_TRY(dev_alloc(&tab.p, (size_t)tabN * sizeof(int), s, "preview export"));
+    // int(d / 1.0f) = d while the float holds d exactly
+    const bool identity = scale == 1.0f && tabN <= (1 << 24);
+    if (!identity) I360B_TRY(dev_alloc(&tab.p, (size_t)tabN * sizeof(int), s, "preview export"));
     I360B_CUDA(cudaMemcpyAsync(desc.p, tiles.data(), tiles.size() * sizeof(ExportTile), cudaMemcpyHostToDevice, s),
                "preview export");
-    k_export_source_table<<<(tabN + 255) / 256, 256, 0, s>>>(scale, tabN, static_cast<int*>(tab.p));
-    I360B_TRY(check_launch("preview source table kernel"));
+    if (!identity)
+    {
+        k_export_source_table<<<(tabN + 255) / 256, 256, 0, s>>>(scale, tabN, static_cast<int*>(tab.p));
+        I360B_TRY(check_launch("preview source table kernel"));
+    }
     const dim3 block(32, 8);
     const ExportTile* dT = static_cast<const ExportTile*>(desc.p);
     const int* dTab = static_cast<const int*>(tab.p);
-    // int(d / 1.0f) = d while the float holds d exactly
-    const bool identity = scale == 1.0f && tabN <= (1 << 24);
     // a row of w pixels spans at most 3w + 3 bytes from its first word on
     auto grid = [&](int w, int h, size_t chunks) {
-        return dim3((unsigned)((3ll * w + 3 + kExportWords * 128 - 1) / (kExportWords * 128)), (unsigned)((h + 7) / 8),
-                    (unsigned)chunks);
+        const long long cols = identity ? (3ll * w + 3 + kExportWords * 128 - 1) / (kExportWords * 128)
+                                        : (w + 32 * kExportPx - 1) / (32 * kExportPx);
+        return dim3((unsigned)cols, (unsigned)((h + 7) / 8), (unsigned)chunks);
     };
     auto place = [&](const dim3& g, int t0) {
-        if (identity) k_export_place<true><<<g, block, 0, s>>>(dT, t0, scale, ow, oh, dTab, clear, dOut);
-        else k_export_place<false><<<g, block, 0, s>>>(dT, t0, scale, ow, oh, dTab, clear, dOut);
+        if (identity) k_export_place<<<g, block, 0, s>>>(dT, t0, scale, ow, oh, clear, dOut);
+        else k_export_scaled<<<g, block, 0, s>>>(dT, t0, scale, ow, oh, dTab, clear, dOut);
         return check_launch("preview placement kernel");
     };
     if (!overlap) return place(grid(maxW, maxH, tiles.size()), 0);
