@@ -160,7 +160,7 @@ int device();
 int sm_count();
 // The calling thread's stream for the synchronous host-buffer API.
 cudaStream_t thread_stream();
-// Stream-ordered allocation from the device's pool (kept for the process life).
+// Stream-ordered allocation from the device's pool (kept until i360b_shutdown).
 int dev_alloc(void** p, size_t bytes, cudaStream_t s, const char* what);
 void dev_free(void* p, cudaStream_t s);
 

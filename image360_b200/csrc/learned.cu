@@ -800,7 +800,7 @@ __global__ void __launch_bounds__(ConvShape<CIN, NPAD, TW, J, STAGES, LD, EP, EW
 // Every wait is bounded; a timeout sets the error flag and the CTA winds down
 // after its loads have landed.
 //
-// 64 windows of 256 x 256, all eight layers with their bias gradients: 0.70
+// 64 windows of 256 x 256, all eight layers with their bias gradients: 0.73
 // ms for 3.3 GB of X and G (0.50 at the measured copy rate); the longest jobs,
 // the 96-channel layer's 63 CTAs, set the end.  With a launch per layer 1.9 ms;
 // with the pixels of an MMA successive (three full copies of G and an upsample
@@ -859,7 +859,7 @@ struct WgradShape
 };
 
 template <int CX, int COUT, bool UP>
-__device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float (&sBias)[128][9], int* error)
+__device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, double (&sBias)[128][9], int* error)
 {
     using S = WgradShape<CX, COUT, UP>;
     extern __shared__ unsigned char smemRaw[];
@@ -971,10 +971,13 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
     {
         // This thread's chunk position and pixels of the planes + 1 and + 0,
         // 128 rows of COUT / 8 chunks; the pixels it sees keep the chunk's
-        // place in the swizzle, so its channels are fixed.
+        // place in the swizzle, so its channels are fixed.  The sums cancel,
+        // so chains of FP32 additions stay as short as 8 tiles.
         constexpr int kO8 = COUT / 8;
         const int pos = tid % kO8, px0 = tid / kO8;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        double total[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        const uint32_t zero = (uint32_t)a.bias >> 1;  // (a.bias is 1 here)
         for (int i = 0; i < myTiles; ++i)
         {
             const int s = i % S::kStages;
@@ -984,20 +987,34 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
                 break;
             }
             const unsigned char* g = smem + s * S::kStage + S::kX + S::kGPlane;
+            uint32_t seen = 0;
 #pragma unroll
             for (int k = 0; k < kWgRows * kWgTW * kO8 / 128; ++k)
             {
                 const int p = px0 + k * (128 / kO8);
+                const uint4 q = *reinterpret_cast<const uint4*>(g + p * COUT * 2 + pos * 16);
+                seen |= q.x;
                 float v[8];
-                unpack8_bf16(*reinterpret_cast<const uint4*>(g + p * COUT * 2 + pos * 16), v);
+                unpack8_bf16(q, v);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) acc[j] += v[j];
             }
+            // The next TMA may overwrite the stage as soon as the arrival is
+            // seen, which loads still in flight are not behind: the tensor
+            // core's fetches can hold them up for longer than a TMA takes.
+            // So the arrival depends on what they returned.
             __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&empty[s]);
+            if (lane == 0) tc::mbar_arrive_after(&empty[s], seen, zero);
+            if ((i & 7) == 7 || i + 1 == myTiles)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                {
+                    total[j] += acc[j];
+                    acc[j] = 0.0f;
+                }
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sBias[tid][j] = acc[j];
+        for (int j = 0; j < 8; ++j) sBias[tid][j] = total[j];
     }
     __syncthreads();
     float* out = a.partial + (size_t)slice * (9 * a.cin * COUT + COUT);
@@ -1029,10 +1046,10 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, float 
         }
         if (bias && tid < COUT)
         {
-            float b = 0.0f;
+            double b = 0.0;
             for (int t = 0; t < 128; ++t)
                 if (swizzled_chunk<COUT>(t / (COUT / 8), t % (COUT / 8)) == tid >> 3) b += sBias[t][tid & 7];
-            out[9 * a.cin * COUT + tid] = b;
+            out[9 * a.cin * COUT + tid] = (float)b;
         }
     }
     if (!ok && lane == 0) atomicOr(error, 1);
@@ -1050,7 +1067,7 @@ __global__ void __launch_bounds__(192, 1) k_conv3x3_wgrad(const __grid_constant_
     while (j + 1 < b.jobs && (int)blockIdx.x >= b.job[j + 1].firstBlock) ++j;
     const WgradJob& a = b.job[j];
     const int slice = blockIdx.x - a.firstBlock;
-    __shared__ float sBias[128][9];
+    __shared__ double sBias[128][9];
     switch (a.kind)
     {
         case WG_16_32: wgrad_slice<16, 32, false>(a, slice, sBias, b.error); break;
@@ -1119,7 +1136,11 @@ __global__ void k_wgrad_reduce(const __grid_constant__ WgradReduce r)
         if (co < a.cout) a.dw[((size_t)co * 9 + dy * 3 + dx) * a.cin + c] = s;
     }
     else if (idx - weights < a.cout)
-        a.db[idx - weights] = s;
+    {
+        double b = 0.0;  // (a sum that cancels)
+        for (int g = 0; g < a.slices; ++g) b += a.partial[(size_t)g * count + idx];
+        a.db[idx - weights] = (float)b;
+    }
 }
 
 // ---------------------------------------------------------------------------

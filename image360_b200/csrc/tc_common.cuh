@@ -234,6 +234,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* mbar, uint32_t b
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
                  : "memory");
 }
+// Arrives once `value` is in its register; zero: 0, not known to the compiler.
+__device__ __forceinline__ void mbar_arrive_after(uint64_t* mbar, uint32_t value, uint32_t zero)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar) + (value & zero)) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");

@@ -376,3 +376,19 @@ def test_conv3x3_forward_tile_edges(backend, cin, cout, ep, skip, n, h, w):
         ref = torch.where(act.float() > 0, ref, torch.zeros_like(ref))
     tol = (1e-4 if ep == 1 else 2 ** -8) * ref.abs() + 1e-4 * ref.abs().max()
     assert bool(((out.float() - ref).abs() <= tol).all())
+
+
+def test_gradients_are_deterministic(backend):
+    """Every weight and bias gradient has a fixed order of sums: repeated calls
+    over a batch that keeps each CTA's ring of tiles busy give the same bits."""
+    from image360_b200 import blendnet as bn
+    n, h, w = 16, 256, 256
+    layers = _layers(23, n, h, w)
+    dl, dt, _, jobs = _device_batch(layers, _owner_target(layers))
+    net = bn.BlendNet(seed=1)
+    net.set_params(_random_params(6))
+    first, _ = net.gradients(jobs, n, w, h)
+    for k in range(40):
+        again, _ = net.gradients(jobs, n, w, h)
+        assert np.array_equal(first, again), (k, int((first != again).sum()))
+    net.close()
