@@ -15,7 +15,7 @@
  *   - i360b_<op>: the IComputeBackend operations.  Host buffers in, host
  *     buffers out, synchronous: results are in host memory on return.  Each
  *     calling thread gets its own CUDA stream.  Device memory comes from a
- *     stream-ordered pool that is kept for the life of the process.
+ *     stream-ordered pool that is kept until i360b_shutdown.
  *   - i360b_launch_<op> / i360b_render_*: device-resident, stream-ordered
  *     launchers for callers that keep frames in HBM.  `stream` is a
  *     cudaStream_t passed as void* (NULL = the legacy default stream).
