@@ -981,7 +981,9 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, double
         for (int i = 0; i < myTiles; ++i)
         {
             const int s = i % S::kStages;
-            if (!tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins))
+            // The warp goes on, or gives up, as one.
+            const bool ready = tc::mbar_wait(&full[s], (i / S::kStages) & 1, kWaitSpins);
+            if (!__all_sync(0xffffffffu, ready))
             {
                 ok = false;
                 break;
@@ -993,7 +995,7 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, double
             {
                 const int p = px0 + k * (128 / kO8);
                 const uint4 q = *reinterpret_cast<const uint4*>(g + p * COUT * 2 + pos * 16);
-                seen |= q.x;
+                seen |= q.x | q.y | q.z | q.w;
                 float v[8];
                 unpack8_bf16(q, v);
 #pragma unroll
@@ -1002,8 +1004,8 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, double
             // The next TMA may overwrite the stage as soon as the arrival is
             // seen, which loads still in flight are not behind: the tensor
             // core's fetches can hold them up for longer than a TMA takes.
-            // So the arrival depends on what they returned.
-            __syncwarp();
+            // So the arrival depends on what every lane's loads returned.
+            seen = __reduce_or_sync(0xffffffffu, seen);
             if (lane == 0) tc::mbar_arrive_after(&empty[s], seen, zero);
             if ((i & 7) == 7 || i + 1 == myTiles)
 #pragma unroll
@@ -1052,7 +1054,7 @@ __device__ __forceinline__ void wgrad_slice(const WgradJob& a, int slice, double
             out[9 * a.cin * COUT + tid] = (float)b;
         }
     }
-    if (!ok && lane == 0) atomicOr(error, 1);
+    if (!ok) atomicOr(error, 1);
     __syncthreads();
     if (warp == 0)
     {

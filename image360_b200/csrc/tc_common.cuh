@@ -235,6 +235,7 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* mbar, uint32_t b
                  : "memory");
 }
 // Arrives once `value` is in its register; zero: 0, not known to the compiler.
+// For a warp's reads, `value` is made from every lane's (__reduce_or_sync).
 __device__ __forceinline__ void mbar_arrive_after(uint64_t* mbar, uint32_t value, uint32_t zero)
 {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar) + (value & zero)) : "memory");

@@ -392,3 +392,19 @@ def test_gradients_are_deterministic(backend):
         again, _ = net.gradients(jobs, n, w, h)
         assert np.array_equal(first, again), (k, int((first != again).sum()))
     net.close()
+
+
+@pytest.mark.parametrize("n,h,w", [(1, 2, 256), (1, 130, 512), (5, 70, 256)])
+def test_gradients_repeat_at_every_ring_fill(backend, n, h, w):
+    """The bias sums read stages that the next tile's loads overwrite: the same
+    bits from repeated calls with rings that never fill, fill once, and wrap."""
+    from image360_b200 import blendnet as bn
+    layers = _layers(31 + n, n, h, w)
+    dl, dt, _, jobs = _device_batch(layers, _owner_target(layers))
+    net = bn.BlendNet(seed=1)
+    net.set_params(_random_params(7))
+    first, _ = net.gradients(jobs, n, w, h)
+    for k in range(20):
+        again, _ = net.gradients(jobs, n, w, h)
+        assert np.array_equal(first, again), (k, int((first != again).sum()))
+    net.close()
