@@ -6,6 +6,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tap_words.cuh"
 
 namespace i360b
 {
@@ -46,24 +47,6 @@ __host__ __device__ __forceinline__ WarpSource warp_source(const unsigned short*
 __host__ __device__ __forceinline__ bool homography_affine(const float* H)
 {
     return H[6] == 0.0f && H[7] == 0.0f && H[8] == 1.0f;
-}
-
-// Two horizontally adjacent RGB48 pixels (six u16) from byte offset o (even)
-// of a frame's words, as three words in memory order: the three or four
-// aligned words that hold them (each read word holds one of the six values;
-// the fourth only where the values reach it), shifted together.  Half the L1
-// accesses of six 2-byte loads.
-template <typename Off>
-__device__ __forceinline__ void load_tap_pair(const uint32_t* words, Off o, uint32_t w[3])
-{
-    const uint32_t* q = words + (o >> 2);
-    const unsigned sh = (unsigned)o << 3;  // 0 or 16, modulo 32
-    const uint32_t r0 = __ldg(q), r1 = __ldg(q + 1), r2 = __ldg(q + 2);
-    uint32_t r3 = 0;
-    if (o & 2) r3 = __ldg(q + 3);
-    w[0] = __funnelshift_r(r0, r1, sh);
-    w[1] = __funnelshift_r(r1, r2, sh);
-    w[2] = __funnelshift_r(r2, r3, sh);
 }
 
 // Both rows of taps at column x0 of row y0, given as 2^23 + x0 and 2^23 + y0.
