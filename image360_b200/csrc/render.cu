@@ -104,6 +104,15 @@ __global__ void k_setup_items(ItemDev* items, const double* toCanvas, const int*
 // freed by the call.  A 4096 x 4096 chunk of 8 contributors needs 2.6 GB.
 constexpr size_t kPooledArenaMax = size_t(4) << 30;
 
+// Stands for a list of Units where only its length is wanted.
+struct UnitCount
+{
+    size_t n = 0;
+    void clear() { n = 0; }
+    void push_back(const Unit&) { ++n; }
+    size_t size() const { return n; }
+};
+
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 
 __global__ void k_count_cov(const ItemDev* items, const TileDev* tiles, int n, unsigned long long* out)
@@ -251,12 +260,16 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
         for (int ws : {0, 1})
         {
             warpShape = ws;
-            make_units(8, units);
-            cap = std::max(cap, units.size());
+            UnitCount most;
+            make_units(8, most);
+            cap = std::max(cap, most.size());
         }
         warpShape = shape;
         unitCap = (int)cap;
     }
+    UnitCount count;
+    make_units(bandRows, count);
+    units.reserve(count.size());
     make_units(bandRows, units);
     if (oneShot) unitCap = (int)units.size();
     std::vector<int> ints;
@@ -341,23 +354,31 @@ int Plan::build(const std::vector<TileSpec>& specs, int numBands, bool renderPat
     dError = reinterpret_cast<int*>(base + metaOff + unitBytes + intBytes + itemBytes + tileBytes);
     dSeamCycles = reinterpret_cast<unsigned long long*>(base + metaOff + unitBytes + intBytes + itemBytes + tileBytes + 256);
     dSeamTile = reinterpret_cast<unsigned long long*>(base + metaOff + unitBytes + intBytes + itemBytes + tileBytes + 512);
-    // The tables lie next to each other (unused list capacity, then zeroed
-    // flags and counters included): one upload.
+    // The work lists, then the tables behind them, which lie next to each
+    // other (zeroed flags and counters included).  A one-chunk plan's lists
+    // fill their capacity, so one upload holds everything.  A kept plan's
+    // lists leave most of theirs unused (it holds bands of any height) and
+    // are megabytes: they go up from where they were built.
     {
-        const size_t metaBytes = bytes - metaOff;
-        std::vector<char> meta(metaBytes, 0);
-        char* m = meta.data();
-        if (!units.empty()) std::memcpy(m, units.data(), units.size() * sizeof(Unit));
-        if (!ints.empty()) std::memcpy(m + unitBytes, ints.data(), ints.size() * sizeof(int));
-        if (nItems) std::memcpy(m + unitBytes + intBytes, items.data(), nItems * sizeof(ItemDev));
-        if (nTiles) std::memcpy(m + unitBytes + intBytes + itemBytes, tiles.data(), nTiles * sizeof(TileDev));
+        const size_t tailOff = pooled ? 0 : unitBytes, tailBytes = bytes - metaOff - tailOff;
+        std::vector<char> tail(tailBytes, 0);
+        auto put = [&](size_t off, const void* src, size_t n) {
+            if (n) std::memcpy(tail.data() + (off - tailOff), src, n);
+        };
+        const size_t listBytes = units.size() * sizeof(Unit);
+        if (pooled) put(0, units.data(), listBytes);
+        put(unitBytes, ints.data(), ints.size() * sizeof(int));
+        put(unitBytes + intBytes, items.data(), nItems * sizeof(ItemDev));
+        put(unitBytes + intBytes + itemBytes, tiles.data(), nTiles * sizeof(TileDev));
         // Scratch that is the caller's or the pool's may still be in use by
         // earlier work on the caller's stream; the copy from pageable memory
         // returns once the source has been read.
-        if (extArena || pooled)
-            I360B_CUDA(cudaMemcpyAsync(base + metaOff, m, metaBytes, cudaMemcpyHostToDevice, stream), "plan upload");
-        else
-            I360B_CUDA(cudaMemcpy(base + metaOff, m, metaBytes, cudaMemcpyHostToDevice), "plan upload");
+        auto upload = [&](size_t off, const void* src, size_t n) {
+            return extArena || pooled ? cudaMemcpyAsync(base + metaOff + off, src, n, cudaMemcpyHostToDevice, stream)
+                                      : cudaMemcpy(base + metaOff + off, src, n, cudaMemcpyHostToDevice);
+        };
+        if (!pooled && listBytes) I360B_CUDA(upload(0, units.data(), listBytes), "plan upload");
+        I360B_CUDA(upload(tailOff, tail.data(), tailBytes), "plan upload");
     }
     seamList = dInts + seamStart;
     return I360B_SUCCESS;
@@ -370,7 +391,8 @@ constexpr int kListBase2 = 3 + (kMaxBands - 1) + kMaxBands + kMaxBands;
 constexpr int kListFine = kListBase2 + 1;
 constexpr int kListsPerChain = kListFine + 1;
 
-void Plan::make_units(int rows, std::vector<Unit>& units)
+template <typename List>
+void Plan::make_units(int rows, List& units)
 {
     units.clear();
     // Band units: `rows` full-width rows each (per-pixel kernels).

@@ -149,7 +149,10 @@ struct Plan
     std::vector<std::pair<int, cudaGraphExec_t>> rangeGraphs;
     int kernels_per_execute() const;
     // Work lists for band height `rows` (fills `lists`).
-    void make_units(int rows, std::vector<Unit>& units);
+    // The work lists for bands of `rows` rows into a vector of Units, or only
+    // their number (UnitCount).
+    template <typename List>
+    void make_units(int rows, List& units);
     // Switches the band height and chamfer ring depth; the next execute
     // recaptures the graph.  Synchronous on `s`.
     int set_tuning(int rows, int slots, cudaStream_t s);

@@ -170,3 +170,40 @@ def test_render_plan_stage_ranges_equal_execute(backend):
     assert pb.execute_stages(3, 1) == ComputeResult.INVALID_PARAM
     pa.close()
     pb.close()
+
+
+def _uploaded_bytes(call, tmp_path):
+    """Host-to-device bytes of a call, from the profiler's record of copies."""
+    import json
+    torch = _torch()
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        result = call()
+        torch.cuda.synchronize()
+    path = str(tmp_path / "trace.json")
+    p.export_chrome_trace(path)
+    with open(path) as f:
+        events = json.load(f)["traceEvents"]
+    copies = [e["args"]["bytes"] for e in events if "HtoD" in e.get("name", "") and "bytes" in e.get("args", {})]
+    if not copies:
+        pytest.skip("no record of copies from the profiler")
+    return result, sum(copies)
+
+
+def test_plan_creation_uploads_only_the_lists_in_use(lib, backend, tmp_path):
+    """A plan's work lists have room for bands of 8 rows.  Creating it uploads
+    the lists of its own 16-row bands: less than retuning to 8 rows does."""
+    torch = _torch()
+    src = torch.zeros((600, 800, 3), dtype=torch.int16, device="cuda")
+    out = torch.zeros((512, 512, 3), dtype=torch.int16, device="cuda")
+    H = np.array([[1.0, 0, 0], [0, 1, 0], [0, 0, 1]])
+    frames = [(src.data_ptr(), 800, 600, H, 1.0)] * 4
+    tiles = [(0, 0, 512, 512, [0, 1, 2, 3], out.data_ptr())] * 24
+    plan, created = _uploaded_bytes(lambda: RenderPlan(frames, tiles, 6, COORDS_REFERENCE), tmp_path)
+    t = plan.tuning()
+    assert t["band_rows"] == 16
+    rc, retuned = _uploaded_bytes(lambda: plan.set_tuning(8, t["dt_slots"], t["fused_levels"], t["warp_shape"]), tmp_path)
+    assert rc == ComputeResult.SUCCESS
+    assert created < retuned, (created, retuned)
+    plan.close()
