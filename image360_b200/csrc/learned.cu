@@ -1512,6 +1512,18 @@ int dispatch_conv(int cin, int npad, int loader, int ep, const ConvArgs& a, cuda
                 ep);
 }
 
+// The kernel of a layer's jobs (of those of a plain input where 96 channels
+// are concatenated), -1 where there is none.
+int wgrad_kind(int cin, int cout)
+{
+    return cout == 64                  ? (cin == 32 || cin == 64 ? WG_32_64 : -1)
+           : cout == 16                ? (cin == 32 ? WG_32_16 : -1)
+           : cout != 32                ? -1
+           : cin == 16                 ? WG_16_32
+           : cin == 32 || cin == 96    ? WG_32_32
+                                       : -1;
+}
+
 // Slices of a layer's sums at most: one 128-row block of (tap, cin) per SM.
 int wgrad_slices(int cin) { return std::max(1, sm_count() / ((9 * cin / 8 + 15) / 16)); }
 
@@ -1560,17 +1572,12 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
     for (int i = 0; i < count; ++i)
     {
         const WgradLayer& L = layers[i];
-        used += L.partials() * sizeof(float);
-        if (used > bytes) return fail(I360B_OUT_OF_MEMORY, "wgrad scratch too small");
-        const int kind = L.cout == 64                    ? (L.cin == 32 || L.cin == 64 ? WG_32_64 : -1)
-                         : L.cout == 16                  ? (L.cin == 32 ? WG_32_16 : -1)
-                         : L.cout != 32                  ? -1
-                         : L.cin == 16                   ? WG_16_32
-                         : L.cin == 32 || L.cin == 96    ? WG_32_32
-                                                         : -1;
+        const int kind = wgrad_kind(L.cin, L.cout);
         if (kind < 0 || L.cs % 32 || (L.cs > 0 && L.cin != 96))
             return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", L.cin, L.cout,
                         L.cs ? LD_CONCAT : LD_PLAIN);
+        used += L.partials() * sizeof(float);
+        if (used > bytes) return fail(I360B_OUT_OF_MEMORY, "wgrad scratch too small");
         for (int c = 0; c < L.cin; c += 32)
         {
             if (b.jobs == kWgJobs) return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: batch too large");
@@ -2282,10 +2289,10 @@ extern "C" int i360b_conv3x3_wgrad(const void* dX, const void* dU, int skipChann
     I360B_CUDA(cudaMemsetAsync(dErr, 0, sizeof(int), s), "error flag");
     int rc = I360B_SUCCESS;
     void* full = nullptr;
-    if ((L.cs > 0) != (cin == 96))
+    if (wgrad_kind(cin, cout) < 0 || (L.cs > 0) != (cin == 96))
         rc = fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", cin, cout,
                   L.cs > 0 ? LD_CONCAT : LD_PLAIN);
-    else if (cin == 96 && cout == 32 && L.cs % 32)
+    else if (L.cs % 32)
     {
         // a skip that is not whole 32-channel jobs: concatenate first
         rc = concatenate(L.x, L.u, L.cs, cin, n, h, w, &full, s);

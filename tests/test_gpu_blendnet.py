@@ -408,3 +408,15 @@ def test_gradients_repeat_at_every_ring_fill(backend, n, h, w):
         again, _ = net.gradients(jobs, n, w, h)
         assert np.array_equal(first, again), (k, int((first != again).sum()))
     net.close()
+
+
+@pytest.mark.parametrize("cin,cout,skip", [(0, 32, 0), (1, 32, 0), (-16, 32, 0), (16, 0, 0), (32, -64, 0), (256, 512, 0),
+                                           (96, 32, 0), (96, 64, 32), (64, 32, 32), (64, 32, 0), (16, 64, 0)])
+def test_wgrad_shapes_without_a_kernel_are_refused(backend, cin, cout, skip):
+    """NOT_SUPPORTED for every other shape, before any size is made of it."""
+    import torch
+    from image360_b200 import ComputeResult
+    from image360_b200 import blendnet as bn
+    t = torch.zeros(1 << 20, dtype=torch.float32, device="cuda")
+    p = t.data_ptr()
+    assert bn._bind().i360b_conv3x3_wgrad(p, p, skip, p, 1, 2, 256, cin, cout, p, None) == ComputeResult.NOT_SUPPORTED
