@@ -1083,17 +1083,18 @@ constexpr uint32_t kWgSmem = std::max({WgradShape<16, 32, false>::kSmem, WgradSh
                                        WgradShape<32, 64, false>::kSmem, WgradShape<32, 16, false>::kSmem,
                                        WgradShape<32, 32, true>::kSmem});
 
-// The concatenation of x (cs channels) and the nearest 2x upsample of u as one
-// tensor, for splits that no kernel above takes directly.
-__global__ void k_concat(const bf16* __restrict__ x, const bf16* __restrict__ u, int cs, int cin, int n, int h, int w,
-                         bf16* __restrict__ out)
+// Channels [c0, c0 + cn) of the concatenation of x (cs channels) and the
+// nearest 2x upsample of u (cin - cs) as a tensor, for splits that no kernel
+// above takes directly.
+__global__ void k_concat(const bf16* __restrict__ x, const bf16* __restrict__ u, int cs, int cin, int c0, int cn, int n,
+                         int h, int w, bf16* __restrict__ out)
 {
-    const int c8n = cin / 8, sc8 = cs / 8;
+    const int c8n = cn / 8, sc8 = cs / 8;
     const long long total = (long long)n * h * w * c8n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x)
     {
-        const int c8 = (int)(i % c8n);
+        const int c8 = c0 / 8 + (int)(i % c8n);
         const long long p = i / c8n;
         const int xx = (int)(p % w);
         const long long r = p / w;
@@ -1536,6 +1537,7 @@ struct WgradLayer
     const bf16* g;  // [n][h][w][cout]
     int n, h, w, cin, cout, coutReal;
     float *dw, *db;  // db may be null
+    const bf16* mixed = nullptr;  // [n][h][w][32]: the 32 channels from cs / 32 * 32 on, where cs % 32 != 0
 
     int slices() const
     {
@@ -1573,7 +1575,7 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
     {
         const WgradLayer& L = layers[i];
         const int kind = wgrad_kind(L.cin, L.cout);
-        if (kind < 0 || L.cs % 32 || (L.cs > 0 && L.cin != 96))
+        if (kind < 0 || (L.cs % 32 && !L.mixed) || (L.cs > 0 && L.cin != 96))
             return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", L.cin, L.cout,
                         L.cs ? LD_CONCAT : LD_PLAIN);
         used += L.partials() * sizeof(float);
@@ -1583,7 +1585,7 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
             if (b.jobs == kWgJobs) return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: batch too large");
             WgradJob& j = b.job[b.jobs++];
             const int cx = std::min(L.cin, 32);
-            const bool up = L.cs > 0 && c >= L.cs;
+            const bool up = L.cs > 0 && c >= L.cs, mixed = L.cs > c && L.cs < c + 32;
             j.kind = up ? WG_UP32_32 : kind;
             j.firstBlock = blocks;
             j.slices = L.slices();
@@ -1592,12 +1594,14 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
             j.w = L.w;
             j.cin = L.cin;
             j.c0 = c;
-            j.xc0 = up ? c - L.cs : c;
+            j.xc0 = up ? c - L.cs : mixed ? 0 : c;
             j.bias = L.db && c == 0;
             j.partial = part;
             if (up)
                 I360B_TRY(make_tile_map(&j.mapX, L.u, L.cin - L.cs, L.n, L.h / 2, L.w / 2, cx, kWgTW / 2, 2,
                                         swizzle_of(cx)));
+            else if (mixed)
+                I360B_TRY(make_parity_map(&j.mapX, L.mixed, cx, L.n, L.h, L.w, cx, kWgTW / 2, kWgRows + 2));
             else
                 I360B_TRY(make_parity_map(&j.mapX, L.x, L.cs > 0 ? L.cs : L.cin, L.n, L.h, L.w, cx, kWgTW / 2,
                                           kWgRows + 2));
@@ -1614,12 +1618,14 @@ int run_wgrad(const WgradLayer* layers, int count, int* error, void* scratch, si
     return check_launch("wgrad reduce kernel");
 }
 
-// The concatenation as a tensor of its own (dev_free it on `s`).
-int concatenate(const bf16* x, const bf16* u, int cs, int cin, int n, int h, int w, void** out, cudaStream_t s)
+// Channels [c0, c0 + cn) of the concatenation as a tensor of its own (dev_free
+// it on `s`).
+int concatenate(const bf16* x, const bf16* u, int cs, int cin, int c0, int cn, int n, int h, int w, void** out,
+                cudaStream_t s)
 {
-    const long long units = (long long)n * h * w * (cin / 8);
+    const long long units = (long long)n * h * w * (cn / 8);
     I360B_TRY(dev_alloc(out, (size_t)units * 16, s, "concatenated input"));
-    k_concat<<<elementwise_grid(units), 256, 0, s>>>(x, u, cs, cin, n, h, w, static_cast<bf16*>(*out));
+    k_concat<<<elementwise_grid(units), 256, 0, s>>>(x, u, cs, cin, c0, cn, n, h, w, static_cast<bf16*>(*out));
     const int rc = check_launch("concatenation kernel");
     if (rc != I360B_SUCCESS)
     {
@@ -1627,6 +1633,31 @@ int concatenate(const bf16* x, const bf16* u, int cs, int cin, int n, int h, int
         *out = nullptr;
     }
     return rc;
+}
+
+// A concatenated input of the forward convolution whose split is not the first
+// tile's 32 channels: concatenated first, a few images at a time, in scratch
+// of at most kConcatBytes (one image where that is more).
+constexpr size_t kConcatBytes = size_t(256) << 20;
+
+int conv_other_split(ConvArgs a, int cin, int npad, int ep, cudaStream_t s)
+{
+    const size_t px = (size_t)a.h * a.w;
+    const int images = a.n, per = (int)std::min<size_t>(images, std::max<size_t>(1, kConcatBytes / (px * cin * sizeof(bf16))));
+    const bf16 *x = a.x, *u = a.u;
+    bf16* out = static_cast<bf16*>(a.out);
+    for (int i = 0; i < images; i += per)
+    {
+        void* full = nullptr;
+        a.n = std::min(per, images - i);
+        I360B_TRY(concatenate(x + i * px * a.cs, u + i * (px / 4) * (cin - a.cs), a.cs, cin, 0, cin, a.n, a.h, a.w, &full, s));
+        a.x = static_cast<const bf16*>(full);
+        a.out = out + i * px * npad;
+        const int rc = dispatch_conv(cin, npad, LD_SPLIT, ep, a, s);
+        dev_free(full, s);
+        if (rc != I360B_SUCCESS) return rc;
+    }
+    return I360B_SUCCESS;
 }
 
 int check_window(int n, int w, int h)
@@ -2249,17 +2280,9 @@ extern "C" int i360b_conv3x3_forward(const void* dX, const void* dU, int skipCha
     a.error = dErr;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     I360B_CUDA(cudaMemsetAsync(dErr, 0, sizeof(int), s), "error flag");
-    int loader = skipChannels > 0 ? LD_CONCAT : LD_PLAIN;
-    void* full = nullptr;
-    if (loader == LD_CONCAT && cin == 96 && cout == 32 && epilogue == EP_RELU && skipChannels != 32)
-    {
-        // a skip other than the first tile's 32 channels: concatenate first
-        I360B_TRY(concatenate(a.x, a.u, skipChannels, cin, n, h, w, &full, s));
-        a.x = static_cast<const bf16*>(full);
-        loader = LD_SPLIT;
-    }
-    const int rc = dispatch_conv(cin, cout, loader, epilogue, a, s);
-    if (full) dev_free(full, s);
+    const bool otherSplit = skipChannels > 0 && skipChannels != 32 && cin == 96 && cout == 32 && epilogue == EP_RELU;
+    const int rc = otherSplit ? conv_other_split(a, cin, cout, epilogue, s)
+                              : dispatch_conv(cin, cout, skipChannels > 0 ? LD_CONCAT : LD_PLAIN, epilogue, a, s);
     if (rc != I360B_SUCCESS) return rc;
     int e = 0;
     I360B_CUDA(cudaMemcpyAsync(&e, dErr, sizeof(int), cudaMemcpyDeviceToHost, s), "error flag");
@@ -2281,26 +2304,24 @@ extern "C" int i360b_conv3x3_wgrad(const void* dX, const void* dU, int skipChann
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     static int* dErr = nullptr;
     if (!dErr) I360B_CUDA(cudaMalloc(&dErr, sizeof(int)), "error flag");
-    const size_t bytes = wgrad_scratch_bytes();
-    void* scratch = nullptr;
-    I360B_TRY(dev_alloc(&scratch, bytes, s, "wgrad scratch"));
     WgradLayer L{static_cast<const bf16*>(dX), static_cast<const bf16*>(dU), std::max(skipChannels, 0),
                  static_cast<const bf16*>(dGrad), n, h, w, cin, cout, cout, dGradW, nullptr};
-    I360B_CUDA(cudaMemsetAsync(dErr, 0, sizeof(int), s), "error flag");
-    int rc = I360B_SUCCESS;
-    void* full = nullptr;
     if (wgrad_kind(cin, cout) < 0 || (L.cs > 0) != (cin == 96))
-        rc = fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", cin, cout,
-                  L.cs > 0 ? LD_CONCAT : LD_PLAIN);
-    else if (L.cs % 32)
+        return fail(I360B_NOT_SUPPORTED, "conv3x3 wgrad: no kernel for cin=%d cout=%d loader=%d", cin, cout,
+                    L.cs > 0 ? LD_CONCAT : LD_PLAIN);
+    const size_t bytes = L.partials() * sizeof(float);
+    void *scratch = nullptr, *mixed = nullptr;
+    I360B_TRY(dev_alloc(&scratch, bytes, s, "wgrad scratch"));
+    int rc = I360B_SUCCESS;
+    if (cudaMemsetAsync(dErr, 0, sizeof(int), s) != cudaSuccess) rc = cuda_fail(cudaGetLastError(), "error flag");
+    if (rc == I360B_SUCCESS && L.cs % 32)
     {
-        // a skip that is not whole 32-channel jobs: concatenate first
-        rc = concatenate(L.x, L.u, L.cs, cin, n, h, w, &full, s);
-        L.x = static_cast<const bf16*>(full);
-        L.cs = 0;
+        // the 32-channel job that takes channels of both inputs
+        rc = concatenate(L.x, L.u, L.cs, cin, L.cs / 32 * 32, 32, n, h, w, &mixed, s);
+        L.mixed = static_cast<const bf16*>(mixed);
     }
     if (rc == I360B_SUCCESS) rc = run_wgrad(&L, 1, dErr, scratch, bytes, s);
-    if (full) dev_free(full, s);
+    if (mixed) dev_free(mixed, s);
     int e = 0;
     cudaMemcpyAsync(&e, dErr, sizeof(int), cudaMemcpyDeviceToHost, s);
     cudaStreamSynchronize(s);

@@ -173,13 +173,17 @@ enum
  * ([n][h][w][skipChannels]) and the nearest 2x upsample of dU
  * ([n][h/2][w/2][cin - skipChannels]).  dWeights is bf16 [cout][3][3][cin],
  * dBias fp32 [cout].  Supported (cin, cout): the layer shapes of the blend
- * network and of its backward pass.  Tensors 16-byte aligned. */
+ * network and of its backward pass.  Tensors 16-byte aligned.  With a skip
+ * other than the network's 32 channels the input is concatenated first, in
+ * scratch of h * w * 192 bytes an image for as many images at a time as 256 MB
+ * hold (one at least). */
 I360B_API int i360b_conv3x3_forward(const void* dX, const void* dU, int skipChannels, int n, int h, int w, int cin,
                                     int cout, const void* dWeights, const float* dBias, int epilogue,
                                     const void* dAct, void* dOut, void* stream);
 /* Weight gradient of that convolution: dGradW[cout][3][3][cin] (fp32,
  * overwritten) = sum over pixels of dGrad[p][co] * input[p + tap][ci];
- * width a multiple of 128. */
+ * width a multiple of 128.  Scratch: up to 5 MB of partial sums, and
+ * n * h * w * 64 bytes where skipChannels is not a multiple of 32. */
 I360B_API int i360b_conv3x3_wgrad(const void* dX, const void* dU, int skipChannels, const void* dGrad, int n, int h,
                                   int w, int cin, int cout, float* dGradW, void* stream);
 

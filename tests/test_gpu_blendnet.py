@@ -420,3 +420,66 @@ def test_wgrad_shapes_without_a_kernel_are_refused(backend, cin, cout, skip):
     t = torch.zeros(1 << 20, dtype=torch.float32, device="cuda")
     p = t.data_ptr()
     assert bn._bind().i360b_conv3x3_wgrad(p, p, skip, p, 1, 2, 256, cin, cout, p, None) == ComputeResult.NOT_SUPPORTED
+
+
+def _pool_high(call):
+    """The most bytes of the device's pool in use during a call."""
+    from cuda.bindings import driver as cu
+
+    def ok(r):
+        assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+        return r[1] if len(r) > 1 else None
+    pool = ok(cu.cuDeviceGetDefaultMemPool(ok(cu.cuDeviceGet(0))))
+    high = cu.CUmemPool_attribute.CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    now = int(ok(cu.cuMemPoolGetAttribute(pool, cu.CUmemPool_attribute.CU_MEMPOOL_ATTR_USED_MEM_CURRENT)))
+    ok(cu.cuMemPoolSetAttribute(pool, high, cu.cuuint64_t(0)))
+    call()
+    return int(ok(cu.cuMemPoolGetAttribute(pool, high))) - now
+
+
+@pytest.mark.parametrize("cin,cout,skip", [(16, 32, 0), (64, 64, 0), (96, 32, 32), (96, 32, 8), (96, 32, 72)])
+def test_wgrad_scratch_is_one_layers(backend, cin, cout, skip):
+    """Partial sums of the layer's own slices (one per SM and 128 rows of taps
+    and channels at most), and 32 channels of the concatenation where a job
+    takes channels of both inputs.  The sums themselves: as with the whole
+    concatenation, in fp64, 1e-4 of the largest as in the tests above."""
+    import torch
+    import torch.nn.functional as F
+    from image360_b200 import blendnet as bn
+    n, h, w = 6, 64, 256
+    rng = np.random.default_rng(cin + skip)
+    x = _bf((n, h, w, skip or cin), rng)
+    u = _bf((n, h // 2, w // 2, cin - skip), rng) if skip else None
+    full = torch.cat([x, u.repeat_interleave(2, 1).repeat_interleave(2, 2)], -1) if skip else x
+    g = _bf((n, h, w, cout), rng)
+    out = torch.zeros((cout, 3, 3, cin), dtype=torch.float32, device="cuda")
+    bn.conv3x3_wgrad(x, g, out, u=u, skip=skip)
+    used = _pool_high(lambda: bn.conv3x3_wgrad(x, g, out, u=u, skip=skip))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    slices = sms // ((9 * cin // 8 + 15) // 16)
+    limit = slices * (9 * cin * cout + cout) * 4 + (n * h * w * 64 if skip % 32 else 0)
+    assert used <= limit + 4096, (used, limit)
+    xp = F.pad(full.double(), (0, 0, 1, 1, 1, 1))
+    ref = torch.stack([torch.stack([torch.einsum("nhwo,nhwi->oi", g.double(), xp[:, ky:ky + h, kx:kx + w])
+                                    for kx in range(3)], 1) for ky in range(3)], 1)
+    assert float((out.double() - ref).abs().max()) <= 1e-4 * float(ref.abs().max())
+
+
+def test_forward_with_another_split_bounds_its_scratch(backend):
+    """A batch whose concatenation would take more than 256 MB is taken some
+    images at a time: the bits of one image at a time."""
+    import torch
+    from image360_b200 import blendnet as bn
+    n, h, w, skip = 25, 256, 256, 8
+    rng = np.random.default_rng(5)
+    x = _bf((1, h, w, skip), rng).repeat(n, 1, 1, 1) * torch.arange(1, n + 1, device="cuda").bfloat16().view(n, 1, 1, 1)
+    u = _bf((1, h // 2, w // 2, 96 - skip), rng).repeat(n, 1, 1, 1)
+    W = _bf((32, 3, 3, 96), rng, 1.0 / np.sqrt(864))
+    b = _t(rng.standard_normal(32).astype(np.float32) * 0.1)
+    out = torch.zeros((n, h, w, 32), dtype=torch.bfloat16, device="cuda")
+    one = torch.zeros((1, h, w, 32), dtype=torch.bfloat16, device="cuda")
+    used = _pool_high(lambda: bn.conv3x3_forward(x, W, b, 32, 0, out, u=u, skip=skip))
+    assert n * h * w * 192 > 256 << 20 and used <= 256 << 20
+    for i in (0, 20, 21, 24):
+        bn.conv3x3_forward(x[i:i + 1], W, b, 32, 0, one, u=u[i:i + 1], skip=skip)
+        assert torch.equal(one[0], out[i]), i
