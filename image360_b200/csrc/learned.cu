@@ -1776,8 +1776,6 @@ struct BlendNet
             bias[l] = biasPacked + ob;
             ob += pad16(kNet[l].cout);
         }
-        wgBytes = wgrad_scratch_bytes();
-        I360B_CUDA(cudaMalloc(&wgScratch, wgBytes), "blendnet wgrad scratch");
         I360B_CUDA(cudaMalloc(&dLoss, sizeof(double)), "blendnet loss");
         I360B_CUDA(cudaMalloc(&dError, sizeof(int)), "blendnet error flag");
         I360B_CUDA(cudaMemset(dError, 0, sizeof(int)), "blendnet error flag");
@@ -1821,13 +1819,18 @@ struct BlendNet
         return check_launch("weight pack kernel");
     }
 
-    // Activation buffers for n windows of w x h; the backward buffers only
-    // when training.
+    // Activation buffers for n windows of w x h; the backward buffers and the
+    // weight gradients' scratch (20 MB) only when training.
     int reserve(int n, int w, int h, bool training)
     {
         const size_t pix = (size_t)n * w * h;
         if (pix <= capPix && (!training || capTraining)) return I360B_SUCCESS;
         cudaDeviceSynchronize();
+        if (training && !wgScratch)
+        {
+            wgBytes = wgrad_scratch_bytes();
+            I360B_CUDA(cudaMalloc(&wgScratch, wgBytes), "blendnet wgrad scratch");
+        }
         cudaFree(act);
         act = nullptr;
         capPix = 0;

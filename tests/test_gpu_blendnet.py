@@ -483,3 +483,25 @@ def test_forward_with_another_split_bounds_its_scratch(backend):
     for i in (0, 20, 21, 24):
         bn.conv3x3_forward(x[i:i + 1], W, b, 32, 0, one, u=u[i:i + 1], skip=skip)
         assert torch.equal(one[0], out[i]), i
+
+
+def test_inference_holds_no_training_scratch(backend):
+    """A network that only infers takes its parameters, their packed forms and
+    the activations (432 bytes a pixel at most): not the 20 MB of the weight
+    gradients' partial sums.  Nets are made twice, so that what the process
+    allocates once is not counted."""
+    import torch
+    from image360_b200 import blendnet as bn
+    n, h, w = 4, 64, 256
+    layers = _layers(2, n, h, w)
+    dl, _, out, jobs = _device_batch(layers)
+    held = []
+    for _ in range(2):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        net = bn.BlendNet(seed=1)
+        net.infer(jobs, n, w, h)
+        torch.cuda.synchronize()
+        held.append(before - torch.cuda.mem_get_info()[0])
+        net.close()
+    assert held[1] <= n * h * w * 432 + 8 * (2 << 20), held[1]
