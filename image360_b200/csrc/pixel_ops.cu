@@ -114,8 +114,8 @@ __device__ void demosaic_border(const unsigned short* __restrict__ cfa, int x, i
     demosaic_matrix(P, rgb[0], rgb[1], rgb[2], out + ((size_t)y * w + x) * 3);
 }
 
-// Any filter word, size and alignment: a thread per 2x2 quad, a tile of the
-// levelled values in shared memory.
+// Any filter word, size and alignment, and small frames: a thread per 2x2
+// quad, a tile of the levelled values in shared memory.
 __global__ void __launch_bounds__(256) k_demosaic(const unsigned short* __restrict__ cfa, int w, int h,
                                                   DemosaicParams P, unsigned short* __restrict__ out)
 {
@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(256) k_demosaic(const unsigned short* __restri
 // arithmetic, took 117 us.
 // ---------------------------------------------------------------------------
 constexpr int kDmRows = 12, kDmCols = 120, kDmWarps = 4;
+constexpr int kDmStripPixels = 4800;  // pixels per SM from which strips are taken
 
 struct BayerParams
 {
@@ -790,9 +791,13 @@ int launch_demosaic(const unsigned short* cfa, int w, int h, unsigned short blac
     }
     // k_demosaic_bayer: a standard layout, rows of whole 8-byte words in and
     // out, multipliers that level to no negative or NaN and a matrix whose
-    // products stay finite.
+    // products stay finite, and a frame large enough: a strip's 24 rows are a
+    // chain of 8.2 us however few strips there are.  500 x 400 takes 5.5 us in
+    // tiles and 8.2 in strips, 800 x 600 6.8 and 8.4, 1000 x 700 7.8 and 8.3,
+    // 900 x 800 8.7 and 8.4, 1200 x 900 10.0 and 8.5.
+    const bool large = (long long)w * h >= (long long)kDmStripPixels * sm_count();
     auto in_range = [](float v, float lo) { return v >= lo && v <= 1e30f; };
-    bool fast = P.std2x2 && w % 4 == 0 && ((reinterpret_cast<uintptr_t>(cfa) | reinterpret_cast<uintptr_t>(out)) & 7) == 0;
+    bool fast = large && P.std2x2 && w % 4 == 0 && ((reinterpret_cast<uintptr_t>(cfa) | reinterpret_cast<uintptr_t>(out)) & 7) == 0;
     for (float m : P.camMul) fast = fast && in_range(m, 0.0f);
     for (float m : P.rgbCam) fast = fast && in_range(m, -1e30f);
     if (fast)

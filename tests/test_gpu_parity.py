@@ -366,3 +366,24 @@ def test_blend_coverage_words(backend, oracle_c, w):
     out = np.zeros((h, w, 3), np.uint16)
     assert backend.blend_chunk_contributors(bufs, w, h, out, 4) == ComputeResult.SUCCESS, backend.get_last_error()
     assert np.array_equal(out, oracle_c.blend(bufs, 4))
+
+
+@pytest.mark.parametrize("filters", [0x94949494, 0x61616161, 0x16161616, 0x49494949])
+@pytest.mark.parametrize("w,h", [(1200, 720), (1204, 721), (1196, 743), (364, 2400), (116, 7105), (35520, 25), (4, 200000),
+                                 (1000, 710), (1000, 711)])
+def test_demosaic_large_strip_edges(backend, oracle_c, filters, w, h):
+    """Frames large enough for the strips of 120 columns and 24 rows, at their
+    edges: whole and partial strips either way, one column of strips, and
+    sizes on either side of the rule that chooses them.  Equal to the oracle."""
+    import torch
+    rng = np.random.default_rng(w * 100 + h)
+    cfa = rng.integers(0, 65536, (h, w)).astype(np.uint16)
+    cfa[rng.random((h, w)) < 0.2] = 65535
+    cm = np.array([2.03, 1.0, 1.61, 0.97], np.float32)
+    rc = np.array([1.7, -0.5, -0.2, 3.5, -0.3, 1.6, -0.35, -40.0, 0.05, -0.6, 1.55, 0.25], np.float32)
+    d_in = torch.from_numpy(cfa.view(np.int16)).cuda()
+    for black in (0, 513):
+        d_out = torch.zeros((h, w, 3), dtype=torch.int16, device="cuda")
+        assert backend.launch_demosaic(d_in.data_ptr(), w, h, black, cm, rc, filters, d_out.data_ptr()) == 0
+        torch.cuda.synchronize()
+        assert np.array_equal(d_out.cpu().numpy().view(np.uint16), oracle_c.demosaic(cfa, black, cm, rc, filters))
