@@ -435,12 +435,53 @@ __global__ void __launch_bounds__(32 * kDmWarps, 5) k_demosaic_bayer(const unsig
 // is paired).  Bound by instruction issue and tap latency: a 2048 x 2048 tile
 // 22.9 us, 26.9 us with scalar arithmetic and 2-byte taps.
 // ---------------------------------------------------------------------------
+constexpr int kWarpPairPixels = 1700;  // destination pixels per SM from which a lane makes two
+
 struct WarpParams
 {
     float H[9];
     float gain;
     int applyGain;
 };
+
+// Small tiles: a pixel per lane, so that twice the threads share the latency
+// of the taps.
+__global__ void __launch_bounds__(256) k_warp_small(const unsigned short* __restrict__ src, int sw, int sh,
+                                                    unsigned short* __restrict__ dst, int dw, int dh, int offX,
+                                                    int offY, WarpParams P)
+{
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    if (x >= dw || y >= dh) return;
+    const float dX = (float)(x + offX), dY = (float)(y + offY);
+    float sx = fadd(fadd(fmul(P.H[0], dX), fmul(P.H[1], dY)), P.H[2]);
+    float sy = fadd(fadd(fmul(P.H[3], dX), fmul(P.H[4], dY)), P.H[5]);
+    const float sw1 = fadd(fadd(fmul(P.H[6], dX), fmul(P.H[7], dY)), P.H[8]);
+    unsigned short o[3] = {0, 0, 0};
+    sx = fdiv(sx, sw1);
+    sy = fdiv(sy, sw1);
+    // (NaN and positions out of range are invalid, as in warp_pair23)
+    if (!(fabsf(sw1) < 1e-10f) && sx >= 0.0f && sx < (float)(sw - 1) && sy >= 0.0f && sy < (float)(sh - 1))
+    {
+        const int x0 = (int)f2u_floor(sx), y0 = (int)f2u_floor(sy);
+        const float fx = fsub(sx, u2f((uint32_t)x0)), fy = fsub(sy, u2f((uint32_t)y0));
+        const float gx = fsub(1.0f, fx), gy = fsub(1.0f, fy);
+        const float w00 = fmul(gx, gy), w10 = fmul(fx, gy), w01 = fmul(gx, fy), w11 = fmul(fx, fy);
+        const unsigned short* r0 = src + ((size_t)y0 * sw + x0) * 3;
+        const unsigned short* r1 = r0 + (size_t)sw * 3;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+            const float v = fadd(fadd(fadd(fmul(w00, u2f(__ldg(r0 + c))), fmul(w10, u2f(__ldg(r0 + 3 + c)))),
+                                      fmul(w01, u2f(__ldg(r1 + c)))),
+                                 fmul(w11, u2f(__ldg(r1 + 3 + c))));
+            o[c] = P.applyGain ? clamp_trunc_u16(fmul(clamp_floor_u16f(v), P.gain)) : clamp_trunc_u16(v);
+        }
+    }
+    unsigned short* d = dst + ((size_t)y * dw + x) * 3;
+    d[0] = o[0];
+    d[1] = o[1];
+    d[2] = o[2];
+}
 
 template <bool AFFINE>
 __global__ void __launch_bounds__(256) k_warp(WarpSource src, unsigned short* __restrict__ dst, int dw, int dh,
@@ -838,8 +879,18 @@ int launch_warp(const unsigned short* src, int sw, int sh, unsigned short* dst, 
     for (int i = 0; i < 9; ++i) P.H[i] = H[i];
     P.gain = gain;
     P.applyGain = gain_is_identity(gain) ? 0 : 1;
+    const dim3 block(32, 8);
+    // A pixel per lane while the tile has too few for two to fill the SMs:
+    // 128 x 128 1.9 us against 2.5 for pairs, 256 x 256 2.1 and 2.5, 400 x 400
+    // 2.7 and 2.8, 480 x 480 3.0 and 3.1; 512 x 512 3.2 for either, 1000 x 1000
+    // 7.0 and 6.2.
+    if ((long long)dw * dh < (long long)kWarpPairPixels * sm_count())
+    {
+        k_warp_small<<<dim3((dw + 31) / 32, (dh + 7) / 8), block, 0, s>>>(src, sw, sh, dst, dw, dh, offX, offY, P);
+        return check_launch("warp kernel");
+    }
     const WarpSource S = warp_source(src, sw, sh);
-    const dim3 grid((dw + 63) / 64, (dh + 7) / 8), block(32, 8);
+    const dim3 grid((dw + 63) / 64, (dh + 7) / 8);
     if (homography_affine(H)) k_warp<true><<<grid, block, 0, s>>>(S, dst, dw, dh, offX, offY, P);
     else k_warp<false><<<grid, block, 0, s>>>(S, dst, dw, dh, offX, offY, P);
     return check_launch("warp kernel");

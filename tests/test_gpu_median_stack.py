@@ -178,3 +178,32 @@ def test_warp_taps_at_every_phase(backend, oracle_c, sw, sh, dw, dh, shift, proj
         assert backend.launch_warp_median([p, p], sw, sh, np.stack([H, H]), out.data_ptr(), dw, dh, *off) == 0
         torch.cuda.synchronize()
         assert np.array_equal(_host(out), ref)
+
+
+@pytest.mark.parametrize("sw,sh,dw,dh,shift,proj", [(301, 200, 502, 501, 0, False), (301, 200, 501, 502, 1, True),
+                                                    (700, 511, 1025, 249, 0, True), (700, 511, 63, 4001, 1, False),
+                                                    (2, 2, 520, 490, 0, False), (333, 77, 500, 503, 1, True),
+                                                    (333, 77, 503, 500, 0, False)])
+def test_warp_of_large_tiles_at_every_phase(backend, oracle_c, sw, sh, dw, dh, shift, proj):
+    """Tiles around and above the size from which a lane makes two pixels, whose
+    taps are words at both phases: widths around the 64-pixel segment, affine
+    and projective homographies, gains.  Full-range values.  Exact."""
+    import torch
+    rng = np.random.default_rng(sw * 100 + dw)
+    src = rng.integers(0, 65536, (sh, sw, 3), dtype=np.uint16)
+    src[0, 0] = 65535
+    src[-1, -1] = 65535
+    buf = torch.zeros(src.size + 1, dtype=torch.int16, device="cuda")
+    buf[shift:shift + src.size] = _dev(src).reshape(-1)
+    H = np.array([[0.93, 0.11, -1.25], [-0.08, 0.97, 0.75], [0, 0, 1]], np.float32)
+    if proj:
+        H[2] = [3e-4, -2e-4, 1.0001]
+    for off in ((0, 0), (-3, 2)):
+        ref = oracle_c.warp(src, dw, dh, H, *off)
+        for gain in (1.0, 1.37, 0.0, -1.0):
+            out = torch.full((dh, dw, 3), 9, dtype=torch.int16, device="cuda")
+            assert backend.launch_warp(buf.data_ptr() + 2 * shift, sw, sh, out.data_ptr(), dw, dh, H, *off,
+                                       gain=gain) == 0
+            torch.cuda.synchronize()
+            exp = ref if gain == 1.0 else oracle_c.gain(ref.copy(), gain).reshape(ref.shape)
+            assert np.array_equal(_host(out), exp), (off, gain)
