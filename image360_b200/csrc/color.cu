@@ -30,7 +30,8 @@
 // Encoded values are needed as 16-bit codes only, and the encode is monotone:
 // the transfer estimates the code from a fast power, to within one, and
 // compares the value with the smallest float that encodes to the next code, a
-// table built on the device once per process from the exact encode.
+// table built on the device once per process from the exact encode (every float
+// against the exact encode: tests/color_encode_check.cu).
 // Whole chunks are processed two pixels at a time in paired FP32 instructions
 // (common.cuh), each half rounded as the scalar code rounds it.
 // The reference's libm powf/cbrtf are within about one ulp of those values, so

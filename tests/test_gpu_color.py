@@ -176,3 +176,22 @@ def test_transfer_pairs_equal_single_pixels(backend, spread):
         torch.cuda.synchronize()
         got.append(view.cpu().numpy())
     assert np.array_equal(got[0], got[1])
+
+
+def test_table_encode_equals_the_exact_encode(tmp_path):
+    """All 2^32 floats give the code of the exact encode, and all 65535 steps
+    of the table are the exact encode's (tests/color_encode_check.cu)."""
+    import os
+    import shutil
+    import subprocess
+    from image360_b200 import build
+    nvcc = shutil.which(build.nvcc())
+    if nvcc is None:
+        pytest.skip("no CUDA compiler")
+    exe = str(tmp_path / "color_encode_check")
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "color_encode_check.cu")
+    subprocess.run([nvcc, *build.ARCH, "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-fmad=false", "-o", exe, src],
+                   check=True, timeout=300)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    print(r.stdout)
+    assert r.returncode == 0, r.stdout
