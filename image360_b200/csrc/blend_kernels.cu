@@ -2019,34 +2019,25 @@ __device__ __forceinline__ float4 nd_at(const float4* nd, size_t q, int half)
     return make_float4(a.x * 256.0f, a.y * 256.0f, b.x * 256.0f, b.y);
 }
 
-// The levels gmin and above of a contributor's pyramid hold, once the band
-// blend of their level has run, the hole-filled Gaussian G = num * (1/den) in
-// place of num: the blend of the level below, the level-0 output (level 1)
-// and the fused fine kernel (level 2) read Up(G) taps, each value about
-// sixteen times, and the reciprocal is then computed once per value instead
-// of once per tap.  The stored G is the value gauss_of would compute, so the
-// taps are bit-identical in the exact mode (with FP16 storage G / 256 is
-// stored as FP16, like num / 256 before).  gmin is 1 with every level
-// materialised (the level-1 blend runs before the output) and 2 with the
-// fused levels (level 1 has no blend of its own).  In the exact mode G is
-// stored only where the contributor's weight at that level is non-zero:
-// every reader takes Up(G) taps only for a pixel of non-zero weight one level
-// below (a blend term, or an owned level-0 pixel), each such tap has that
-// pixel in its 5-tap footprint (align-corners: |x - 2 x0| <= 2), and the
-// weight there is then a sum containing a positive product - non-zero.  A
-// tap elsewhere only enters a term of weight zero, which is +-0 for any
-// finite value.  (FP16 weights can round to zero, so that mode stores G
-// wherever the blend passes.)
-__device__ __forceinline__ bool g_stored(int level, int gmin) { return level >= gmin; }
-
-__device__ __forceinline__ float3 g_at(const float4* nd, size_t q, int level, int gmin, int half)
+// Every level that is blended holds, once the band blend of that level has
+// run, the hole-filled Gaussian G = num * (1/den) in place of num: the blend
+// of the level below, the level-0 output (level 1, where that is blended) and
+// the fused fine kernel (level 2) read Up(G) taps, each value about sixteen
+// times, and the reciprocal is then computed once per value instead of once
+// per tap.  The stored G is the value gauss_of computes, so the taps are
+// bit-identical in the exact mode (with FP16 storage G / 256 is stored as
+// FP16, like num / 256 before).  In the exact mode G is stored only where the
+// contributor's weight at that level is non-zero: every reader takes Up(G)
+// taps only for a pixel of non-zero weight one level below (a blend term, or
+// an owned level-0 pixel), each such tap has that pixel in its 5-tap footprint
+// (align-corners: |x - 2 x0| <= 2), and the weight there is then a sum
+// containing a positive product - non-zero.  A tap elsewhere only enters a
+// term of weight zero, which is +-0 for any finite value.  (FP16 weights can
+// round to zero, so that mode stores G wherever the blend passes.)
+__device__ __forceinline__ float3 g_at(const float4* nd, size_t q, int half)
 {
-    if (g_stored(level, gmin))
-    {
-        const float4 v = nd_at(nd, q, half);
-        return make_float3(v.x, v.y, v.z);
-    }
-    return gauss_of(nd_at(nd, q, half));
+    const float4 v = nd_at(nd, q, half);
+    return make_float3(v.x, v.y, v.z);
 }
 
 __device__ __forceinline__ void g_store(const float4* nd, size_t q, float3 g, int half)
@@ -2372,8 +2363,7 @@ __global__ void __launch_bounds__(256, 4) k_down0s(BlendArgs a, const Unit* __re
 }
 
 // One pixel of a blended band (the general path).
-__device__ __noinline__ void blend_pixel(const TileDev& T, const ItemCache& C, int level, int K, long long pl, int half,
-                                        int gmin)
+__device__ __noinline__ void blend_pixel(const TileDev& T, const ItemCache& C, int level, int K, long long pl, int half)
 {
     const int lw = T.lw[level];
     const bool top = level == T.bands - 1;
@@ -2388,18 +2378,17 @@ __device__ __noinline__ void blend_pixel(const TileDev& T, const ItemCache& C, i
         const int4 B = C.box[k];
         if (x < B.x || x > B.z || y < B.y || y > B.w) continue;  // weight 0: the term is +-0
         float wv = wg_at(C.wg[k], p, half);
-        const bool store = g_stored(level, gmin) && (half || wv != 0.0f);
-        if (wv == 0.0f && !store) continue;  // the term is +-0 and no reader needs G here
+        if (wv == 0.0f && !half) continue;  // the term is +-0 and no reader needs G here
         float3 g = gauss_of(nd_at(C.nd[k], p, half));
-        if (store) g_store(C.nd[k], p, g, half);
+        g_store(C.nd[k], p, g, half);
         if (wv == 0.0f) continue;
         if (!top)
         {
             const size_t up = T.loff[level + 1];
-            float3 a00 = g_at(C.nd[k], up + (size_t)c.y0 * uw + c.x0, level + 1, gmin, half);
-            float3 a10 = g_at(C.nd[k], up + (size_t)c.y0 * uw + c.x1, level + 1, gmin, half);
-            float3 a01 = g_at(C.nd[k], up + (size_t)c.y1 * uw + c.x0, level + 1, gmin, half);
-            float3 a11 = g_at(C.nd[k], up + (size_t)c.y1 * uw + c.x1, level + 1, gmin, half);
+            float3 a00 = g_at(C.nd[k], up + (size_t)c.y0 * uw + c.x0, half);
+            float3 a10 = g_at(C.nd[k], up + (size_t)c.y0 * uw + c.x1, half);
+            float3 a01 = g_at(C.nd[k], up + (size_t)c.y1 * uw + c.x0, half);
+            float3 a11 = g_at(C.nd[k], up + (size_t)c.y1 * uw + c.x1, half);
             g.x = fsub(g.x, up_mix(a00.x, a10.x, a01.x, a11.x, c.wx, c.wy));
             g.y = fsub(g.y, up_mix(a00.y, a10.y, a01.y, a11.y, c.wx, c.wy));
             g.z = fsub(g.z, up_mix(a00.z, a10.z, a01.z, a11.z, c.wx, c.wy));
@@ -2420,7 +2409,7 @@ __device__ __noinline__ void blend_pixel(const TileDev& T, const ItemCache& C, i
 // texels and reciprocals computed once per contributor; every pixel's sum
 // still runs over the contributors in index order with its own weights.
 __device__ __forceinline__ void blend_quad(const TileDev& T, const ItemCache& C, int level, int K, long long pl,
-                                           int y, int x, int half, int gmin)
+                                           int y, int x, int half)
 {
     const int uw = T.lw[level + 1], uh = T.lh[level + 1];
     int x0[4];
@@ -2441,7 +2430,7 @@ __device__ __forceinline__ void blend_quad(const TileDev& T, const ItemCache& C,
     float acc[4][3];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = acc[i][2] = 0.0f;
-    const bool storeAll = g_stored(level, gmin) && half;  // FP16: G stored wherever the blend passes
+    const bool storeAll = half;  // FP16: G stored wherever the blend passes
     for (int k = 0; k < K; ++k)
     {
         const int4 B = C.box[k];
@@ -2453,11 +2442,11 @@ __device__ __forceinline__ void blend_quad(const TileDev& T, const ItemCache& C,
         const float4* nd = C.nd[k];
         const size_t up = T.loff[level + 1];
         int cur = x0[0];
-        float3 L0 = g_at(nd, up + (size_t)y0 * uw + cur, level + 1, gmin, half),
-               L1 = g_at(nd, up + (size_t)y1 * uw + cur, level + 1, gmin, half);
+        float3 L0 = g_at(nd, up + (size_t)y0 * uw + cur, half),
+               L1 = g_at(nd, up + (size_t)y1 * uw + cur, half);
         int nx = min(cur + 1, uw - 1);
-        float3 R0 = g_at(nd, up + (size_t)y0 * uw + nx, level + 1, gmin, half),
-               R1 = g_at(nd, up + (size_t)y1 * uw + nx, level + 1, gmin, half);
+        float3 R0 = g_at(nd, up + (size_t)y0 * uw + nx, half),
+               R1 = g_at(nd, up + (size_t)y1 * uw + nx, half);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
         {
@@ -2467,12 +2456,12 @@ __device__ __forceinline__ void blend_quad(const TileDev& T, const ItemCache& C,
                 L0 = R0;
                 L1 = R1;
                 nx = min(cur + 1, uw - 1);
-                R0 = g_at(nd, up + (size_t)y0 * uw + nx, level + 1, gmin, half);
-                R1 = g_at(nd, up + (size_t)y1 * uw + nx, level + 1, gmin, half);
+                R0 = g_at(nd, up + (size_t)y0 * uw + nx, half);
+                R1 = g_at(nd, up + (size_t)y1 * uw + nx, half);
             }
             if (wv[i] == 0.0f && !storeAll) continue;
             float3 g = gauss_of(nd_at(nd, p + i, half));
-            if (g_stored(level, gmin)) g_store(nd, p + i, g, half);
+            g_store(nd, p + i, g, half);
             if (wv[i] == 0.0f) continue;
             g.x = fsub(g.x, up_mix(L0.x, R0.x, L1.x, R1.x, wx[i], wy));
             g.y = fsub(g.y, up_mix(L0.y, R0.y, L1.y, R1.y, wx[i], wy));
@@ -2509,13 +2498,9 @@ __device__ __forceinline__ void blend_quad(const TileDev& T, const ItemCache& C,
 // Gaussian is finite), and adding +-0 to a sum that started at +0 changes
 // nothing, so skipping contributors outside their weight support (the whole
 // pyramid of one that owns no pixel) equals the reference's full sum.
-// HALF: the pyramids' storage.  Every level that is blended here, and the one
-// above it, holds G (BlendArgs::gmin is at most the lowest level blended), so
-// the taps need no reciprocals: kStored.  With both known at compile time the
-// band blend of a 24-frame panorama takes 1.51 instead of 1.60 ms and its
-// level-0 output 2.42 instead of 2.86.
-constexpr int kStored = 0;  // as gmin: every level stored
-
+// HALF: the pyramids' storage.  Known at compile time, and with the taps read
+// without a reciprocal (see g_at), the band blend of a 24-frame panorama takes
+// 1.51 instead of 1.60 ms and its level-0 output 2.42 instead of 2.86.
 template <bool HALF>
 __global__ void __launch_bounds__(256, 3) k_blend_level(BlendArgs a, const Unit* __restrict__ units, int level)
 {
@@ -2539,10 +2524,10 @@ __global__ void __launch_bounds__(256, 3) k_blend_level(BlendArgs a, const Unit*
         const int cnt = min(4, lw - x);
         if (!top && cnt == 4)
         {
-            blend_quad(T, C, level, K, pl, y, x, HALF, kStored);
+            blend_quad(T, C, level, K, pl, y, x, HALF);
             continue;
         }
-        for (int i = 0; i < cnt; ++i) blend_pixel(T, C, level, K, pl + i, HALF, kStored);
+        for (int i = 0; i < cnt; ++i) blend_pixel(T, C, level, K, pl + i, HALF);
     }
 }
 
@@ -2659,7 +2644,7 @@ __device__ __forceinline__ void final_store(unsigned short* o, const float* r)
 
 // One output pixel (the general path).
 __device__ __noinline__ void final_pixel(const TileDev& T, const ItemCache& C, const float* rc, int uw, int uh,
-                                            long long p, int own, int half, int gmin)
+                                            long long p, int own, int half)
 {
     unsigned short* o = T.out + p * 3;
     if (own < 0)
@@ -2676,10 +2661,10 @@ __device__ __noinline__ void final_pixel(const TileDev& T, const ItemCache& C, c
         const UpCoef c = up_coef_s(T.usx[0], T.usy[0], uw, uh, x, y);
         const float4* nd = C.nd[own];
         const size_t l1 = T.loff[1];
-        const float3 a00 = g_at(nd, l1 + (size_t)c.y0 * uw + c.x0, 1, gmin, half);
-        const float3 a10 = g_at(nd, l1 + (size_t)c.y0 * uw + c.x1, 1, gmin, half);
-        const float3 a01 = g_at(nd, l1 + (size_t)c.y1 * uw + c.x0, 1, gmin, half);
-        const float3 a11 = g_at(nd, l1 + (size_t)c.y1 * uw + c.x1, 1, gmin, half);
+        const float3 a00 = g_at(nd, l1 + (size_t)c.y0 * uw + c.x0, half);
+        const float3 a10 = g_at(nd, l1 + (size_t)c.y0 * uw + c.x1, half);
+        const float3 a01 = g_at(nd, l1 + (size_t)c.y1 * uw + c.x0, half);
+        const float3 a11 = g_at(nd, l1 + (size_t)c.y1 * uw + c.x1, half);
         const float lap[3] = {fsub(r[0], up_mix(a00.x, a10.x, a01.x, a11.x, c.wx, c.wy)),
                               fsub(r[1], up_mix(a00.y, a10.y, a01.y, a11.y, c.wx, c.wy)),
                               fsub(r[2], up_mix(a00.z, a10.z, a01.z, a11.z, c.wx, c.wy))};
@@ -2704,12 +2689,12 @@ struct TapColumn
 };
 
 __device__ __forceinline__ TapColumn tap_column(const float4* nd, size_t l1, const float* rc, int uw, int y0, int y1,
-                                                int col, int half, int gmin)
+                                                int col, int half)
 {
     const size_t q0 = (size_t)y0 * uw + col, q1 = (size_t)y1 * uw + col;
     TapColumn t;
-    t.g0 = g_at(nd, l1 + q0, 1, gmin, half);
-    t.g1 = g_at(nd, l1 + q1, 1, gmin, half);
+    t.g0 = g_at(nd, l1 + q0, half);
+    t.g1 = g_at(nd, l1 + q1, half);
     t.u0 = make_float3(__ldg(rc + q0 * 3), __ldg(rc + q0 * 3 + 1), __ldg(rc + q0 * 3 + 2));
     t.u1 = make_float3(__ldg(rc + q1 * 3), __ldg(rc + q1 * 3 + 1), __ldg(rc + q1 * 3 + 2));
     return t;
@@ -2722,15 +2707,15 @@ __device__ __forceinline__ TapColumn tap_column(const float4* nd, size_t l1, con
 // column's texels and reciprocals computed once; every pixel still combines
 // its own four taps with its own weights in the reference's order.
 __device__ __forceinline__ void final_quad(const TileDev& T, const ItemCache& C, const float* rc, int uw, int uh,
-                                           long long p, int y, int x, int own, int half, int gmin)
+                                           long long p, int y, int x, int own, int half)
 {
     const float4* g1 = C.nd[own];
     const size_t l1 = T.loff[1];
     const float sx = T.usx[0];
     UpCoef c = up_coef_s(sx, T.usy[0], uw, uh, x, y);
     int cur = c.x0;
-    TapColumn L = tap_column(g1, l1, rc, uw, c.y0, c.y1, cur, half, gmin);
-    TapColumn R = tap_column(g1, l1, rc, uw, c.y0, c.y1, c.x1, half, gmin);
+    TapColumn L = tap_column(g1, l1, rc, uw, c.y0, c.y1, cur, half);
+    TapColumn R = tap_column(g1, l1, rc, uw, c.y0, c.y1, c.x1, half);
     const unsigned short* px = C.img[own] + p * 3;
     // the quad's 12 source values: three 8-byte loads when aligned
     uint32_t pw[6];
@@ -2765,7 +2750,7 @@ __device__ __forceinline__ void final_quad(const TileDev& T, const ItemCache& C,
             {
                 cur = x0;
                 L = R;
-                R = tap_column(g1, l1, rc, uw, c.y0, c.y1, min(x0 + 1, uw - 1), half, gmin);
+                R = tap_column(g1, l1, rc, uw, c.y0, c.y1, min(x0 + 1, uw - 1), half);
             }
         }
         float r[3];
@@ -2838,12 +2823,12 @@ __global__ void __launch_bounds__(256) k_final0(BlendArgs a, const Unit* __restr
         }
         if (cnt == 4 && T.bands > 1 && own[0] >= 0 && own[1] == own[0] && own[2] == own[0] && own[3] == own[0])
         {
-            final_quad(T, C, rc, uw, uh, p, y, x, own[0], HALF, kStored);
+            final_quad(T, C, rc, uw, uh, p, y, x, own[0], HALF);
             continue;
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            if (i < cnt) final_pixel(T, C, rc, uw, uh, p + i, own[i], HALF, kStored);
+            if (i < cnt) final_pixel(T, C, rc, uw, uh, p + i, own[i], HALF);
     }
 }
 
@@ -3334,7 +3319,7 @@ __global__ void __launch_bounds__(256) k_fine(BlendArgs a, const Unit* __restric
                 for (int idx = tid; idx < nP * nQ; idx += blockDim.x)
                 {
                     const int r = idx / nP, c = idx - r * nP;
-                    const float3 g = g_at(S.nd[k], g2 + (size_t)(Q0 + r) * lw2 + P0 + c, 2, a.gmin, a.half);
+                    const float3 g = g_at(S.nd[k], g2 + (size_t)(Q0 + r) * lw2 + P0 + c, a.half);
                     S.g2[0][r][c] = g.x;
                     S.g2[1][r][c] = g.y;
                     S.g2[2][r][c] = g.z;
