@@ -619,8 +619,8 @@ __global__ void __launch_bounds__(32 * kDtWarps, 1) k_dt(BlendArgs a, const int*
     // Cells outside the box are uncovered, so d == 0 there; the cells of R
     // outside the box are uncovered too and come out 0 whatever lies beyond
     // R, and every cell inside the box reads only cells of R.  So the
-    // recurrence on R with +inf beyond it gives the tile transform's values
-    // on R.  Nothing is written outside R: the ownership kernel, the fields'
+    // recurrence on R, with cells without a seed beside and below it and +inf
+    // above, gives the tile transform's values on R.  Nothing is written outside R: the ownership kernel, the fields'
     // only reader, takes d == 0 outside the covered box.
     const int rx0 = max(it.bbox[0] - 1, 0) & ~1, rx1 = min((it.bbox[2] + 1) | 1, Wt - 1);
     const int ry0 = max(it.bbox[1] - 1, 0), ry1 = min(it.bbox[3] + 1, Ht - 1);
@@ -3497,8 +3497,10 @@ size_t dt_prog_bytes(int maxH) { return (size_t)(((maxH + 31) >> 5) + 1) * sizeo
 
 int dt_rows_in_flight(int maxW, int maxH)
 {
-    // (counted by a row of W + 8 floats and 40 KB of staging; launch_dt takes
-    // the warps that fit beside the slots)
+    // Slots of W + 8 floats beside 40 KB of staging: up to kDtRing of them in
+    // half of the shared memory, which leaves room for all warps' staging
+    // tiles, else the two that a ring needs (launch_dt takes the warps that
+    // fit beside them).  This is also the limit of a chunk's width.
     const size_t row = (size_t)((maxW + 8) & ~3) * sizeof(float);
     const size_t fixed = dt_prog_bytes(maxH) + 40 * 1024;
     auto fit = [&](size_t budget) { return budget > fixed ? (int)((budget - fixed) / row) : 0; };

@@ -4,17 +4,15 @@
 // blends overlaps with SeamBlend.cpp:549-587 only); the network's shape is in
 // include/image360_b200_blendnet.h.
 //
-// Convolution as GEMM, per CTA tile of R image rows x 128 pixels:
-//   D[pixel][cout] += A[pixel][(tap, cin)] * B[cout][(tap, cin)]
-// with M = 128 pixels of one row, N = cout, K = 9 * cin in steps of 16.
-// The input halo ((R+2) rows x 130 pixels x cin) sits in shared memory as
-// 8-channel chunks, each a [pixel][8 channels] array of 16-byte rows; any
-// 8 consecutive pixels of it are one 8x16-byte "core matrix" of the K-major
-// no-swizzle layout, so the A operand of tap (dy, dx) is the same buffer with
-// the descriptor's start address moved by (dy * 130 + dx) * 16 bytes - no
-// im2col copy.  Weights are K-major [k/8][cout][8].  fp32 accumulators live in
-// TMEM, two slots so the epilogue of one tile overlaps the MMAs of the next,
-// and halos are double-buffered with cp.async so the next load overlaps both.
+// Convolution as GEMM: D[pixel][cout] += A[pixel][(tap, cin)] * B[cout][(tap,
+// cin)], M = 128 pixels of 8 columns x 16 rows, K in steps of 16.  A tile's
+// input halo sits in shared memory as TMA writes it, a pixel's channels a
+// swizzled row; the swizzle is a function of the address, so the A operand of
+// any tap is the same buffer from another start address - no im2col copy - and
+// with the 16 rows of a block J apart one operand serves three taps of three
+// blocks, N = 3 cout.  fp32 accumulators live in TMEM in two sets, so the
+// epilogue of one tile overlaps the MMAs of the next, and the halos in a ring
+// of stages, so the next load overlaps both (see k_conv3x3).
 //
 // Weight gradient: D[(dy, cin)][(dx, cout)] += X[q + dy][cin] * G[q - dx][cout]
 // summed over pixels q (K), all nine taps in one MMA per 16 pixels; each CTA
@@ -297,11 +295,15 @@ __device__ __forceinline__ void composite_pixel(const i360b_blend_job& J, int y,
 // pixels are successive there, and two rows' taps the same row.
 //
 // Roles:
-//   warp EW lane 0 TMA producer: one 4-D box (channels x (TW+2) x (16J+2)) per
-//                  tile into a STAGES-deep ring, zero fill outside the image;
-//   warp EW+1 lane 0 MMA issuer, into one of two sets of TMEM accumulators;
-//                  commits free the ring stage and publish the accumulators;
-//   warps 0..EW-1  epilogue (EW = 4 or 8): TMEM lanes 32q..32q+31, q = w % 4
+//   warp EW        lane 0 loads a tile's halo by TMA into a STAGES-deep ring, zero
+//                  fill outside the image: one 4-D box (channels x (TW+2) x
+//                  (16J+2)), two for 96 channels of one tensor, or the skip's
+//                  odd and even columns as 5-D boxes and the half-resolution
+//                  tensor's 4-D box;
+//   warp EW+1      issues the MMAs, converged, by one elected thread, into one of
+//                  two sets of TMEM accumulators; commits free the ring stage
+//                  and publish the accumulators;
+//   warps 0..EW-1  epilogue (EW = 4, 8 or 16): TMEM lanes 32q..32q+31, q = w % 4
 //                  (4 rows of each M block) -> bias/ReLU, mask or raw,
 //                  then by TMA from shared memory, or blend head -> global.
 // Every wait is bounded; a timeout sets the error flag and the CTA winds

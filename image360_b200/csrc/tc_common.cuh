@@ -95,7 +95,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, one thread.
 // True in one thread of the (converged) warp.
 __device__ __forceinline__ bool elect_one()
 {
@@ -110,6 +109,7 @@ __device__ __forceinline__ bool elect_one()
     return p != 0;
 }
 
+// D[tmem] (+)= A[smem] * B[smem]^T, one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t idesc, uint32_t accum)
 {
     asm volatile(
@@ -263,7 +263,7 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0,
         : "memory");
 }
 
-// TMEM allocation size: a power of two of at least 32 columns.
+// 5-D tiled TMA load (no multicast), as tma_load_4d.
 __device__ __forceinline__ void tma_load_5d(void* dst, const void* tmap, int c0, int c1, int c2, int c3, int c4,
                                             uint64_t* mbar)
 {
@@ -293,6 +293,7 @@ __device__ __forceinline__ void bulk_wait_read()
 }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// TMEM allocation size: a power of two of at least 32 columns.
 __host__ __device__ constexpr uint32_t tmem_cols(uint32_t n)
 {
     return n <= 32 ? 32u : n <= 64 ? 64u : n <= 128 ? 128u : n <= 256 ? 256u : 512u;

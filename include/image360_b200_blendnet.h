@@ -99,8 +99,9 @@ I360B_API int i360b_blendnet_infer(i360b_blendnet* net, const i360b_blend_job* j
                                    void* stream);
 
 /* One inference pass timed kernel by kernel with CUDA events: kernelMs
- * receives up to maxKernels times (10 kernels, names from
- * i360b_blendnet_kernel_name).  Synchronous. */
+ * receives up to maxKernels times (10 entries, names from
+ * i360b_blendnet_kernel_name; "pool" is about 0, the pool is a part of the
+ * kernel before it).  Synchronous. */
 I360B_API int i360b_blendnet_profile(i360b_blendnet* net, const i360b_blend_job* jobs, int n, int w, int h,
                                      float* kernelMs, int maxKernels);
 I360B_API const char* i360b_blendnet_kernel_name(int kernel);
