@@ -1699,7 +1699,7 @@ struct BlendNet
     float* logits = nullptr;
     bf16 *g8 = nullptr, *gA = nullptr, *gB = nullptr, *du = nullptr, *gh1 = nullptr, *gh2 = nullptr, *dp = nullptr,
          *gC = nullptr, *gh3 = nullptr;
-    void* wgScratch = nullptr;
+    void* wgScratch = nullptr;  // behind the activations
     size_t wgBytes = 0;
     double* dLoss = nullptr;
     int* dError = nullptr;
@@ -1733,7 +1733,6 @@ struct BlendNet
         cudaFree(packed);
         cudaFree(biasPacked);
         cudaFree(act);
-        cudaFree(wgScratch);
         cudaFree(dLoss);
         cudaFree(dError);
         cudaFree(dJobs);
@@ -1828,11 +1827,6 @@ struct BlendNet
         const size_t pix = (size_t)n * w * h;
         if (pix <= capPix && (!training || capTraining)) return I360B_SUCCESS;
         cudaDeviceSynchronize();
-        if (training && !wgScratch)
-        {
-            wgBytes = wgrad_scratch_bytes();
-            I360B_CUDA(cudaMalloc(&wgScratch, wgBytes), "blendnet wgrad scratch");
-        }
         cudaFree(act);
         act = nullptr;
         capPix = 0;
@@ -1846,6 +1840,8 @@ struct BlendNet
         size_t total = 0;
         for (size_t c : counts) total += (c * sizeof(bf16) + 255) / 256 * 256;
         total += pix * 4 * sizeof(float);
+        wgBytes = tr * wgrad_scratch_bytes();
+        total += wgBytes;
         cudaError_t e = cudaMalloc(&act, total);
         if (e != cudaSuccess)
         {
@@ -1862,6 +1858,7 @@ struct BlendNet
             o += (counts[i] * sizeof(bf16) + 255) / 256 * 256;
         }
         logits = reinterpret_cast<float*>(act + o);
+        wgScratch = act + o + pix * 4 * sizeof(float);
         capPix = pix;
         capTraining = training;
         return I360B_SUCCESS;
