@@ -432,8 +432,10 @@ __global__ void __launch_bounds__(32 * kDmWarps, 5) k_demosaic_bayer(const unsig
 // WarpPerspectiveKernels.h:16-43), with RenderExecutor's ApplyGain fused.
 // A warp makes 64 consecutive pixels of a row, lane l the pixels l and l + 32
 // (consecutive lanes gather neighbouring taps, and the two pixels' arithmetic
-// is paired).  Bound by instruction issue and tap latency: a 2048 x 2048 tile
-// 22.9 us, 26.9 us with scalar arithmetic and 2-byte taps.
+// is paired).  Bound by instruction issue and tap latency.  A 2048 x 2048 tile,
+// all of it covered: 24.5 us with the frame in L2, 29.5 from HBM, where fewer
+// threads hide the longer taps; a pixel per lane with scalar arithmetic and
+// 2-byte taps (k_warp_small) 29.1 and 30.2.
 // ---------------------------------------------------------------------------
 constexpr int kWarpPairPixels = 1700;  // destination pixels per SM from which a lane makes two
 

@@ -15,10 +15,14 @@
  *   - i360b_<op>: the IComputeBackend operations.  Host buffers in, host
  *     buffers out, synchronous: results are in host memory on return.  Each
  *     calling thread gets its own CUDA stream.  Device memory comes from a
- *     stream-ordered pool that is kept until i360b_shutdown.
+ *     stream-ordered pool that is kept until i360b_shutdown (what it holds
+ *     idle serves this process's other allocations before they fail).
  *   - i360b_launch_<op> / i360b_render_*: device-resident, stream-ordered
  *     launchers for callers that keep frames in HBM.  `stream` is a
  *     cudaStream_t passed as void* (NULL = the legacy default stream).
+ *     Warps read a source frame as aligned 4-byte words: of a frame at an
+ *     address that is no multiple of 4 the 2 bytes before it (its
+ *     allocation's) may be read, never one past its end.
  *
  * Pixel format: RGB48 = interleaved unsigned short x3, row-major; (0,0,0)
  * means "no data" (WindowsApp.Core/SourceFiles/SeamBlend.cpp:565).
